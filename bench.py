@@ -325,7 +325,8 @@ def run_single(args, world, rank, local):
     alg_k2 = (40 + 64) * N
     k2_gbs = alg_k2 / (kt["flux_ms"] * 1e-3) / 1e9
     roofline = {"bound": "hbm", "achieved": k2_gbs, "peak": hbm, "unit": "GB/s", "frac": k2_gbs / hbm,
-                "traffic": None, "kernel": "k_flux (K2)", "peak_source": peak_kind, "kernel_ms": kt["flux_ms"],
+                "traffic": None, "kernel": "k_stage (one fused stage)" if kt["recon_launches"] == 0 else "k_flux (K2)",
+                "peak_source": peak_kind, "kernel_ms": kt["flux_ms"],
                 "recon_ms": kt["recon_ms"], "alg_bytes_per_launch": alg_k2,
                 "note": "one case: the state is L2-resident and the launches are latency-bound"}
     cpu = None
@@ -413,16 +414,19 @@ def run_throughput(args, world, rank, local, report=True):
     B_eff = B if args.workload != "ragged" else B / len(mesh[0])
     alg_step_bytes = 80 + 128 / B_eff
 
-    # dominant kernel: K2 flux/update, timed per launch with events on its stream
+    # dominant kernel: the fused stage (or K2 at a requested launch shape), timed per launch with events on its stream
     kt = s.profile_step(8)
     hbm, peak_kind = peaks()
     alg_k2 = (40 + 64 / B_eff) * N * B
     k2_gbs = alg_k2 / (kt["flux_ms"] * 1e-3) / 1e9
     # DRAM traffic per item of the K2 form in use, from its ncu summary
     traffic = None
+    fused = kt["recon_launches"] == 0
     patches = bool(tuning.get("k2_patches"))
-    k2_name = "k_flux_patch (K2 by patches)" if patches else "k_flux (K2 per cell)"
-    pf = ROOT / "profiles" / ("k_flux_patch_naca0012_h0.025_b128.md" if patches else "k_flux_naca0012_h0.025_b128.md")
+    k2_name = ("k_stage_pair (one fused stage)" if fused else
+               "k_flux_patch (K2 by patches)" if patches else "k_flux (K2 per cell)")
+    pf = ROOT / "profiles" / ("k_stage_pair_naca0012_h0.025_b96.md" if fused else
+                              "k_flux_patch_naca0012_h0.025_b128.md" if patches else "k_flux_naca0012_h0.025_b128.md")
     if pf.exists():
         for line in pf.read_text().splitlines():
             if line.startswith("traffic_bytes_per_item_per_launch"):
@@ -432,7 +436,7 @@ def run_throughput(args, world, rank, local, report=True):
                 "kernel": k2_name, "peak_source": peak_kind, "kernel_ms": kt["flux_ms"],
                 "recon_ms": kt["recon_ms"], "alg_bytes_per_launch": alg_k2,
                 "workload": f"batched {args.workload} workload, {B} cases per GPU, one launch",
-                "note": "K2 is issue-bound; see profiles/"}
+                "note": "issue-bound; see profiles/"}
 
     # end to end through the public API with host buffers
     e2e = None

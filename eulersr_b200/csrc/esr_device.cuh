@@ -11,6 +11,10 @@
 //              load is a broadcast and every branch on boundary type uniform)
 //   geometry   per mesh, one record of G_COUNT values per cell
 //              (geo[cell * G_COUNT + field], esr_layout.h), read as float4/double4 groups
+//   stage      one Runge-Kutta stage of a MUSCL solve in one kernel
+//              (esr_stage.cuh); the separate pair below remains for fast
+//              float32 HLLC at a requested launch shape, K2 also for constant
+//              reconstruction
 //   K1 recon   cell + 3 neighbour primitives, LSQ gradient, Venkatakrishnan
 //              limiter, the 3 MUSCL face states of the cell -> FV[k][item]
 //   K2 flux    per cell: the 3 face fluxes (HLLC or Rusanov) from its own
@@ -34,6 +38,31 @@ template <typename T> __host__ __device__ inline V4<T> mk4(T a, T b, T c, T d) {
   V4<T> r; r.x = a; r.y = b; r.z = c; r.w = d; return r;
 }
 
+// Records of the fused stage kernel's tiles (esr_stage.cuh), laid out tile by
+// tile so that a block reads each table front to back.
+template <typename T>
+struct alignas(16) StageCell {   // own or ring-1 cell: neighbours' rows, face-state slots, reconstruction geometry
+  uint16_t nbr[3], slot[3];
+  uint32_t kinds;
+  T gc[12];                      // LSQ coefficients and face offsets (geometry groups 3-5)
+};
+template <typename T>
+struct alignas(16) StageOwn {    // own cell: update geometry
+  int cell;
+  T s[3], area, blend3, n[6];
+};
+template <typename T>
+struct alignas(16) StageFace {   // normal of the left side; left | right << 16 (TileFace)
+  T nx, ny;
+  uint32_t slots;
+  int kind;
+};
+template <typename T>
+struct alignas(16) StageGhost {
+  T nx, ny;
+  int cell, kind;
+};
+
 template <typename T>
 struct Seg {                 // one mesh and its B case slots
   int n_cells;
@@ -51,6 +80,13 @@ struct Seg {                 // one mesh and its B case slots
   const int* patch_start;    // first cell of every patch of the renumbering (+ n_cells)
   const int4* live;          // (A, magic, shift, -): slots 0..A-1 may hold running cases (A = B
                              // until a batch's queue is empty and its running cases are packed)
+  const TileHead* tile_head;   // tiles of the fused stage kernel (esr_stage.cuh)
+  const int* tile_list;
+  const StageCell<T>* tile_cells;
+  const StageOwn<T>* tile_own;
+  const StageFace<T>* tile_faces;
+  const StageGhost<T>* tile_ghosts;
+  int slot_shift;              // a tile's block covers 1 << slot_shift case slots
   int n_patches;
   int n_wall;
   int b_shift;               // item / B = (umulhi(item, b_magic) + item) >> b_shift
@@ -111,12 +147,14 @@ __device__ __forceinline__ void block_origin(const BlockMap<T>& bm, Seg<T>& s, i
   }
 }
 
-// Precision policy. FAST = false keeps IEEE division and the reference's
-// exact operation sequence: every float64 kernel, and the float32 kernels of
-// the reference-fidelity mode (compiled without FMA contraction in their own
-// translation unit, esr_faithful.cu). FAST float32 kernels (the default) use
-// the approximate divide (div.approx, <= 2 ulp) and reciprocal-multiplies.
+// Precision policy. The float32 kernels of the reference-fidelity mode (FAST =
+// false, compiled without FMA contraction in their own translation unit,
+// esr_faithful.cu) keep the reference's exact operation sequence. FAST float32
+// (the default) uses approximate reciprocals and square roots (1 ulp); float64
+// uses IEEE division and square root, with the formulas of xr:: below.
 template <typename T, bool FAST> constexpr bool kFastPath = FAST && sizeof(T) == 4;
+// kernels whose numerics are the xr:: functions: fast float32 and float64 MUSCL + HLLC
+template <typename T, bool FAST> constexpr bool kXr = FAST || sizeof(T) == 8;
 template <typename T, bool FAST = (sizeof(T) == 4)>
 __device__ __forceinline__ T dv(T a, T b) {
   if constexpr (kFastPath<T, FAST>) return __fdividef(a, b);
@@ -324,63 +362,332 @@ __device__ __forceinline__ void geo_groups(const Seg<T>& s, int c, int g0, T out
   }
 }
 
-// --------------------------------------------------------------- K1 recon
-// euler_solver.py:106-122 build_reconstruction for MUSCL: BC ghosts, LSQ
-// gradient (helper.py:136-153), limiter (euler_solver.py:45-67) and the cell's
-// own MUSCL face states (euler_solver.py:69-98). Writes FV[k][item] (primitive).
-// With LOCALDT it also writes the per-cell CFL time step of the state.
-// MUSCL=false only computes the local dt (constant reconstruction needs no face states).
-template <typename T, bool FAST, bool MUSCL, bool LOCALDT, int MINB = 0>
-__global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, LOCALDT ? ESR_K1_MINB_LOCAL : ESR_K1_MINB>)) k_recon(const BlockMap<T> bm,
-                                               const V4<T>* __restrict__ W, V4<T>* __restrict__ FV,
-                                               long long total, Cases<T> cs, Consts<T> kc, int pos,
-                                               T* __restrict__ dt_local) {
-  Seg<T> s;
-  int first;
-  block_origin(bm, s, first);
-  int c, b;
-  if (!item_slot(s, first + threadIdx.x, c, b)) return;
-  const int g = s.case0 + b;
-  if (!cs.active[g] || cs.step[g] + pos >= cs.nmax[g]) return;
-  const long long gi = s.off + (long long)c * s.B + b;
-  const V4<T> Wc = W[gi];
-  T Pc[4];
-  prim<T, FAST>(Wc, kc.gm1, kc.half, Pc);
-  if (LOCALDT) {
-    T gn[12];
-    geo_groups<T, 3>(s, c, 0, gn);
-    const T cel = sqrt(fabs(kc.gamma * Pc[3] / Pc[0]));
-    T lam = T(0);
+enum Stage { ST_FIRST = 0, ST_SRK2_SECOND = 1, ST_RK2_SECOND = 2 };
+
+// ---- the fast float32 numerics with every rounding written out (__fmul_rn /
+// __fadd_rn / __fmaf_rn are never fused or split by the compiler), so every
+// kernel that reaches a face or a cell rounds it identically: a case's result
+// does not depend on which kernels ran. Written once over V = float (one case
+// slot) and V = float2 (two case slots of one cell: Blackwell's packed
+// float32 multiply, add and multiply-add do both in one instruction with the
+// same roundings).
+namespace xr {
+struct mask2 { bool x, y; };
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// 1 / x to 1 ulp, subnormals taken as zero: one instruction, where
+// __fdividef without -ftz adds scaling steps around it
+__device__ __forceinline__ float rcp(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float root(float x) {   // to 1 ulp
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float mag(float x) { return fabsf(x); }
+__device__ __forceinline__ float neg(float x) { return -x; }
+__device__ __forceinline__ float lower(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float upper(float a, float b) { return fmaxf(a, b); }
+// three-operand minimum and maximum (one instruction each on sm_100)
+__device__ __forceinline__ float lower(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float upper(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ bool gt(float a, float b) { return a > b; }
+__device__ __forceinline__ bool any(bool m) { return m; }
+__device__ __forceinline__ bool ge(float a, float b) { return a >= b; }
+__device__ __forceinline__ bool eq(float a, float b) { return a == b; }
+__device__ __forceinline__ bool either(bool a, bool b) { return a || b; }
+__device__ __forceinline__ float pick(bool m, float a, float b) { return m ? a : b; }
+__device__ __forceinline__ bool pick(bool m, bool a, bool b) { return m ? a : b; }
+__device__ __forceinline__ bool no(bool m) { return !m; }
+
+// float64: IEEE division and square root
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
+__device__ __forceinline__ double root(double x) { return sqrt(x); }
+__device__ __forceinline__ double mag(double x) { return fabs(x); }
+__device__ __forceinline__ double neg(double x) { return -x; }
+__device__ __forceinline__ double lower(double a, double b) { return fmin(a, b); }
+__device__ __forceinline__ double upper(double a, double b) { return fmax(a, b); }
+__device__ __forceinline__ double lower(double a, double b, double c) { return fmin(fmin(a, b), c); }
+__device__ __forceinline__ double upper(double a, double b, double c) { return fmax(fmax(a, b), c); }
+__device__ __forceinline__ bool gt(double a, double b) { return a > b; }
+__device__ __forceinline__ bool ge(double a, double b) { return a >= b; }
+__device__ __forceinline__ bool eq(double a, double b) { return a == b; }
+__device__ __forceinline__ double pick(bool m, double a, double b) { return m ? a : b; }
+
+__device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// a - b: b times -1 is exact, so the multiply-add rounds once, as the subtraction does
+__device__ __forceinline__ float2 sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 rcp(float2 a) { return make_float2(rcp(a.x), rcp(a.y)); }
+__device__ __forceinline__ float2 root(float2 a) { return make_float2(root(a.x), root(a.y)); }
+__device__ __forceinline__ float2 mag(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
+__device__ __forceinline__ float2 neg(float2 a) { return __fmul2_rn(a, make_float2(-1.f, -1.f)); }
+__device__ __forceinline__ float2 lower(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
+__device__ __forceinline__ float2 upper(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+__device__ __forceinline__ float2 lower(float2 a, float2 b, float2 c) {
+  return make_float2(lower(a.x, b.x, c.x), lower(a.y, b.y, c.y));
+}
+__device__ __forceinline__ float2 upper(float2 a, float2 b, float2 c) {
+  return make_float2(upper(a.x, b.x, c.x), upper(a.y, b.y, c.y));
+}
+__device__ __forceinline__ bool any(mask2 m) { return m.x || m.y; }
+__device__ __forceinline__ mask2 gt(float2 a, float2 b) { return {a.x > b.x, a.y > b.y}; }
+__device__ __forceinline__ mask2 ge(float2 a, float2 b) { return {a.x >= b.x, a.y >= b.y}; }
+__device__ __forceinline__ mask2 eq(float2 a, float2 b) { return {a.x == b.x, a.y == b.y}; }
+__device__ __forceinline__ mask2 either(mask2 a, mask2 b) { return {a.x || b.x, a.y || b.y}; }
+__device__ __forceinline__ float2 pick(mask2 m, float2 a, float2 b) {
+  return make_float2(m.x ? a.x : b.x, m.y ? a.y : b.y);
+}
+__device__ __forceinline__ mask2 pick(mask2 m, mask2 a, mask2 b) { return {m.x ? a.x : b.x, m.y ? a.y : b.y}; }
+__device__ __forceinline__ mask2 no(mask2 m) { return {!m.x, !m.y}; }
+
+template <typename V> struct ScalarOf { using type = V; };
+template <> struct ScalarOf<float2> { using type = float; };
+template <typename V> using Scalar = typename ScalarOf<V>::type;
+template <typename V> __device__ __forceinline__ V splat(Scalar<V> a) { return a; }
+template <> __device__ __forceinline__ float2 splat<float2>(float a) { return make_float2(a, a); }
+
+// helper.py:37-46 (M = 1), W = (rho, rho u, rho v, E)
+template <typename V>
+__device__ __forceinline__ void prim(const V W[4], Scalar<V> gm1, Scalar<V> half, V P[4]) {
+  const V ri = rcp(W[0]), u = mul(W[1], ri), v = mul(W[2], ri);
+  P[0] = W[0]; P[1] = u; P[2] = v;
+  P[3] = mul(sub(W[3], mul(mul(splat<V>(half), W[0]), fma(u, u, mul(v, v)))), splat<V>(gm1));
+}
+template <typename T>
+__device__ __forceinline__ void prim4(const V4<T>& W, T gm1, T half, T P[4]) {
+  const T w[4] = {W.x, W.y, W.z, W.w};
+  prim<T>(w, gm1, half, P);
+}
+// helper.py:25-35 (M = 1)
+template <typename T>
+__device__ __forceinline__ V4<T> cons(const T P[4], T inv_gm1, T half) {
+  const T r = P[0], u = P[1], v = P[2];
+  return mk4<T>(r, mul(r, u), mul(r, v), fma(mul(half, r), fma(u, u, mul(v, v)), mul(P[3], inv_gm1)));
+}
+// helper.py:233-256 boundary states, as primitives of the ghost (gamma 1.4)
+template <typename T>
+__device__ __forceinline__ void ghost_prim(int kind, const V4<T>& Wc, T nx, T ny, const V4<T>& inlet,
+                                           const Consts<T>& k, T Q[4]) {
+  T P[4];
+  if (kind == K_INLET) { prim4<T>(inlet, k.gm1, k.half, Q); return; }
+  if (kind != K_WALL && kind != K_SUBSONIC) { prim4<T>(Wc, k.gm1, k.half, Q); return; }   // outlet
+  prim4<T>(Wc, k.gm1_14, k.half, P);
+  T G[4];
+  if (kind == K_WALL) {       // helper.py:196-204
+    const T t = mul(T(2), fma(P[1], nx, mul(P[2], ny)));
+    G[0] = P[0]; G[1] = sub(P[1], mul(t, nx)); G[2] = sub(P[2], mul(t, ny)); G[3] = P[3];
+  } else {                    // helper.py:179-194
+    G[0] = k.sub_rho; G[1] = k.sub_u; G[2] = k.sub_v; G[3] = P[3];
+  }
+  prim4<T>(cons<T>(G, k.inv_gm1_14, k.half), k.gm1, k.half, Q);
+}
+// euler_solver.py:273-374 HLLC flux of two face states (primitive) through
+// the unit normal (nx, ny). In the star region of side K the flux
+// F_K + S_K (U*_K - U_K) is that of the star state itself, (rho* S*,
+// rho* S*^2 + p*, rho* S* u_t, (E* + p*) S*): the same in real arithmetic,
+// with no difference of nearly equal numbers. So the wave fan selects a state
+// (density, normal velocity, pressure, energy) and one flux formula ends it.
+template <typename V>
+__device__ __forceinline__ void hllc(const V PL[4], const V PR[4], Scalar<V> nx_, Scalar<V> ny_,
+                                     const Consts<Scalar<V>>& k, V F[4]) {
+  const V nx = splat<V>(nx_), ny = splat<V>(ny_), zero = splat<V>(0), half = splat<V>(k.half);
+  const V rL = PL[0], pL = PL[3], rR = PR[0], pR = PR[3];
+  const V unL = fma(PL[1], nx, mul(PL[2], ny)), unR = fma(PR[1], nx, mul(PR[2], ny));
+  const V aL = root(mag(mul(mul(splat<V>(k.gamma), pL), rcp(rL))));
+  const V aR = root(mag(mul(mul(splat<V>(k.gamma), pR), rcp(rR))));
+  V SL = lower(sub(unL, aL), sub(unR, aR));
+  V SR = upper(add(unL, aL), add(unR, aR));
+  V mL = mul(rL, sub(SL, unL)), mR = mul(rR, sub(SR, unR)), den = sub(mL, mR);
+  if (any(eq(den, zero))) {
+    // the reference's nudges. Equal speeds mean that both sound speeds are
+    // zero, so that they always come with a zero denominator.
+    SL = pick(eq(SL, SR), sub(SL, splat<V>(k.ss_eps)), SL);
+    SR = pick(eq(SL, SR), add(SR, splat<V>(k.ss_eps)), SR);
+    mL = mul(rL, sub(SL, unL));
+    mR = mul(rR, sub(SR, unR));
+    den = sub(mL, mR);
+    den = pick(eq(den, zero), splat<V>(k.den_eps), den);
+  }
+  const V Ss = mul(fma(mL, unL, sub(sub(pR, pL), mul(mR, unR))), rcp(den));
+  const V PsL = fma(mL, sub(Ss, unL), pL), PsR = fma(mR, sub(Ss, unR), pR);
+  const V Ps = mul(half, add(PsL, PsR));
+  const auto left = either(ge(SL, zero), ge(Ss, zero));
+  const auto star = pick(left, no(ge(SL, zero)), ge(SR, zero));
+  const V rK = pick(left, rL, rR), uK = pick(left, PL[1], PR[1]), vK = pick(left, PL[2], PR[2]);
+  const V pK = pick(left, pL, pR), unK = pick(left, unL, unR), SK = pick(left, SL, SR);
+  const V dK = sub(SK, unK), mK = mul(rK, dK);
+  const V EK = fma(mul(half, rK), fma(uK, uK, mul(vK, vK)), mul(pK, splat<V>(k.inv_gm1)));
+  const V inv = rcp(sub(SK, Ss));
+  const V Es = mul(fma(Ps, Ss, sub(mul(dK, EK), mul(pK, unK))), inv);
+  const V r = pick(star, mul(mK, inv), rK), un = pick(star, Ss, unK), p = pick(star, Ps, pK), E = pick(star, Es, EK);
+  const V ut = sub(mul(vK, nx), mul(uK, ny));
+  const V m = mul(r, un), Fn = fma(m, un, p), Ft = mul(m, ut);
+  F[0] = m;
+  F[1] = sub(mul(Fn, nx), mul(Ft, ny));
+  F[2] = fma(Fn, ny, mul(Ft, nx));
+  F[3] = mul(add(E, p), un);
+}
+// the canonical flux of a face through the cell's edge of outward normal n:
+// evaluated from the face's owner (the lower cell), negated on the other side
+__device__ __forceinline__ void face_flux(const float qOwn[4], const float qOther[4], float nx, float ny,
+                                          bool other_owns, const Consts<float>& k, float F[4]) {
+  if (other_owns) {
+    hllc<float>(qOther, qOwn, -nx, -ny, k, F);
+    F[0] = -F[0]; F[1] = -F[1]; F[2] = -F[2]; F[3] = -F[3];
+  } else {
+    hllc<float>(qOwn, qOther, nx, ny, k, F);
+  }
+}
+// sum_k s_k F_k in slot order: face k's term added to acc
+template <typename V>
+__device__ __forceinline__ void accumulate(int k, Scalar<V> sk_, const V F[4], V acc[4]) {
+  const V sk = splat<V>(sk_);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const T un = Pc[1] * gn[G_N0X + 2 * k] + Pc[2] * gn[G_N0Y + 2 * k];
-      const T term = (cel + fabs(un)) * gn[G_S0 + k];
-      lam = (k == 0) ? term : lam + term;
+  for (int v = 0; v < 4; ++v) acc[v] = k == 0 ? mul(sk, F[v]) : fma(sk, F[v], acc[v]);
+}
+// euler_solver.py:602-643: residual acc / area - sponge and the stage update
+template <int STAGE, typename V>
+__device__ __forceinline__ void cell_update(const V acc[4], Scalar<V> area, V sig, const V inlet[4], const V Wc[4],
+                                            const V W0[4], V dt, Scalar<V> half_, V* R0_out, V out[4]) {
+  const V ra = splat<V>(rcp(area)), half = splat<V>(half_);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    const V R = sub(mul(acc[v], ra), mul(sig, sub(inlet[v], Wc[v])));
+    if (v == 0) *R0_out = R;
+    const V h = neg(dt);
+    // second stage (SRK2 and RK2 alike): (W0 + Wc - dt R) / 2 as
+    // W0 + (Wc - W0 - dt R) / 2, which rounds once at the state's magnitude
+    if (STAGE == ST_FIRST) out[v] = fma(h, R, Wc[v]);
+    else out[v] = fma(half, fma(h, R, sub(Wc[v], W0[v])), W0[v]);
+  }
+}
+template <int STAGE, typename T>
+__device__ __forceinline__ V4<T> cell_update4(const T acc[4], T area, T sig, const V4<T>& inlet, const V4<T>& Wc,
+                                              const V4<T>& W0, T dt, T half, T* R0_out) {
+  const T in[4] = {inlet.x, inlet.y, inlet.z, inlet.w}, wc[4] = {Wc.x, Wc.y, Wc.z, Wc.w};
+  const T w0[4] = {W0.x, W0.y, W0.z, W0.w};
+  T o[4];
+  cell_update<STAGE, T>(acc, area, sig, in, wc, w0, dt, half, R0_out, o);
+  return mk4<T>(o[0], o[1], o[2], o[3]);
+}
+// the LSQ gradient, the Venkatakrishnan limiter (minimum over the three
+// faces, 1 where the face increment is below eps_lim) and the face states.
+// With hi = max(P_k - P_c, 0) and lo = min(P_k - P_c, 0) (exact: subtraction
+// is monotonic) a face of increment d has
+// phi = (a a + 2 a d) / (a a + 2 d d + a d + eps), a = hi or lo by d's sign.
+// NV variables at a time: each is independent of the others.
+template <typename V, int NV>
+__device__ __forceinline__ void limited_faces(const V Pc[NV], const V Pk[3][NV], const Scalar<V> gc[12],
+                                              const Consts<Scalar<V>>& k, V out[3][NV]) {
+  const V zero = splat<V>(0), one = splat<V>(1), veps = splat<V>(k.venk_eps), leps = splat<V>(k.eps_lim);
+  V c[12];
+#pragma unroll
+  for (int i = 0; i < 12; ++i) c[i] = splat<V>(gc[i]);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const V d0 = sub(Pk[0][v], Pc[v]), d1 = sub(Pk[1][v], Pc[v]), d2 = sub(Pk[2][v], Pc[v]);
+    const V gx = fma(c[G_C2X - 12], d2, fma(c[G_C1X - 12], d1, mul(c[G_C0X - 12], d0)));
+    const V gy = fma(c[G_C2Y - 12], d2, fma(c[G_C1Y - 12], d1, mul(c[G_C0Y - 12], d0)));
+    const V hi = upper(d0, d1, upper(d2, zero)), lo = lower(d0, d1, lower(d2, zero));
+    V D[3], phi[3], least;
+    V dens[3];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const V d = fma(c[G_F0Y - 12 + 2 * f], gy, mul(c[G_F0X - 12 + 2 * f], gx));
+      D[f] = d;
+      const V a = pick(gt(d, zero), hi, lo), b2 = add(d, d), aa = mul(a, a);
+      const V den = fma(a, d, fma(b2, d, add(aa, veps)));
+      if constexpr (sizeof(Scalar<V>) == 8) {   // numerator and denominator: one division below
+        const auto on = gt(mag(d), leps);
+        phi[f] = pick(on, fma(b2, a, aa), one);
+        dens[f] = pick(on, den, one);
+      } else {
+        phi[f] = pick(gt(mag(d), leps), mul(fma(b2, a, aa), rcp(den)), one);
+      }
     }
-    dt_local[gi] = gn[G_AREA] / lam * cs.dt[g];   // cs.dt holds the case CFL in local mode
-  }
-  if (!MUSCL) return;
-  const int4 nb = __ldg(s.nbr + c);
-  const int nbk[3] = {nb.x, nb.y, nb.z};
-  T Pk[3][4];
-  const V4<T> inlet = cs.inlet[g];
+    if constexpr (sizeof(Scalar<V>) == 8) {
+      // A float64 division costs as much as the rest of a face's limiter, so
+      // the smallest of the three fractions (denominators positive) is found
+      // by cross-multiplication and divided once.
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const int kind = slot_kind(nb.w, k);
-    V4<T> Wk;
-    if (kind == K_INTERIOR) Wk = W[s.off + (long long)nbk[k] * s.B + b];
-    else Wk = ghost_cons<T, FAST>(kind, Wc, geo(s, G_N0X + 2 * k, c), geo(s, G_N0Y + 2 * k, c), inlet, kc);
-    prim<T, FAST>(Wk, kc.gm1, kc.half, Pk[k]);
+      for (int f = 1; f < 3; ++f) {
+        const auto less = gt(mul(phi[0], dens[f]), mul(phi[f], dens[0]));
+        phi[0] = pick(less, phi[f], phi[0]);
+        dens[0] = pick(less, dens[f], dens[0]);
+      }
+      least = phi[0] / dens[0];
+    } else {
+      least = lower(phi[0], phi[1], phi[2]);
+    }
+#pragma unroll
+    for (int f = 0; f < 3; ++f) out[f][v] = fma(least, D[f], Pc[v]);
   }
-  T gc[12];   // LSQ coefficients and face offsets (groups 3-5)
-  geo_groups<T, 3>(s, c, 3, gc);
+}
+// helper.py:8-18 for one cell
+template <typename V>
+__device__ __forceinline__ V local_dt(const V P[4], const Scalar<V> n[6], const Scalar<V> len[3], Scalar<V> area,
+                                      const Consts<Scalar<V>>& k) {
+  const V cel = root(mag(mul(mul(splat<V>(k.gamma), P[3]), rcp(P[0]))));
+  V lam = splat<V>(0);
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+    const V un = fma(P[1], splat<V>(n[2 * f]), mul(P[2], splat<V>(n[2 * f + 1])));
+    const V a = add(cel, mag(un)), s = splat<V>(len[f]);
+    lam = f == 0 ? mul(a, s) : fma(a, s, lam);
+  }
+  return mul(splat<V>(area), rcp(lam));
+}
+}  // namespace xr
+
+// primitives of a cell state, and of a boundary slot's ghost, in the run's rounding
+template <typename T, bool FAST>
+__device__ __forceinline__ void cell_prim(const V4<T>& W, const Consts<T>& k, T P[4]) {
+  if constexpr (kXr<T, FAST>) xr::prim4<T>(W, k.gm1, k.half, P);
+  else prim<T, FAST>(W, k.gm1, k.half, P);
+}
+template <typename T, bool FAST>
+__device__ __forceinline__ void ghost_prim(int kind, const V4<T>& Wc, T nx, T ny, const V4<T>& inlet,
+                                           const Consts<T>& k, T Q[4]) {
+  if constexpr (kXr<T, FAST>) xr::ghost_prim<T>(kind, Wc, nx, ny, inlet, k, Q);
+  else prim<T, FAST>(ghost_cons<T, FAST>(kind, Wc, nx, ny, inlet, k), k.gm1, k.half, Q);
+}
+
+// The cell's limited gradient and its three MUSCL face states (primitive)
+// from its own and its neighbours' (or ghosts') primitives: LSQ gradient
+// (helper.py:136-153), limiter (euler_solver.py:45-67), face states
+// (euler_solver.py:69-98). gc: LSQ coefficients and face offsets.
+template <typename T, bool FAST>
+__device__ __forceinline__ void limited_faces(const T Pc[4], const T Pk[3][4], const T gc[12], const LsqRef* lsq, int c,
+                                              const Consts<T>& kc, T out[3][4]) {
+  if constexpr (kXr<T, FAST>) {
+    xr::limited_faces<T, 4>(Pc, Pk, gc, kc, out);
+  } else {
   T gx[4], gy[4];
   if constexpr (!FAST && sizeof(T) == 4) {
     // helper.py:136-153 per call, in the reference's float32 rounding:
     // b = sum_k (w_k dW_k) dx_k summed k = 0, 1, 2 in turn, then the 2x2
     // solve with partial pivoting in float64 rounded to float32 (what
     // numpy.linalg.solve computes for float32 operands)
-    const LsqRef L = s.lsq[c];
+    const LsqRef L = lsq[c];
     const double a00 = L.a[0], a01 = L.a[1], a10 = L.a[2], a11 = L.a[3];
     const bool sw = fabs(a10) > fabs(a00);
     const double p00 = sw ? a10 : a00, p01 = sw ? a11 : a01, p10 = sw ? a00 : a10, p11 = sw ? a01 : a11;
@@ -428,13 +735,80 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, LOCALDT ? ESR_
     phi[v] = ph;
   }
 #pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) out[k][v] = Pc[v] + phi[v] * D[k][v];
+  }
+}
+
+// per-cell CFL time step over the case's CFL number (helper.py:8-18)
+template <typename T, bool FAST>
+__device__ __forceinline__ T local_dt(const T P[4], const T n[6], const T len[3], T area, const Consts<T>& kc) {
+  if constexpr (kXr<T, FAST>) {
+    return xr::local_dt<T>(P, n, len, area, kc);
+  } else {
+    const T cel = sqrt(fabs(kc.gamma * P[3] / P[0]));
+    T lam = T(0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const T un = P[1] * n[2 * k] + P[2] * n[2 * k + 1];
+      const T term = (cel + fabs(un)) * len[k];
+      lam = (k == 0) ? term : lam + term;
+    }
+    return area / lam;
+  }
+}
+
+// --------------------------------------------------------------- K1 recon
+// euler_solver.py:106-122 build_reconstruction for MUSCL: BC ghosts, LSQ
+// gradient (helper.py:136-153), limiter (euler_solver.py:45-67) and the cell's
+// own MUSCL face states (euler_solver.py:69-98). Writes FV[k][item] (primitive).
+// With LOCALDT it also writes the per-cell CFL time step of the state.
+// MUSCL=false only computes the local dt (constant reconstruction needs no face states).
+template <typename T, bool FAST, bool MUSCL, bool LOCALDT, int MINB = 0>
+__global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, LOCALDT ? ESR_K1_MINB_LOCAL : ESR_K1_MINB>)) k_recon(const BlockMap<T> bm,
+                                               const V4<T>* __restrict__ W, V4<T>* __restrict__ FV,
+                                               long long total, Cases<T> cs, Consts<T> kc, int pos,
+                                               T* __restrict__ dt_local) {
+  Seg<T> s;
+  int first;
+  block_origin(bm, s, first);
+  int c, b;
+  if (!item_slot(s, first + threadIdx.x, c, b)) return;
+  const int g = s.case0 + b;
+  if (!cs.active[g] || cs.step[g] + pos >= cs.nmax[g]) return;
+  const long long gi = s.off + (long long)c * s.B + b;
+  const V4<T> Wc = W[gi];
+  T Pc[4];
+  cell_prim<T, FAST>(Wc, kc, Pc);
+  if (LOCALDT) {
+    T gn[12];
+    geo_groups<T, 3>(s, c, 0, gn);
+    dt_local[gi] = local_dt<T, FAST>(Pc, gn + G_N0X, gn + G_S0, gn[G_AREA], kc) * cs.dt[g];   // cs.dt holds the case CFL in local mode
+  }
+  if (!MUSCL) return;
+  const int4 nb = __ldg(s.nbr + c);
+  const int nbk[3] = {nb.x, nb.y, nb.z};
+  T Pk[3][4];
+  const V4<T> inlet = cs.inlet[g];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int kind = slot_kind(nb.w, k);
+    if (kind == K_INTERIOR)
+      cell_prim<T, FAST>(W[s.off + (long long)nbk[k] * s.B + b], kc, Pk[k]);
+    else
+      ghost_prim<T, FAST>(kind, Wc, geo(s, G_N0X + 2 * k, c), geo(s, G_N0Y + 2 * k, c), inlet, kc, Pk[k]);
+  }
+  T gc[12];   // LSQ coefficients and face offsets (groups 3-5)
+  geo_groups<T, 3>(s, c, 3, gc);
+  T q[3][4];
+  limited_faces<T, FAST>(Pc, Pk, gc, s.lsq, c, kc, q);
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int kind = slot_kind(nb.w, k);
     V4<T> o;
-    if (kind == K_INTERIOR)
-      o = mk4<T>(Pc[0] + phi[0] * D[k][0], Pc[1] + phi[1] * D[k][1], Pc[2] + phi[2] * D[k][2], Pc[3] + phi[3] * D[k][3]);
-    else
-      o = mk4<T>(Pc[0], Pc[1], Pc[2], Pc[3]);
+    if (kind == K_INTERIOR) o = mk4<T>(q[k][0], q[k][1], q[k][2], q[k][3]);
+    else o = mk4<T>(Pc[0], Pc[1], Pc[2], Pc[3]);
     FV[(long long)k * total + gi] = o;
   }
 }
@@ -475,128 +849,6 @@ __global__ void k_grad_export(const Seg<T>* __restrict__ segs, int seg, int b, c
 }
 
 // ----------------------------------------------------------------- K2 flux
-enum Stage { ST_FIRST = 0, ST_SRK2_SECOND = 1, ST_RK2_SECOND = 2 };
-
-// ---- the fast float32 face flux and cell update with every rounding written
-// out (__fmul_rn / __fadd_rn / __fsub_rn / __fmaf_rn are never fused or
-// split by the compiler), so the per-cell K2 and K2 by patches, which reach
-// the same faces from different code, round every face flux and every cell
-// update identically: a case's result does not depend on which K2 ran.
-namespace xr {
-__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-
-// helper.py:37-46 (M = 1)
-__device__ __forceinline__ void prim(const float4& W, float gm1, float half, float P[4]) {
-  const float r = W.x, ri = __fdividef(1.0f, r);
-  const float u = mul(W.y, ri), v = mul(W.z, ri);
-  P[0] = r; P[1] = u; P[2] = v;
-  P[3] = mul(sub(W.w, mul(mul(half, r), fma(u, u, mul(v, v)))), gm1);
-}
-// helper.py:25-35 (M = 1)
-__device__ __forceinline__ float4 cons(const float P[4], float inv_gm1, float half) {
-  const float r = P[0], u = P[1], v = P[2];
-  return make_float4(r, mul(r, u), mul(r, v), fma(mul(half, r), fma(u, u, mul(v, v)), mul(P[3], inv_gm1)));
-}
-// helper.py:233-256 boundary states, as primitives of the ghost (gamma 1.4)
-__device__ __forceinline__ void ghost_prim(int kind, const float4& Wc, float nx, float ny, const float4& inlet,
-                                           const Consts<float>& k, float Q[4]) {
-  float P[4];
-  if (kind == K_INLET) { prim(inlet, k.gm1, k.half, Q); return; }
-  if (kind != K_WALL && kind != K_SUBSONIC) { prim(Wc, k.gm1, k.half, Q); return; }   // outlet
-  prim(Wc, k.gm1_14, k.half, P);
-  float G[4];
-  if (kind == K_WALL) {       // helper.py:196-204
-    const float t = mul(2.0f, fma(P[1], nx, mul(P[2], ny)));
-    G[0] = P[0]; G[1] = sub(P[1], mul(t, nx)); G[2] = sub(P[2], mul(t, ny)); G[3] = P[3];
-  } else {                    // helper.py:179-194
-    G[0] = k.sub_rho; G[1] = k.sub_u; G[2] = k.sub_v; G[3] = P[3];
-  }
-  prim(cons(G, k.inv_gm1_14, k.half), k.gm1, k.half, Q);
-}
-// euler_solver.py:273-374 HLLC flux from the face primitives, the conserved
-// variables formed only for the side the wave fan selects
-__device__ __forceinline__ void hllc(const float PL[4], const float PR[4], float nx, float ny,
-                                     const Consts<float>& k, float F[4]) {
-  const float rL = PL[0], uL = PL[1], vL = PL[2], pL = PL[3];
-  const float rR = PR[0], uR = PR[1], vR = PR[2], pR = PR[3];
-  const float unL = fma(uL, nx, mul(vL, ny)), unR = fma(uR, nx, mul(vR, ny));
-  const float tx = -ny, ty = nx;
-  const float aL = sqrtf(fabsf(__fdividef(mul(k.gamma, pL), rL)));
-  const float aR = sqrtf(fabsf(__fdividef(mul(k.gamma, pR), rR)));
-  float SL = fminf(sub(unL, aL), sub(unR, aR));
-  float SR = fmaxf(add(unL, aL), add(unR, aR));
-  if (SL == SR) SL = sub(SL, k.ss_eps);
-  if (SL == SR) SR = add(SR, k.ss_eps);
-  const float dL = sub(SL, unL), dR = sub(SR, unR);
-  float den = sub(mul(rL, dL), mul(rR, dR));
-  if (den == 0.0f) den = k.den_eps;
-  const float Ss = __fdividef(sub(fma(mul(rL, unL), dL, sub(pR, pL)), mul(mul(rR, unR), dR)), den);
-  const float PsL = fma(mul(rL, dL), sub(Ss, unL), pL);
-  const float PsR = fma(mul(rR, dR), sub(Ss, unR), pR);
-  const float Ps = mul(k.half, add(PsL, PsR));
-  const bool c1 = SL >= 0.0f;
-  const bool c2 = (SL <= 0.0f) && (Ss >= 0.0f);
-  const bool c3 = (Ss <= 0.0f) && (SR >= 0.0f);
-  const bool left = c1 || c2;
-  const float rK = left ? rL : rR, uK = left ? uL : uR, vK = left ? vL : vR, pK = left ? pL : pR;
-  const float unK = left ? unL : unR, SK = left ? SL : SR, dK = left ? dL : dR;
-  const float EK = fma(mul(k.half, rK), fma(uK, uK, mul(vK, vK)), mul(pK, k.inv_gm1));
-  const float ruK = mul(rK, uK), rvK = mul(rK, vK);
-  const float FK0 = mul(rK, unK), FK1 = fma(pK, nx, mul(ruK, unK)), FK2 = fma(pK, ny, mul(rvK, unK));
-  const float FK3 = mul(add(EK, pK), unK);
-  if (left ? !c1 : c3) {
-    const float inv = __fdividef(1.0f, sub(SK, Ss));
-    const float rs = mul(mul(rK, dK), inv);
-    const float Us3 = mul(fma(Ps, Ss, sub(mul(dK, EK), mul(pK, unK))), inv);
-    const float utK = fma(uK, tx, mul(vK, ty));
-    const float Us1 = mul(rs, fma(Ss, nx, mul(utK, tx))), Us2 = mul(rs, fma(Ss, ny, mul(utK, ty)));
-    F[0] = fma(SK, sub(rs, rK), FK0);
-    F[1] = fma(SK, sub(Us1, ruK), FK1);
-    F[2] = fma(SK, sub(Us2, rvK), FK2);
-    F[3] = fma(SK, sub(Us3, EK), FK3);
-  } else {
-    F[0] = FK0; F[1] = FK1; F[2] = FK2; F[3] = FK3;
-  }
-}
-// the canonical flux of a face through the cell's edge of outward normal n:
-// evaluated from the face's owner (the lower cell), negated on the other side
-__device__ __forceinline__ void face_flux(const float qOwn[4], const float qOther[4], float nx, float ny,
-                                          bool other_owns, const Consts<float>& k, float F[4]) {
-  if (other_owns) {
-    hllc(qOther, qOwn, -nx, -ny, k, F);
-    F[0] = -F[0]; F[1] = -F[1]; F[2] = -F[2]; F[3] = -F[3];
-  } else {
-    hllc(qOwn, qOther, nx, ny, k, F);
-  }
-}
-// sum_k s_k F_k in slot order: face k's term added to acc
-__device__ __forceinline__ void accumulate(int k, float sk, const float F[4], float acc[4]) {
-  if (k == 0) { acc[0] = mul(sk, F[0]); acc[1] = mul(sk, F[1]); acc[2] = mul(sk, F[2]); acc[3] = mul(sk, F[3]); }
-  else { acc[0] = fma(sk, F[0], acc[0]); acc[1] = fma(sk, F[1], acc[1]); acc[2] = fma(sk, F[2], acc[2]); acc[3] = fma(sk, F[3], acc[3]); }
-}
-// euler_solver.py:602-643: residual acc / area - sponge and the stage update
-template <int STAGE>
-__device__ __forceinline__ float4 cell_update(const float acc[4], float area, float sig, const float4& inlet,
-                                              const float4& Wc, const float4& W0, float dt, float half,
-                                              float* R0_out) {
-  const float R0 = sub(__fdividef(acc[0], area), mul(sig, sub(inlet.x, Wc.x)));
-  const float R1 = sub(__fdividef(acc[1], area), mul(sig, sub(inlet.y, Wc.y)));
-  const float R2 = sub(__fdividef(acc[2], area), mul(sig, sub(inlet.z, Wc.z)));
-  const float R3 = sub(__fdividef(acc[3], area), mul(sig, sub(inlet.w, Wc.w)));
-  *R0_out = R0;
-  const float m = -dt;
-  if (STAGE == ST_FIRST) return make_float4(fma(m, R0, Wc.x), fma(m, R1, Wc.y), fma(m, R2, Wc.z), fma(m, R3, Wc.w));
-  if (STAGE == ST_SRK2_SECOND)
-    return make_float4(mul(half, fma(m, R0, add(W0.x, Wc.x))), mul(half, fma(m, R1, add(W0.y, Wc.y))),
-                       mul(half, fma(m, R2, add(W0.z, Wc.z))), mul(half, fma(m, R3, add(W0.w, Wc.w))));
-  return make_float4(mul(half, add(fma(m, R0, W0.x), Wc.x)), mul(half, add(fma(m, R1, W0.y), Wc.y)),
-                     mul(half, add(fma(m, R2, W0.z), Wc.z)), mul(half, add(fma(m, R3, W0.w), Wc.w)));
-}
-}  // namespace xr
-
 // euler_solver.py:602-628 residual = sum_k F_k s_k / area - sponge (helper.py:262-295),
 // then the stage update of :630-653.
 template <typename T, bool FAST, int FLUX, bool MUSCL, int STAGE, bool LOCALDT, int MINB = 0>
@@ -634,17 +886,17 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, ESR_K2_MINB>))
         const float4 fr = FV[(long long)slot_opp(nb.w, k) * total + s.off + (long long)nbk[k] * s.B + b];
         qR[0] = fr.x; qR[1] = fr.y; qR[2] = fr.z; qR[3] = fr.w;
       } else {
-        xr::ghost_prim(kind, Wc, nx, ny, inlet, kc, qR);
+        xr::ghost_prim<float>(kind, Wc, nx, ny, inlet, kc, qR);
       }
       float F[4];
       xr::face_flux(qL, qR, nx, ny, kind == K_INTERIOR && nbk[k] < c, kc, F);
-      xr::accumulate(k, gk[G_S0 + k], F, acc);
+      xr::accumulate<float>(k, gk[G_S0 + k], F, acc);
     }
     const float sig = xr::mul(cs.strength[g], gk[G_BLEND3]);
     const float dt = LOCALDT ? dt_local[gi] : cs.dt[g];
     const float4 W0 = (STAGE == ST_FIRST) ? Wc : Wbase[gi];
     float R0;
-    const float4 o = xr::cell_update<STAGE>(acc, gk[G_AREA], sig, inlet, Wc, W0, dt, kc.half, &R0);
+    const float4 o = xr::cell_update4<STAGE, float>(acc, gk[G_AREA], sig, inlet, Wc, W0, dt, kc.half, &R0);
     if (STAGE == ST_FIRST && res_out != nullptr) res_out[gi] = R0;
     Wout[gi] = o;
   } else {
@@ -653,40 +905,12 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, ESR_K2_MINB>))
     for (int k = 0; k < 3; ++k) {
       const int kind = slot_kind(nb.w, k);
       const T nx = gk[G_N0X + 2 * k], ny = gk[G_N0Y + 2 * k];
-      V4<T> WL, WR;
       T PL[4], PR[4];
-      if (MUSCL) {
-        const V4<T> fl = FV[(long long)k * total + gi];
-        T qL[4] = {fl.x, fl.y, fl.z, fl.w};
-        T qR[4];
-        if (kind == K_INTERIOR) {
-          const V4<T> fr = FV[(long long)slot_opp(nb.w, k) * total + s.off + (long long)nbk[k] * s.B + b];
-          qR[0] = fr.x; qR[1] = fr.y; qR[2] = fr.z; qR[3] = fr.w;
-        } else {
-          prim<T, FAST>(ghost_cons<T, FAST>(kind, Wc, nx, ny, inlet, kc), kc.gm1, kc.half, qR);
-        }
-        if constexpr (kFastPath<T, FAST>) {
-          // float32: the face primitives are used as reconstructed (the
-          // reference converts them to conserved and back, a rounding-level
-          // step); HLLC forms the conserved state of the selected side itself
-  #pragma unroll
-          for (int v = 0; v < 4; ++v) { PL[v] = qL[v]; PR[v] = qR[v]; }
-          if (FLUX != 0) {
-            WL = cons<T, FAST>(qL, kc.gm1, kc.inv_gm1, kc.half);
-            WR = cons<T, FAST>(qR, kc.gm1, kc.inv_gm1, kc.half);
-          }
-        } else {
-          WL = cons<T, FAST>(qL, kc.gm1, kc.inv_gm1, kc.half);
-          WR = cons<T, FAST>(qR, kc.gm1, kc.inv_gm1, kc.half);
-          prim<T, FAST>(WL, kc.gm1, kc.half, PL);
-          prim<T, FAST>(WR, kc.gm1, kc.half, PR);
-        }
-      } else {
-        WL = Wc;
-        WR = (kind == K_INTERIOR) ? Win[s.off + (long long)nbk[k] * s.B + b] : ghost_cons<T, FAST>(kind, Wc, nx, ny, inlet, kc);
-        prim<T, FAST>(WL, kc.gm1, kc.half, PL);
-        prim<T, FAST>(WR, kc.gm1, kc.half, PR);
-      }
+      const V4<T> WL = Wc;
+      const V4<T> WR = (kind == K_INTERIOR) ? Win[s.off + (long long)nbk[k] * s.B + b]
+                                            : ghost_cons<T, FAST>(kind, Wc, nx, ny, inlet, kc);
+      prim<T, FAST>(WL, kc.gm1, kc.half, PL);
+      prim<T, FAST>(WR, kc.gm1, kc.half, PR);
       T F[4];
       if (FLUX == 0) {
         hllc<T, FAST>(WL, PL, WR, PR, nx, ny, kc, F);
@@ -816,7 +1040,7 @@ __global__ void __launch_bounds__(32 * kPatchWarps, MINB) k_flux_patch(const Seg
           const float4 fr = FV[(long long)ko * total + s.off + (long long)j * s.B + b];
           qR[0] = fr.x; qR[1] = fr.y; qR[2] = fr.z; qR[3] = fr.w;
         } else {
-          xr::ghost_prim(kind, Win[gi], nx, ny, inlet, kc, qR);
+          xr::ghost_prim<float>(kind, Win[gi], nx, ny, inlet, kc, qR);
         }
       }
       float F[4];
@@ -838,13 +1062,13 @@ __global__ void __launch_bounds__(32 * kPatchWarps, MINB) k_flux_patch(const Seg
     for (int k = 0; k < 3; ++k) {
       const float4 f = G[lc][k][lane];
       const float F[4] = {f.x, f.y, f.z, f.w};
-      xr::accumulate(k, gk[G_S0 + k], F, acc);
+      xr::accumulate<float>(k, gk[G_S0 + k], F, acc);
     }
     const float sig = xr::mul(cs.strength[g], gk[G_BLEND3]);
     const float dt = LOCALDT ? dt_local[gi] : cs.dt[g];
     const float4 W0 = (STAGE == ST_FIRST) ? Wc : Wbase[gi];
     float R0;
-    const float4 o = xr::cell_update<STAGE>(acc, gk[G_AREA], sig, inlet, Wc, W0, dt, kc.half, &R0);
+    const float4 o = xr::cell_update4<STAGE, float>(acc, gk[G_AREA], sig, inlet, Wc, W0, dt, kc.half, &R0);
     if (STAGE == ST_FIRST && res_out != nullptr) res_out[gi] = R0;
     Wout[gi] = o;
   }

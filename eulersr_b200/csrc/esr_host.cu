@@ -22,6 +22,7 @@
 
 #include "esr_device.cuh"
 #include "esr_faithful.h"
+#include "esr_stage.cuh"
 #include "esr_internal.h"
 
 namespace {
@@ -112,7 +113,7 @@ struct SolverT : SolverBase {
   int block = 128;
 
   struct MeshDev {
-    HostMesh own;            // the solver's copy: the caller may destroy its mesh
+    std::shared_ptr<const HostMesh> own;   // shared with the handle, which the caller may destroy
     const HostMesh* hm = nullptr;
     DevBuf<T> geo;
     DevBuf<int4> nbr;
@@ -121,6 +122,12 @@ struct SolverT : SolverBase {
     DevBuf<LsqRef> lsq;  // reference-fidelity float32: per-call least-squares data
     DevBuf<int> patch;   // first cell of every patch (+ n_cells)
     DevBuf<int> inv;  // caller cell -> solver cell
+    DevBuf<TileHead> tile_head;   // fused stage kernel: see TileSet
+    DevBuf<int> tile_list;
+    DevBuf<StageCell<T>> tile_cells;
+    DevBuf<StageOwn<T>> tile_own;
+    DevBuf<StageFace<T>> tile_faces;
+    DevBuf<StageGhost<T>> tile_ghosts;
     int B = 0, case0 = 0;
     long long off = 0;
   };
@@ -140,6 +147,12 @@ struct SolverT : SolverBase {
   bool use_patch = false;
   // second register budget of each fast float32 kernel (autotuned)
   bool k1_alt = false, k2_alt = false, kp_alt = false;
+  // MUSCL stages by the fused kernel (esr_stage.cuh); the separate K1 / K2
+  // remain for fast float32 HLLC at launch shapes that ask for them
+  bool fused = false;
+  DevBuf<int4> d_sblk;   // several meshes: (segment, tile, first slot) per block
+  StageLaunch<T> stage{};
+  bool muscl() const { return P.reconstruction == ESR_RECON_MUSCL; }
   // K2 per cell for a batch's tail: once few cases run, a patch block's lanes
   // (one per slot of a 32-slot group) are mostly idle while the per-cell K2
   // maps its threads onto the live slots alone; both give the same bits
@@ -259,8 +272,8 @@ struct SolverT : SolverBase {
     int max_cells = 0;
     for (int m = 0; m < nm; ++m) {
       auto md = std::make_unique<MeshDev>();
-      md->own = ms[m]->hm;
-      md->hm = &md->own;
+      md->own = ms[m]->host;
+      md->hm = md->own.get();
       md->B = slots[m];
       md->case0 = case0;
       md->off = off;
@@ -292,6 +305,7 @@ struct SolverT : SolverBase {
     if (block != 64 && block != 128 && block != 256)
       return fail(ESR_ERR_ARG, "solver: block_size must be 0, 64, 128, 256 or ESR_BLOCK_PATCHES");
     // upload meshes
+    choose_tiles(nm, sms);
     std::vector<Seg<T>> hsegs;
     std::vector<int> hseg_of(n_slots), hslot_of(n_slots), hnc(n_slots);
     for (int m = 0; m < nm; ++m) {
@@ -341,6 +355,7 @@ struct SolverT : SolverBase {
       s.lsq = md.lsq.p;
       s.patch_start = md.patch.p;
       s.n_patches = (int)hm.patch_start.size() - 1;
+      if (muscl()) ESR_TRY(upload_tiles(md, s, g));
       ESR_TRY(set_divider(s));
       h_live_full.push_back(make_int4(s.B, (int)s.b_magic, s.b_shift, 0));
       hsegs.push_back(s);
@@ -354,6 +369,7 @@ struct SolverT : SolverBase {
     hseg0 = hsegs[0];
     ESR_TRY(build_blocks(block));
     ESR_TRY(build_patch_blocks());
+    if (muscl()) ESR_TRY(build_stage_blocks());
     ESR_TRY(d_case_seg.alloc(n_slots));
     ESR_TRY(d_case_slot.alloc(n_slots));
     ESR_TRY(d_ncells.alloc(n_slots));
@@ -364,7 +380,6 @@ struct SolverT : SolverBase {
     ESR_TRY(W.alloc(total));
     ESR_TRY(Wa.alloc(total));
     ESR_TRY(Wref.alloc(total));
-    if (P.reconstruction == ESR_RECON_MUSCL) ESR_TRY(FV.alloc(3 * total));
     if (P.dt_mode == ESR_DT_LOCAL) ESR_TRY(dt_local.alloc(total));
     if (P.stop_rule == ESR_STOP_DENSITY_L2) ESR_TRY(res.alloc(total));
     ESR_CUDA(cudaMemsetAsync(W.p, 0, total * sizeof(V), stream));
@@ -397,6 +412,10 @@ struct SolverT : SolverBase {
     ESR_CUDA(cudaMemsetAsync(inlet.p, 0, n_slots * sizeof(V), stream));
     hcase_index.assign(n_slots, -1);
     ESR_CUDA(cudaStreamSynchronize(stream));
+    if (p->block_size != 0 && patch_eligible()) {   // a launch shape was asked for
+      fused = false;
+      ESR_TRY(FV.reserve(3 * total));
+    }
     if (p->block_size == 0) ESR_TRY(autotune());
     return ESR_OK;
   }
@@ -430,6 +449,133 @@ struct SolverT : SolverBase {
     return ESR_OK;
   }
 
+  // Tile size and slots per block of the fused stage kernel. Eight slots of
+  // one cell are 128 B: full lines from memory and conflict-free shared
+  // reads (four in float64). Bigger tiles recompute fewer ring cells (1.44
+  // times the tile's own reconstructions at 64 cells, 1.6 at 32), but a small
+  // solve needs blocks: it is latency that bounds it.
+#ifndef ESR_TILE_CELLS
+#define ESR_TILE_CELLS 64
+#endif
+  int tile_cells = ESR_TILE_CELLS;
+  void choose_tiles(int nm, int sms) {
+    long long blocks = 0;
+    for (int m = 0; m < nm; ++m) {
+      const int w = 1 << slot_shift_of(meshes[m]->B);
+      blocks += (long long)((meshes[m]->hm->n_cells + tile_cells - 1) / tile_cells) * ((meshes[m]->B + w - 1) / w);
+    }
+    if (blocks < 2 * sms) tile_cells = std::min(tile_cells, 32);
+  }
+  static int slot_shift_of(int B) {
+    int sh = 0;
+    while ((1 << sh) < B && (1 << sh) * sizeof(V) < 128) ++sh;
+    return sh;
+  }
+  int upload_tiles(MeshDev& md, Seg<T>& s, const std::vector<T>& g) {
+    const bool canon = !faithful();
+    const std::shared_ptr<const TileSet> shared = tiles_of(*md.hm, tile_cells, canon, sizeof(T) == 8);
+    const TileSet& ts = *shared;
+    auto geo = [&](int c) { return g.data() + (size_t)c * G_COUNT; };
+    std::vector<StageCell<T>> cells(ts.cells.size());
+    for (size_t i = 0; i < cells.size(); ++i) {
+      const TileCell& c = ts.cells[i];
+      for (int k = 0; k < 3; ++k) { cells[i].nbr[k] = c.nbr[k]; cells[i].slot[k] = c.slot[k]; }
+      cells[i].kinds = c.kinds;
+      std::copy(geo(c.cell) + 12, geo(c.cell) + 24, cells[i].gc);
+    }
+    std::vector<StageOwn<T>> own;
+    own.reserve(md.hm->n_cells);
+    for (const TileHead& h : ts.head)
+      for (int i = 0; i < h.n_own; ++i) {
+        const int c = ts.list[h.list + i];
+        const T* q = geo(c);
+        own.push_back(StageOwn<T>{c, {q[G_S0], q[G_S1], q[G_S2]}, q[G_AREA], q[G_BLEND3],
+                                  {q[G_N0X], q[G_N0Y], q[G_N1X], q[G_N1Y], q[G_N2X], q[G_N2Y]}});
+      }
+    std::vector<StageFace<T>> faces(ts.faces.size());
+    for (size_t i = 0; i < faces.size(); ++i) {
+      const TileFace& f = ts.faces[i];
+      const T* n = geo(f.cell) + 2 * f.edge;
+      faces[i] = StageFace<T>{n[0], n[1], (uint32_t)f.left | (uint32_t)f.right << 16, f.kind};
+    }
+    std::vector<StageGhost<T>> ghosts(ts.ghosts.size());
+    for (size_t i = 0; i < ghosts.size(); ++i) {
+      const TileGhost& w = ts.ghosts[i];
+      const T* n = geo(w.cell) + 2 * w.edge;
+      ghosts[i] = StageGhost<T>{n[0], n[1], w.cell, w.kind};
+    }
+    auto up = [&](auto& buf, const auto& v) -> int {
+      using E = typename std::decay_t<decltype(v)>::value_type;
+      ESR_TRY(buf.alloc(std::max<size_t>(v.size(), 1)));
+      if (!v.empty()) ESR_CUDA(cudaMemcpy(buf.p, v.data(), v.size() * sizeof(E), cudaMemcpyHostToDevice));
+      return ESR_OK;
+    };
+    ESR_TRY(up(md.tile_head, ts.head));
+    ESR_TRY(up(md.tile_list, ts.list));
+    ESR_TRY(up(md.tile_cells, cells));
+    ESR_TRY(up(md.tile_own, own));
+    ESR_TRY(up(md.tile_faces, faces));
+    ESR_TRY(up(md.tile_ghosts, ghosts));
+    s.tile_head = md.tile_head.p;
+    s.tile_list = md.tile_list.p;
+    s.tile_cells = md.tile_cells.p;
+    s.tile_own = md.tile_own.p;
+    s.tile_faces = md.tile_faces.p;
+    s.tile_ghosts = md.tile_ghosts.p;
+    s.slot_shift = slot_shift_of(md.B);
+    max_p = std::max(max_p, ts.max_rows);
+    max_fv = std::max(max_fv, ts.max_slots);
+    max_own = std::max(max_own, ts.max_own);
+    max_shift = std::max(max_shift, s.slot_shift);
+    n_tiles.push_back(ts.n_tiles);
+    return ESR_OK;
+  }
+  int max_p = 0, max_fv = 0, max_own = 0, max_shift = 0;
+  std::vector<int> n_tiles;
+  // grid of the fused kernel: every tile x groups of slots, the groups of one
+  // tile next to each other (their state rows are)
+  int build_stage_blocks() {
+    stage.map.segs = d_segs.p;
+    stage.map.seg0 = hseg0;
+    std::vector<int4> h;
+    long long blocks = 0;
+    const bool packed = patch_eligible() && max_shift >= 1;
+    for (int m = 0; m < (int)meshes.size(); ++m) {
+      const int w = 1 << (packed ? max_shift : slot_shift_of(meshes[m]->B)), groups = (meshes[m]->B + w - 1) / w;
+      blocks += (long long)n_tiles[m] * groups;
+      stage.map.groups = groups;
+      if (meshes.size() > 1)
+        for (int t = 0; t < n_tiles[m]; ++t)
+          for (int q = 0; q < groups; ++q) h.push_back(make_int4(m, t, q * w, 0));
+    }
+    if (blocks > INT_MAX) return fail(ESR_ERR_ARG, "solver: too many tiles x slot groups");
+    if (meshes.size() > 1) {
+      ESR_TRY(d_sblk.alloc(h.size()));
+      ESR_CUDA(cudaMemcpy(d_sblk.p, h.data(), h.size() * sizeof(int4), cudaMemcpyHostToDevice));
+      stage.map.groups = 0;
+    }
+    stage.map.blk = d_sblk.p;
+    stage.blocks = (int)blocks;
+    stage.threads = (max_own << max_shift) <= 64 ? 128 : kStageThreads<T>;
+    // pairs of slots once any mesh has two: the packed kernel (fast float32
+    // HLLC), whose blocks all cover the widest mesh's number of slots
+    stage.pairs = patch_eligible() && max_shift >= 1 ? max_shift - 1 : -1;
+    const int rows = stage.pairs >= 0 ? stage.pairs : max_shift;
+    stage.p_rows = max_p << rows;
+    stage.fv_rows = max_fv << rows;
+    const int fx_rows = faithful() ? (3 * max_own) << rows : 0;
+    stage.smem = (stage.p_rows + stage.fv_rows + fx_rows) * (int)sizeof(V) * (stage.pairs >= 0 ? 2 : 1);
+    if (stage.smem > kStageSmemMax) return fail(ESR_ERR_STATE, "stage tiles need more shared memory than a block has");
+    const bool rus = P.flux == ESR_FLUX_RUSANOV, local = P.dt_mode == ESR_DT_LOCAL;
+    if (faithful()) {
+      if constexpr (sizeof(T) == 4) ESR_CUDA(faithful_allow_stage(rus, local));
+    } else {
+      ESR_CUDA((allow_stage<T, kF>(rus, local)));
+    }
+    fused = true;
+    return ESR_OK;
+  }
+
   // block table of K2 by patches: every patch of every mesh x groups of 32 slots
   int build_patch_blocks() {
     std::vector<int4> h;
@@ -460,7 +606,7 @@ struct SolverT : SolverBase {
   // cells and slots), so a second solver of the same shape skips the timing.
   struct TuneChoice {
     int block = 256;
-    bool patches = false, k1 = false, k2 = false, kp = false;
+    bool patches = false, k1 = false, k2 = false, kp = false, fused = false;
   };
   struct TuneEntry {
     TuneChoice choice;
@@ -488,6 +634,8 @@ struct SolverT : SolverBase {
   int apply_choice(const TuneChoice& c) {
     ESR_TRY(build_blocks(c.block));
     use_patch = c.patches && patch_eligible();
+    fused = muscl() && (c.fused || !patch_eligible());
+    if (muscl() && !fused) ESR_TRY(FV.reserve(3 * total));
     k1_alt = c.k1;
     k2_alt = c.k2;
     kp_alt = c.kp;
@@ -516,6 +664,7 @@ struct SolverT : SolverBase {
   esr_tuning tuning{};
   TuneChoice chosen;
   int autotune() {
+    if (muscl() && !patch_eligible()) return ESR_OK;   // the fused stage kernel alone: nothing to choose
     const std::string key = tune_key();
     {
       std::lock_guard<std::mutex> lock(tune_mutex());
@@ -556,8 +705,7 @@ struct SolverT : SolverBase {
       tuning.step_ms[i] = ms;
     }
     const int best_blk = best_c.block;
-    const bool muscl = P.reconstruction == ESR_RECON_MUSCL;
-    if (fast_float() && muscl && P.flux == ESR_FLUX_HLLC) {   // K2 per cell, second budget
+    if (patch_eligible()) {   // K2 per cell, second budget
       TuneChoice c;
       c.block = best_blk;
       c.k2 = true;
@@ -574,13 +722,22 @@ struct SolverT : SolverBase {
       c.kp = true;
       ESR_TRY(consider(c));
     }
-    if (fast_float() && muscl) {   // K1, second budget, with the best K2
+    if (patch_eligible()) {   // K1, second budget, with the best K2
       TuneChoice c = best_c;
       c.k1 = true;
       ESR_TRY(consider(c));
     }
-    launches = before;
     chosen = best_c;
+    // The fused stage kernel runs unless a launch shape is asked for: it was
+    // faster than the best separate pair at every size measured (us per step,
+    // 1 slot of 1,450 cells 9 against 25, 32 x 1,810 cells 14 against 26,
+    // 32 x 25,968 62 against 76, 256 x 25,049 386 against 456). The record
+    // above serves callers that set a shape.
+    if (patch_eligible()) {
+      chosen.fused = true;
+      ESR_TRY(FV.alloc(0));   // the face states of the separate kernels
+    }
+    launches = before;
     ESR_TRY(apply_choice(chosen));
     tuning.block_size = chosen.block;
     tuning.k2_patches = use_patch ? 1 : 0;
@@ -690,14 +847,12 @@ struct SolverT : SolverBase {
   }
   template <int STAGE>
   void flux_dispatch(const V* win, const V* wbase, V* wout, const Cases<T>& cs, int pos) {
-    const bool muscl = P.reconstruction == ESR_RECON_MUSCL;
     const bool local = P.dt_mode == ESR_DT_LOCAL;
     const bool rus = P.flux == ESR_FLUX_RUSANOV;
     if constexpr (sizeof(T) == 4) {
-      if (faithful()) {
+      if (faithful()) {   // constant reconstruction
         tap_begin(1);
-        faithful_flux(STAGE, bmap(), win, wbase, wout, FV.p, total, cs, kc, pos, dt_local.p, res.p, rus, muscl, local,
-                      n_blk, block, stream);
+        faithful_flux(STAGE, bmap(), win, wbase, wout, cs, kc, pos, dt_local.p, res.p, rus, local, n_blk, block, stream);
         tap_end();
         ++launches;
         return;
@@ -710,37 +865,61 @@ struct SolverT : SolverBase {
         ++launches;
         return;
       }
-    }
-#define ESR_FLUX_CASE(F, M, L) if (rus == (F == 1) && muscl == M && local == L) { launch_flux<F, M, STAGE, L>(win, wbase, wout, cs, pos); return; }
-    ESR_FLUX_CASE(0, true, false) ESR_FLUX_CASE(0, true, true) ESR_FLUX_CASE(0, false, false) ESR_FLUX_CASE(0, false, true)
-    ESR_FLUX_CASE(1, true, false) ESR_FLUX_CASE(1, true, true) ESR_FLUX_CASE(1, false, false) ESR_FLUX_CASE(1, false, true)
-#undef ESR_FLUX_CASE
-  }
-  void recon(const V* w, const Cases<T>& cs, int pos, bool write_dt) {
-    const bool muscl = P.reconstruction == ESR_RECON_MUSCL;
-    if (!muscl && !write_dt) return;   // constant reconstruction needs K1 only for the local dt
-    if constexpr (sizeof(T) == 4) {
-      if (faithful()) {
-        tap_begin(0);
-        faithful_recon(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p, muscl, write_dt, n_blk, block, stream);
-        tap_end();
-        ++launches;
+      if (muscl()) {   // fast HLLC; every other MUSCL solve runs fused
+        if (local) launch_flux<0, true, STAGE, true>(win, wbase, wout, cs, pos);
+        else launch_flux<0, true, STAGE, false>(win, wbase, wout, cs, pos);
         return;
       }
     }
-    if (!muscl) {
+#define ESR_FLUX_CASE(F, L) if (rus == (F == 1) && local == L) { launch_flux<F, false, STAGE, L>(win, wbase, wout, cs, pos); return; }
+    ESR_FLUX_CASE(0, false) ESR_FLUX_CASE(0, true) ESR_FLUX_CASE(1, false) ESR_FLUX_CASE(1, true)
+#undef ESR_FLUX_CASE
+  }
+  void recon(const V* w, const Cases<T>& cs, int pos, bool write_dt) {
+    if (!muscl() && !write_dt) return;   // constant reconstruction needs K1 only for the local dt
+    if (!muscl()) {
+      if constexpr (sizeof(T) == 4) {
+        if (faithful()) {
+          tap_begin(0);
+          faithful_local_dt(bmap(), w, cs, kc, pos, dt_local.p, n_blk, block, stream);
+          tap_end();
+          ++launches;
+          return;
+        }
+      }
       k_recon<T, kF, false, true><<<n_blk, block, 0, stream>>>(bmap(), w, nullptr, 0, cs, kc, pos, dt_local.p);
       ++launches;
       return;
     }
-    tap_begin(0);
-    if (write_dt) {   // the local-dt K1 keeps its one budget
-      k_recon<T, kF, true, true><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
-    } else if (sizeof(T) == 4 && k1_alt) {
-      k_recon<T, kF, true, false, (sizeof(T) == 4 ? ESR_K1_MINB_ALT : 0)><<<n_blk, block, 0, stream>>>(
-          bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
+    if constexpr (sizeof(T) == 4) {
+      tap_begin(0);
+      if (write_dt)   // the local-dt K1 keeps its one budget
+        k_recon<T, kF, true, true><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
+      else if (k1_alt)
+        k_recon<T, kF, true, false, ESR_K1_MINB_ALT><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos,
+                                                                                  dt_local.p);
+      else
+        k_recon<T, kF, true, false><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
+      tap_end();
+      ++launches;
+    }
+  }
+  // one Runge-Kutta stage of every live slot: wout from win (and wbase, the
+  // state the step started from)
+  template <int STAGE>
+  void run_stage(const V* win, const V* wbase, V* wout, const Cases<T>& cs, int pos) {
+    const bool local = P.dt_mode == ESR_DT_LOCAL, rus = P.flux == ESR_FLUX_RUSANOV;
+    if (!fused) {
+      recon(win, cs, pos, local && STAGE == ST_FIRST);
+      flux_dispatch<STAGE>(win, wbase, wout, cs, pos);
+      return;
+    }
+    tap_begin(1);
+    if (faithful()) {
+      if constexpr (sizeof(T) == 4)
+        faithful_stage(stage, rus, STAGE, local, win, wbase, wout, cs, kc, pos, dt_local.p, res.p, stream);
     } else {
-      k_recon<T, kF, true, false><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
+      launch_stage<T, kF>(stage, rus, STAGE, local, win, wbase, wout, cs, kc, pos, dt_local.p, res.p, stream);
     }
     tap_end();
     ++launches;
@@ -759,38 +938,23 @@ struct SolverT : SolverBase {
   }
   // one time step of every live slot, step index `pos` inside the chunk
   void step_kernels(const Cases<T>& cs, int pos) {
-    const bool local = P.dt_mode == ESR_DT_LOCAL;
-    switch (P.time_scheme) {
-      case ESR_TIME_EE:
-        recon(W.p, cs, pos, local);
-        flux_dispatch<ST_FIRST>(W.p, nullptr, Wa.p, cs, pos);
-        k_commit<T><<<n_blk, block, 0, stream>>>(d_segs.p, d_blk.p, Wa.p, W.p, cs, pos);
-        ++launches;
-        break;
-      case ESR_TIME_RK2:
-        recon(W.p, cs, pos, local);
-        flux_dispatch<ST_FIRST>(W.p, nullptr, Wa.p, cs, pos);
-        recon(Wa.p, cs, pos, false);
-        flux_dispatch<ST_RK2_SECOND>(Wa.p, W.p, W.p, cs, pos);
-        break;
-      default:  // SRK2
-        recon(W.p, cs, pos, local);
-        flux_dispatch<ST_FIRST>(W.p, nullptr, Wa.p, cs, pos);
-        recon(Wa.p, cs, pos, false);
-        flux_dispatch<ST_SRK2_SECOND>(Wa.p, W.p, W.p, cs, pos);
-        break;
+    run_stage<ST_FIRST>(W.p, nullptr, Wa.p, cs, pos);
+    if (P.time_scheme == ESR_TIME_EE) {
+      k_commit<T><<<n_blk, block, 0, stream>>>(d_segs.p, d_blk.p, Wa.p, W.p, cs, pos);
+      ++launches;
+    } else if (P.time_scheme == ESR_TIME_RK2) {
+      run_stage<ST_RK2_SECOND>(Wa.p, W.p, W.p, cs, pos);
+    } else {  // SRK2
+      run_stage<ST_SRK2_SECOND>(Wa.p, W.p, W.p, cs, pos);
     }
   }
   // One step of the slots active in `cs` written to scratch instead of W
   // (the residual probe); returns the buffer that holds the stepped state.
   V* probe_kernels(const Cases<T>& cs) {
-    const bool local = P.dt_mode == ESR_DT_LOCAL;
-    recon(W.p, cs, 0, local);
-    flux_dispatch<ST_FIRST>(W.p, nullptr, Wa.p, cs, 0);
+    run_stage<ST_FIRST>(W.p, nullptr, Wa.p, cs, 0);
     if (P.time_scheme == ESR_TIME_EE) return Wa.p;
-    recon(Wa.p, cs, 0, false);
-    if (P.time_scheme == ESR_TIME_RK2) flux_dispatch<ST_RK2_SECOND>(Wa.p, W.p, Wp.p, cs, 0);
-    else flux_dispatch<ST_SRK2_SECOND>(Wa.p, W.p, Wp.p, cs, 0);
+    if (P.time_scheme == ESR_TIME_RK2) run_stage<ST_RK2_SECOND>(Wa.p, W.p, Wp.p, cs, 0);
+    else run_stage<ST_SRK2_SECOND>(Wa.p, W.p, Wp.p, cs, 0);
     return Wp.p;
   }
   void check_point(int pos) {
@@ -876,11 +1040,10 @@ struct SolverT : SolverBase {
     return ESR_OK;
   }
   int64_t chunk_launches(bool run, int len) {
-    const bool muscl = P.reconstruction == ESR_RECON_MUSCL;
-    const bool local = P.dt_mode == ESR_DT_LOCAL;
+    const bool k1 = muscl() && !fused, k1_dt = !muscl() && P.dt_mode == ESR_DT_LOCAL;
     int per_step;
-    if (P.time_scheme == ESR_TIME_EE) per_step = 2 + ((muscl || local) ? 1 : 0);
-    else per_step = 2 + (muscl ? 2 : (local ? 1 : 0));
+    if (P.time_scheme == ESR_TIME_EE) per_step = 2 + ((k1 || k1_dt) ? 1 : 0);
+    else per_step = 2 + (k1 ? 2 : (k1_dt ? 1 : 0));
     int64_t n = (int64_t)per_step * len + 1;
     if (run) {
       const int ce = std::max(1, P.check_every);
@@ -1760,7 +1923,7 @@ struct SolverT : SolverBase {
       cudaError_t e = cudaGraphInstantiate(&pb.gexec, graph, 0);
       cudaGraphDestroy(graph);
       if (e != cudaSuccess) { pb.gexec = nullptr; return fail(ESR_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)); }
-      if (use_patch && n_pblk > 0) {   // the tail form: K2 per cell
+      if (use_patch && !fused && n_pblk > 0) {   // the tail form: K2 per cell
         ESR_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         tail_cell_k2 = true;
         const int64_t b2 = launches;
@@ -1799,7 +1962,7 @@ struct SolverT : SolverBase {
       }
       if (rc == ESR_OK) {
         // the done counter and, for K2 by patches, each mesh's live slots
-        const bool watch = use_patch && n_pblk > 0;
+        const bool watch = use_patch && !fused && n_pblk > 0;
         h_live_poll.resize(meshes.size());
         cudaError_t e = cudaMemcpyAsync(&pb.done, pb.Bp->n_done.p, sizeof(int), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess && watch)

@@ -1,5 +1,6 @@
 // esr_layout.h -- data-layout constants shared by host and device code.
 #pragma once
+#include <stdint.h>
 
 namespace esr {
 
@@ -37,6 +38,17 @@ static_assert(sizeof(LsqRef) == 64, "one 64-byte record per cell");
 #define ESR_PATCH_CELLS 24
 #endif
 constexpr int kPatchCells = ESR_PATCH_CELLS;
+
+// Tiles of the fused stage kernel (esr_stage.cuh). A tile owns a compact
+// group of cells; its block also reconstructs the ring of cells around them
+// and reads the state of the ring around that.
+constexpr uint16_t kNoSlot = 0xFFFF;
+struct TileHead {
+  int list, cells, ghosts, faces;   // first entry of the tile in each table (own cells: entry `own`)
+  int own, n_own, n1, n2;           // own cells, own + ring 1, own + ring 1 + ring 2
+  int n_ghosts, n_faces, pad[2];
+};
+static_assert(sizeof(TileHead) == 48, "three 16-byte loads");
 
 // n / d without an integer divide for 0 <= n < 2^31: q = (umulhi(n, magic) +
 // n) >> shift with shift = ceil(log2 d), magic = floor(2^32 (2^shift - d) / d)

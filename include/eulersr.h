@@ -298,8 +298,8 @@ int esr_kernel_launches(const esr_solver* solver, int64_t* n);
  * without graphs, CUDA events recorded on the solver's stream around every
  * launch. The steps advance the state like esr_step. */
 typedef struct esr_kernel_times {
-    double recon_ms;          /* K1: gradient, limiter, MUSCL face states */
-    double flux_ms;           /* K2: face fluxes, residual, stage update */
+    double recon_ms;          /* K1: gradient, limiter, MUSCL face states (0 with the fused stage kernel) */
+    double flux_ms;           /* K2: face fluxes, residual, stage update; or the whole fused stage */
     double other_ms;          /* bookkeeping kernels */
     int32_t recon_launches;
     int32_t flux_launches;
@@ -308,9 +308,14 @@ typedef struct esr_kernel_times {
 } esr_kernel_times;
 int esr_profile_step(esr_solver* solver, int32_t nsteps, esr_kernel_times* out);
 
-/* The autotuner's record: with esr_params.block_size = 0 the solver times one
- * full step of all its slots for each launch shape at creation and keeps the
- * fastest (no reference counterpart: XLA picks launch shapes). Shapes: the
+/* The record of launch shapes: MUSCL solves run each Runge-Kutta stage as one
+ * fused kernel. A float32 fast-fidelity HLLC solver can also run it as the
+ * separate kernels K1 (reconstruction) and K2 (fluxes), at a shape given by
+ * esr_params.block_size or esr_solver_set_shape; with block_size = 0 it times
+ * one full step of all its slots for each of those shapes at creation and
+ * records them, with the fastest in the fields below (no reference
+ * counterpart: XLA picks launch shapes). Constant reconstruction has no fused
+ * form: its solver keeps the fastest block size. Shapes: the
  * cell kernels at 64, 128 and 256 threads per block; at the best of those,
  * where the float32 fast kernels run, K2's second register budget, K2 by
  * patches at both of its budgets (float32 fast fidelity, HLLC + MUSCL), and
@@ -353,7 +358,7 @@ int esr_solver_set_shape(esr_solver* solver, const esr_tuning_variant* shape);
 /* Solve n_cases cases through the solver's slots: every slot retired by the
  * stop rule is refilled in place with the next queued case. init_fields[i]
  * is a (n_cells,4) conserved warm start or NULL; final_states[i] receives the
- * final state when non-NULL. results has n_cases entries. A solver on K2 by
+ * final state when non-NULL. results has n_cases entries. A solver set to K2 by
  * patches runs the batch's tail (every mesh down to 24 running cases or
  * fewer) with the per-cell K2, whose threads cover the running slots alone;
  * the results are the same. */

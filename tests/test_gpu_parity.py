@@ -551,3 +551,33 @@ def test_solver_refuses_cells_times_slots_beyond_2_31(diamond02):
     with pytest.raises(EsrError) as e:
         Solver(diamond02, slots, precision='f32', block_size=128)
     assert e.value.code == 1 and "2^31" in str(e.value)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("slots", [1, 2, 3, 5, 8, 9, 17])
+@pytest.mark.parametrize("dt_mode", ["global", "local"])
+def test_fused_stage_equals_separate_kernels(diamond02, naca02, slots, dt_mode):
+    """The fused stage kernel (one slot: k_stage, more: k_stage_pair with two
+    slots per thread) gives the bits of the separate reconstruction and flux
+    kernels, on one mesh and on two, at slot counts around its groups of 2, 4
+    and 8 (the last pair half full, the last group partly empty), with a slot
+    left idle."""
+    from eulersr_b200.solver import Solver, FlowCase, DeviceMesh
+    rng = np.random.default_rng(slots)
+    for meshes in ([naca02], [diamond02, naca02]):
+        dms = [DeviceMesh(m) for m in meshes]
+        n = slots * len(dms)
+        states = []
+        for block in (0, 128):
+            s = Solver(dms, slots, precision="f32", dt_mode=dt_mode, block_size=block)
+            r = np.random.default_rng(slots)
+            for g in range(n):
+                if n > 2 and g == 1:
+                    continue   # an idle slot inside a group
+                s.set_case(g, FlowCase(mach=float(r.uniform(0.7, 3.0)), aoa_deg=float(r.uniform(-5, 5)), tf=1.0,
+                                       dtype=np.float32))
+            s.step(7)
+            states.append([s.get_state(g) for g in range(n)])
+            s.close()
+        for g, (a, b) in enumerate(zip(*states)):
+            assert np.all(np.isfinite(a)) and np.array_equal(a, b), (slots, g)
