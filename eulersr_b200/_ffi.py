@@ -95,6 +95,12 @@ class TuningVariant(C.Structure):
                 "k1_minb": int(self.k1_minb), "k2_minb": int(self.k2_minb), "step_ms": float(self.step_ms)}
 
 
+class Reduction(C.Structure):
+    """esr_reduction"""
+    _fields_ = [("part", C.c_void_p), ("out", C.c_void_p), ("stride", C.c_int64), ("n", C.c_int64),
+                ("splits", C.c_int32), ("reserved", C.c_int32)]
+
+
 class Tuning(C.Structure):
     _fields_ = [("block_size", C.c_int32), ("n_candidates", C.c_int32), ("candidates", C.c_int32 * 4),
                 ("k2_patches", C.c_int32), ("cached", C.c_int32), ("step_ms", C.c_double * 4),
@@ -181,6 +187,7 @@ _SIGS = {
     "esr_mlp_loss": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p,
                                C.c_void_p]),
     "esr_reduce_splits": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
+    "esr_reduce_many": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p]),
     "esr_colsum_bf16": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]),
     "esr_adamw": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float,
                             C.c_float, C.c_float, C.c_float, C.c_int32, C.c_void_p, C.c_void_p]),

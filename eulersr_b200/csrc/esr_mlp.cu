@@ -12,20 +12,23 @@
 //   EPI_FWD   z = acc + bias; out = residual + relu(z)   (z kept for backward)
 //   EPI_BWD   dh = acc + dh_next; dz_prev = dh * (z_prev > 0)
 // The 4-wide head, the loss, AdamW and the fixed-order reductions are plain
-// SIMT kernels. Every reduction is deterministic (no atomics).
+// SIMT kernels, bound by reading their operands once. Every reduction is deterministic (no atomics).
 #include <cuda_bf16.h>
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 
 #include "esr_internal.h"
+#include "esr_mlp.cuh"
 
 namespace {
 
 using bf16 = __nv_bfloat16;
+using namespace esr;
 
 constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3, THREADS = 256;
 constexpr int PAD = 8;
@@ -33,6 +36,40 @@ constexpr int LD_K = BK + PAD;     // row stride of K-contiguous tiles (elements
 constexpr int LD_MN = BM + PAD;    // row stride of M/N-contiguous tiles
 
 enum { EPI_F32 = 0, EPI_FWD = 1, EPI_BWD = 2 };
+
+// Eight consecutive BF16 values, as one 16-byte access (VEC) or one by one
+// where a caller's buffer is not aligned for it.
+template <bool VEC>
+__device__ __forceinline__ void load8(const bf16* p, float v[8]) {
+  if (VEC) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __bfloat162float(p[i]);
+  }
+}
+template <bool VEC>
+__device__ __forceinline__ void store8(bf16* p, const float v[8]) {
+  if (VEC) {
+    unsigned w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const unsigned*>(&b);
+    }
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i] = __float2bfloat16(v[i]);
+  }
+}
+inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 struct Epi {
   const float* bias;     // FWD: per-column bias
@@ -42,6 +79,7 @@ struct Epi {
   bf16* out1;            // FWD: z; BWD: dz_prev
   int ldo;               // leading dimension of res/aux/out0/out1
   long long split_stride;// F32: elements between split-K partial tiles
+  bool vec;              // every pointer and row of this epilogue is 16-byte aligned
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -215,18 +253,154 @@ __global__ void k_head_fwd(const bf16* __restrict__ H, int rows, int K, const fl
   if (lane < 4) y[(size_t)r * 4 + lane] = s[lane] + b[lane] + (base ? base[(size_t)r * 4 + lane] : 0.f);
 }
 
-// dH[r][k] = sum_j dY[r][j] W[j][k] as BF16, and dz = dH * (z > 0) of the
-// last hidden pre-activation
-__global__ void k_head_bwd_dx(const float* __restrict__ dY, int rows, int K, const float* __restrict__ W,
-                              const bf16* __restrict__ z, bf16* __restrict__ dH, bf16* __restrict__ dZ) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)rows * K) return;
-  const int r = (int)(i / K), k = (int)(i % K);
-  float s = 0.f;
+// The same sums in the same order for 256 columns: a lane keeps its columns
+// (lane + 32 i) of W in registers, a warp walks groups of 4 rows and requests
+// the next group before it sums the current one. Bound by reading H once:
+// 32,768 rows take 13 us, 17 us row by row.
+__global__ void __launch_bounds__(256, 2) k_head_fwd256(const bf16* __restrict__ H, int rows,
+                                                        const float* __restrict__ W, const float* __restrict__ b,
+                                                        const float* __restrict__ base, float* __restrict__ y) {
+  constexpr int R = 4;
+  const int lane = threadIdx.x & 31, step = R * gridDim.x * (blockDim.x >> 5);
+  int r0 = R * (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  bf16 h[R][8], hn[R][8];
+  auto fetch = [&](int r, bf16 v[R][8]) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) s += dY[(size_t)r * 4 + j] * W[j * K + k];
-  dH[i] = __float2bfloat16(s);
-  dZ[i] = __float2bfloat16(__bfloat162float(z[i]) > 0.f ? s : 0.f);
+    for (int q = 0; q < R; ++q)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[q][i] = H[(size_t)min(r + q, rows - 1) * 256 + lane + 32 * i];
+  };
+  fetch(r0, h);
+  float w[4][8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[j][i] = W[j * 256 + lane + 32 * i];
+  const float bias = b[lane & 3];
+  for (; r0 < rows; r0 += step) {
+    fetch(r0 + step, hn);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float v = __bfloat162float(h[q][i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[j] += v * w[j][i];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+      if (lane < 4 && r0 + q < rows) {
+        const float v = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
+        y[(size_t)(r0 + q) * 4 + lane] = v + bias + (base ? base[(size_t)(r0 + q) * 4 + lane] : 0.f);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h[q][i] = hn[q][i];
+  }
+}
+
+// Two consecutive BF16 values, as one 4-byte access (VEC) or one by one.
+template <bool VEC>
+__device__ __forceinline__ __nv_bfloat162 load2(const bf16* p) {
+  if (VEC) return *reinterpret_cast<const __nv_bfloat162*>(p);
+  __nv_bfloat162 v;
+  v.x = p[0];
+  v.y = p[1];
+  return v;
+}
+template <bool VEC>
+__device__ __forceinline__ void store2(bf16* p, float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  if (VEC) {
+    *reinterpret_cast<__nv_bfloat162*>(p) = v;
+  } else {
+    p[0] = v.x;
+    p[1] = v.y;
+  }
+}
+
+// The head's backward over 256 columns, one block per `rows_per_block` rows:
+// dH[r][k] = sum_j dY[r][j] W[j][k] and dZ = dH * (z > 0) as BF16, and the
+// block's partials of dW[j][k] = sum_r dY[r][j] H[r][k] and db[j] = sum_r
+// dY[r][j], summed row by row. A thread owns two columns (their W and dW in
+// registers); dY waits in shared memory and the next kHeadRows rows of H and Z
+// are requested before the current ones are used, since it is the memory that
+// must be kept busy, not the chains over rows. 32,768 rows take 26 us; 102 us
+// as a thread per element and a second kernel that waits for each row.
+constexpr int kHeadRows = 16, kHeadSlab = 256;
+template <bool VEC>
+__global__ void __launch_bounds__(128) k_head_bwd(const float* __restrict__ dY, const bf16* __restrict__ H,
+                                                  const bf16* __restrict__ Z, int rows, const float* __restrict__ W,
+                                                  bf16* __restrict__ dH, bf16* __restrict__ dZ, int rows_per_block,
+                                                  float* __restrict__ part) {
+  constexpr int K = 256;
+  __shared__ float4 sd[kHeadSlab];
+  const int col = threadIdx.x * 2;
+  const int r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
+  float w[4][2], g[4][2], gb[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    w[j][0] = W[j * K + col];
+    w[j][1] = W[j * K + col + 1];
+    g[j][0] = g[j][1] = gb[j] = 0.f;
+  }
+  __nv_bfloat162 h[kHeadRows], z[kHeadRows], hn[kHeadRows], zn[kHeadRows];
+  auto fetch = [&](int r, __nv_bfloat162* hv, __nv_bfloat162* zv) {
+#pragma unroll
+    for (int q = 0; q < kHeadRows; ++q) {
+      const size_t o = (size_t)min(r + q, r1 - 1) * K + col;
+      hv[q] = load2<VEC>(H + o);
+      zv[q] = load2<VEC>(Z + o);
+    }
+  };
+  fetch(r0, h, z);
+  for (int slab = r0; slab < r1; slab += kHeadSlab) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < min(kHeadSlab, r1 - slab); i += blockDim.x) {
+      const float* p = dY + (size_t)(slab + i) * 4;
+      sd[i] = make_float4(p[0], p[1], p[2], p[3]);
+    }
+    __syncthreads();
+    for (int r = slab; r < min(slab + kHeadSlab, r1); r += kHeadRows) {
+      fetch(r + kHeadRows, hn, zn);
+#pragma unroll
+      for (int q = 0; q < kHeadRows; ++q) {
+        if (r + q < r1) {
+          const float4 dv = sd[r + q - slab];
+          const float d[4] = {dv.x, dv.y, dv.z, dv.w};
+          const float h0 = __bfloat162float(h[q].x), h1 = __bfloat162float(h[q].y);
+          float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            s0 += d[j] * w[j][0];
+            s1 += d[j] * w[j][1];
+            g[j][0] += d[j] * h0;
+            g[j][1] += d[j] * h1;
+            gb[j] += d[j];
+          }
+          const size_t o = (size_t)(r + q) * K + col;
+          store2<VEC>(dH + o, s0, s1);
+          store2<VEC>(dZ + o, __bfloat162float(z[q].x) > 0.f ? s0 : 0.f, __bfloat162float(z[q].y) > 0.f ? s1 : 0.f);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kHeadRows; ++q) { h[q] = hn[q]; z[q] = zn[q]; }
+    }
+  }
+  float* p = part + (size_t)blockIdx.x * (4 * K + 4);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    p[j * K + col] = g[j][0];
+    p[j * K + col + 1] = g[j][1];
+  }
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[4 * K + j] = gb[j];
 }
 
 // Per-cell inputs of one case (BF16 rows of `ld` columns, zero padded):
@@ -235,22 +409,22 @@ __global__ void k_head_bwd_dx(const float* __restrict__ dY, int rows, int K, con
 __global__ void k_features(const float* __restrict__ stat5, const float* __restrict__ idw_prim,
                            const float* __restrict__ idw_gradp, int rows, float mach_n, float aoa_n,
                            const float* __restrict__ mu, const float* __restrict__ sig, int ld, bf16* __restrict__ X,
-                           float* __restrict__ base) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  bf16* x = X + (size_t)r * ld;
-  for (int j = 0; j < 5; ++j) x[j] = __float2bfloat16(stat5[(size_t)r * 5 + j]);
-  for (int v = 0; v < 4; ++v) {
-    const float q = (idw_prim[(size_t)r * 4 + v] - mu[v]) / sig[v];
-    x[5 + v] = __float2bfloat16(q);
-    if (base) base[(size_t)r * 4 + v] = q;   // the IDW prediction the MLP corrects
+                           float* __restrict__ base, bool vec) {
+  __shared__ __align__(16) bf16 sh[kFeatureRows][16];
+  const int r = blockIdx.x * kFeatureRows + threadIdx.x;
+  if (r < rows) {
+    float prim[4], gradp[2], q[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) prim[v] = idw_prim[(size_t)r * 4 + v];
+    gradp[0] = idw_gradp[(size_t)r * 2];
+    gradp[1] = idw_gradp[(size_t)r * 2 + 1];
+    feature_row(stat5 + (size_t)r * 5, prim, gradp, mach_n, aoa_n, mu, sig, sh[threadIdx.x], q);
+    if (base)   // the IDW prediction the MLP corrects
+#pragma unroll
+      for (int v = 0; v < 4; ++v) base[(size_t)r * 4 + v] = q[v];
   }
-  const float sp = sig[3] + 1e-8f;
-  x[9] = __float2bfloat16(asinhf(idw_gradp[(size_t)r * 2] / sp));
-  x[10] = __float2bfloat16(asinhf(idw_gradp[(size_t)r * 2 + 1] / sp));
-  x[11] = __float2bfloat16(mach_n);
-  x[12] = __float2bfloat16(aoa_n);
-  for (int j = 13; j < ld; ++j) x[j] = __float2bfloat16(0.f);
+  __syncthreads();
+  store_features(sh, blockIdx.x * kFeatureRows, rows, ld, X, vec);
 }
 
 // normalised primitive prediction -> conserved state (float64 rows), with
@@ -270,45 +444,71 @@ __global__ void k_decode(const float* __restrict__ pred_n, int rows, const float
   W[(size_t)r * 4 + 3] = (double)p / (gamma - 1.0) + 0.5 * (double)rho * ((double)u * u + (double)v * v);
 }
 
-// per-block partials of dW_head[j][k] = sum_r dY[r][j] H[r][k] and db[j] = sum_r dY[r][j]
-__global__ void k_head_bwd_dw(const float* __restrict__ dY, const bf16* __restrict__ H, int rows, int K,
-                              int rows_per_block, float* __restrict__ part) {
-  const int k = threadIdx.x;            // blockDim.x == K (256)
-  const int r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
-  float s[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int r = r0; r < r1; ++r) {
-    const float h = __bfloat162float(H[(size_t)r * K + k]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float d = dY[(size_t)r * 4 + j];
-      s[j] += d * h;
-      sb[j] += d;
-    }
-  }
-  float* p = part + (size_t)blockIdx.x * (4 * K + 4);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) p[j * K + k] = s[j];
-  if (k < 4) p[4 * K + k] = sb[k];
-}
-
-// out[i] = sum_s part[s * stride + i] in split order
-__global__ void k_reduce_splits(const float* __restrict__ part, int splits, long long stride, long long n,
-                                float* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// out[i] = sum_s part[s * stride + i] in split order, for several sets of
+// partials in one launch (a block per 256 outputs of one set). The loads of 16
+// splits are in flight at once: 256 outputs of 128 partials take 3 us, 11 us
+// load by load.
+struct Reduction {
+  const float* part;
+  float* out;
+  long long stride, n;
+  int splits, blocks;    // blocks before this set's
+};
+constexpr int kMaxReductions = 16;
+struct Reductions {
+  Reduction r[kMaxReductions];
+  int n;
+};
+__global__ void __launch_bounds__(256) k_reduce_splits(const __grid_constant__ Reductions q) {
+  int k = 0;
+  while (k + 1 < q.n && (int)blockIdx.x >= q.r[k + 1].blocks) ++k;
+  const Reduction& r = q.r[k];
+  const long long i = (long long)((int)blockIdx.x - r.blocks) * 256 + threadIdx.x;
+  if (i >= r.n) return;
+  const float* p = r.part + i;
   float s = 0.f;
-  for (int z = 0; z < splits; ++z) s += part[(size_t)z * stride + i];
-  out[i] = s;
+  int z = 0;
+  for (; z + 16 <= r.splits; z += 16) {
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = p[(size_t)(z + u) * r.stride];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s += v[u];
+  }
+  for (; z < r.splits; ++z) s += p[(size_t)z * r.stride];
+  r.out[i] = s;
 }
 
-// column sums of a BF16 [rows x C] matrix in fixed row blocks (bias gradients)
-__global__ void k_colsum_part(const bf16* __restrict__ X, int rows, int C, int rows_per_block, float* __restrict__ part) {
-  const int c = blockIdx.y * blockDim.x + threadIdx.x;
+// column sums of a BF16 [rows x C] matrix in fixed row blocks, row by row
+// (bias gradients). A thread owns two columns with 32 rows in flight:
+// 32,768 x 256 (16.8 MB) takes 5 us (as a quarter of one launch), 22 us load by load.
+template <bool VEC>
+__global__ void __launch_bounds__(128) k_colsum_part(const bf16* __restrict__ X, int rows, int C, int rows_per_block,
+                                                     float* __restrict__ part) {
+  constexpr int U = 32;
+  const int c = 2 * (blockIdx.y * blockDim.x + threadIdx.x);
   if (c >= C) return;
   const int r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
-  float s = 0.f;
-  for (int r = r0; r < r1; ++r) s += __bfloat162float(X[(size_t)r * C + c]);
-  part[(size_t)blockIdx.x * C + c] = s;
+  float s0 = 0.f, s1 = 0.f;
+  if (c + 1 < C) {
+    int r = r0;
+    for (; r + U <= r1; r += U) {
+      __nv_bfloat162 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = load2<VEC>(X + (size_t)(r + u) * C + c);
+#pragma unroll
+      for (int u = 0; u < U; ++u) { s0 += __bfloat162float(v[u].x); s1 += __bfloat162float(v[u].y); }
+    }
+    for (; r < r1; ++r) {
+      const __nv_bfloat162 v = load2<VEC>(X + (size_t)r * C + c);
+      s0 += __bfloat162float(v.x);
+      s1 += __bfloat162float(v.y);
+    }
+    part[(size_t)blockIdx.x * C + c + 1] = s1;
+  } else {
+    for (int r = r0; r < r1; ++r) s0 += __bfloat162float(X[(size_t)r * C + c]);
+  }
+  part[(size_t)blockIdx.x * C + c] = s0;
 }
 
 // shock-weighted relative MSE (loss.py:20-23) on pred = base + head:
@@ -597,7 +797,61 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(int M, int N, int K_split, 
       tc_fence_after();
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(BN));
     }
-    // epilogue in row-contiguous order: a warp covers 32 column pairs of one row
+    if (e.vec) {
+      // epilogue in row-contiguous order, 8 columns per thread: every global
+      // access is 16 bytes, and the loads of 4 row groups are in flight
+      // before the first is used
+      constexpr int IT = (BM * 128 / 8) / THREADS, GROUP = 4;
+#pragma unroll 1
+      for (int it0 = 0; it0 < IT; it0 += GROUP) {
+        float res[GROUP][8], aux[GROUP][8];
+#pragma unroll
+        for (int u = 0; u < GROUP; ++u) {
+          const int q = (it0 + u) * THREADS + tid;
+          const size_t o = (size_t)(m_blk + q / 16) * e.ldo + n_blk + h * 128 + (q % 16) * 8;
+          if (EPI != EPI_F32 && e.res) load8<true>(e.res + o, res[u]);
+          if (EPI == EPI_BWD && e.aux) load8<true>(e.aux + o, aux[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < GROUP; ++u) {
+          const int q = (it0 + u) * THREADS + tid, r = q / 16, c = (q % 16) * 8;
+          const int n = n_blk + h * 128 + c;
+          const size_t o = (size_t)(m_blk + r) * e.ldo + n;
+          const float4 a0 = *reinterpret_cast<const float4*>(stile + r * SLD + c);
+          const float4 a1 = *reinterpret_cast<const float4*>(stile + r * SLD + c + 4);
+          float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+          if (EPI == EPI_F32) {
+            float* out = static_cast<float*>(e.out0) + (size_t)blockIdx.z * e.split_stride + o;
+            *reinterpret_cast<float4*>(out) = a0;
+            *reinterpret_cast<float4*>(out + 4) = a1;
+          } else if (EPI == EPI_FWD) {
+            const float4 b0 = *reinterpret_cast<const float4*>(e.bias + n);
+            const float4 b1 = *reinterpret_cast<const float4*>(e.bias + n + 4);
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            float hv[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              v[i] += b[i];
+              hv[i] = (e.res ? res[u][i] : 0.f) + fmaxf(v[i], 0.f);
+            }
+            store8<true>(e.out1 + o, v);
+            store8<true>(static_cast<bf16*>(e.out0) + o, hv);
+          } else {
+            if (e.res)
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i] += res[u][i];
+            store8<true>(static_cast<bf16*>(e.out0) + o, v);
+            if (e.aux) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) v[i] = aux[u][i] > 0.f ? v[i] : 0.f;
+              store8<true>(e.out1 + o, v);
+            }
+          }
+        }
+      }
+      continue;
+    }
+    // buffers that are not 16-byte aligned: a warp covers 32 column pairs of one row
 #pragma unroll 4
     for (int it = 0; it < (BM * 128 / 2) / THREADS; ++it) {
       const int q = it * THREADS + tid;
@@ -745,7 +999,9 @@ int esr_gemm_bf16(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_
                   void* out0, void* out1, int32_t ldo, int32_t splits, void* stream) {
   const int rc = gemm_check(trans_a, trans_b, M, N, K, A, lda, B, ldb, epi, bias, aux, out0, out1, ldo, splits, tc::BK);
   if (rc != ESR_OK) return rc;
-  Epi e{bias, (const bf16*)res, (const bf16*)aux, out0, (bf16*)out1, ldo, (long long)M * ldo};
+  // rows and buffers aligned for the 16-byte epilogue (a null one is not touched)
+  const bool vec = ldo % 8 == 0 && aligned16(bias) && aligned16(res) && aligned16(aux) && aligned16(out0) && aligned16(out1);
+  Epi e{bias, (const bf16*)res, (const bf16*)aux, out0, (bf16*)out1, ldo, (long long)M * ldo, vec};
   cudaStream_t st = (cudaStream_t)stream;
   const bf16* a = (const bf16*)A;
   const bf16* b = (const bf16*)B;
@@ -768,7 +1024,7 @@ int esr_gemm_bf16_mma_sync(int32_t trans_a, int32_t trans_b, int32_t M, int32_t 
                            const void* aux, void* out0, void* out1, int32_t ldo, int32_t splits, void* stream) {
   const int rc = gemm_check(trans_a, trans_b, M, N, K, A, lda, B, ldb, epi, bias, aux, out0, out1, ldo, splits, BK);
   if (rc != ESR_OK) return rc;
-  Epi e{bias, (const bf16*)res, (const bf16*)aux, out0, (bf16*)out1, ldo, (long long)M * ldo};
+  Epi e{bias, (const bf16*)res, (const bf16*)aux, out0, (bf16*)out1, ldo, (long long)M * ldo, false};
   cudaStream_t st = (cudaStream_t)stream;
   const bf16* a = (const bf16*)A;
   const bf16* b = (const bf16*)B;
@@ -802,7 +1058,11 @@ int esr_mlp_head_fwd(const void* H, int32_t rows, int32_t K, const float* W, con
                      float* y, void* stream) {
   if (!H || !W || !b || !y || rows <= 0 || K <= 0) return mfail(ESR_ERR_ARG, "head_fwd: bad argument");
   const int wpb = 8;
-  k_head_fwd<<<(rows + wpb - 1) / wpb, wpb * 32, 0, (cudaStream_t)stream>>>((const bf16*)H, rows, K, W, b, base, y);
+  if (K == 256)   // four rows per warp and pass, two resident blocks per SM
+    k_head_fwd256<<<std::min((rows + 4 * wpb - 1) / (4 * wpb), 148 * 2), wpb * 32, 0, (cudaStream_t)stream>>>(
+        (const bf16*)H, rows, W, b, base, y);
+  else
+    k_head_fwd<<<(rows + wpb - 1) / wpb, wpb * 32, 0, (cudaStream_t)stream>>>((const bf16*)H, rows, K, W, b, base, y);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, cudaGetErrorString(err));
 }
@@ -814,9 +1074,8 @@ int esr_mlp_head_bwd(const float* dY, const void* H, const void* Z, int32_t rows
   if (!dY || !H || !Z || !W || !dH || !dZ || !part || rows <= 0 || K != 256 || rpb <= 0)
     return mfail(ESR_ERR_ARG, "head_bwd: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
-  const long long n = (long long)rows * K;
-  k_head_bwd_dx<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dY, rows, K, W, (const bf16*)Z, (bf16*)dH, (bf16*)dZ);
-  k_head_bwd_dw<<<(rows + rpb - 1) / rpb, K, 0, st>>>(dY, (const bf16*)H, rows, K, rpb, part);
+  auto* k = (((uintptr_t)H | (uintptr_t)Z | (uintptr_t)dH | (uintptr_t)dZ) & 3) == 0 ? k_head_bwd<true> : k_head_bwd<false>;
+  k<<<(rows + rpb - 1) / rpb, 128, 0, st>>>(dY, (const bf16*)H, (const bf16*)Z, rows, W, (bf16*)dH, (bf16*)dZ, rpb, part);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, cudaGetErrorString(err));
 }
@@ -825,8 +1084,8 @@ int esr_mlp_features(const float* stat5, const float* idw_prim, const float* idw
                      float aoa_n, const float* mu, const float* sig, int32_t ld, void* X, float* base, void* stream) {
   if (!stat5 || !idw_prim || !idw_gradp || !mu || !sig || !X || rows <= 0 || ld < 13)
     return mfail(ESR_ERR_ARG, "features: bad argument");
-  k_features<<<(rows + 127) / 128, 128, 0, (cudaStream_t)stream>>>(stat5, idw_prim, idw_gradp, rows, mach_n, aoa_n,
-                                                                   mu, sig, ld, (bf16*)X, base);
+  k_features<<<(rows + kFeatureRows - 1) / kFeatureRows, kFeatureRows, 0, (cudaStream_t)stream>>>(
+      stat5, idw_prim, idw_gradp, rows, mach_n, aoa_n, mu, sig, ld, (bf16*)X, base, ld % 8 == 0 && aligned16(X));
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, cudaGetErrorString(err));
 }
@@ -840,16 +1099,34 @@ int esr_mlp_decode(const float* pred_n, int32_t rows, const float* mu, const flo
 }
 
 int esr_reduce_splits(const float* part, int32_t splits, int64_t stride, int64_t n, float* out, void* stream) {
-  if (!part || !out || splits <= 0 || n <= 0 || stride < n) return mfail(ESR_ERR_ARG, "reduce_splits: bad argument");
-  k_reduce_splits<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(part, splits, stride, n, out);
+  const esr_reduction r{part, out, stride, n, splits, 0};
+  return esr_reduce_many(&r, 1, stream);
+}
+
+int esr_reduce_many(const esr_reduction* sets, int32_t n_sets, void* stream) {
+  if (n_sets < 0 || n_sets > kMaxReductions || (n_sets > 0 && !sets))
+    return mfail(ESR_ERR_ARG, "reduce_splits: between 0 and " + std::to_string(kMaxReductions) + " sets");
+  Reductions q{};
+  long long blocks = 0;
+  for (int i = 0; i < n_sets; ++i) {
+    const esr_reduction& r = sets[i];
+    if (!r.part || !r.out || r.splits <= 0 || r.n <= 0 || r.stride < r.n)
+      return mfail(ESR_ERR_ARG, "reduce_splits: bad argument");
+    q.r[q.n++] = Reduction{r.part, r.out, r.stride, r.n, r.splits, (int)blocks};
+    blocks += (r.n + 255) / 256;
+    if (blocks > INT32_MAX) return mfail(ESR_ERR_ARG, "reduce_splits: too many outputs");
+  }
+  if (blocks == 0) return ESR_OK;
+  k_reduce_splits<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(q);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, cudaGetErrorString(err));
 }
 
 int esr_colsum_bf16(const void* X, int32_t rows, int32_t C, int32_t rpb, float* part, void* stream) {
   if (!X || !part || rows <= 0 || C <= 0 || rpb <= 0) return mfail(ESR_ERR_ARG, "colsum: bad argument");
-  dim3 grid((rows + rpb - 1) / rpb, (C + 127) / 128);
-  k_colsum_part<<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16*)X, rows, C, rpb, part);
+  dim3 grid((rows + rpb - 1) / rpb, (C + 255) / 256);
+  auto* k = C % 2 == 0 && ((uintptr_t)X & 3) == 0 ? k_colsum_part<true> : k_colsum_part<false>;
+  k<<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16*)X, rows, C, rpb, part);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, cudaGetErrorString(err));
 }

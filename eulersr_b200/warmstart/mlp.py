@@ -141,29 +141,36 @@ class MLP:
         rpb = 256
         nblk = (rows + rpb - 1) // rpb
         part_head = self._buf("part_head", (nblk, 4 * H + 4), torch.float32)
-        dh = self._buf("dh3", (rows, H), torch.bfloat16)
-        dz = self._buf("dz3", (rows, H), torch.bfloat16)
+        # the layers' dz back to back: their column sums are one call
+        dzs = self._buf("dz", (4, rows, H), torch.bfloat16)
+        dh, dz = self._buf("dh3", (rows, H), torch.bfloat16), dzs[3]
         F.check(self.L.esr_mlp_head_bwd(_p(dY), _p(h[3]), _p(z[3]), rows, H, _p(self.view("W4")), _p(dh), _p(dz),
                                         _p(part_head), rpb, st))
         # W4 and b4 are contiguous in the flat layout, as in the partials
-        F.check(self.L.esr_reduce_splits(_p(part_head), nblk, 4 * H + 4, 4 * H + 4, _p(self.gview("W4")), st))
-        part = self._buf("part_w", (splits, H, H), torch.float32)
-        cpart = self._buf("part_c", (nblk, H), torch.float32)
+        sums = [(part_head, nblk, 4 * H + 4, 4 * H + 4, self.gview("W4"))]
+        part = self._buf("part_w", (4, splits, H, H), torch.float32)
+        cpart = self._buf("part_c", (4, nblk, H), torch.float32)
         for l in (3, 2, 1, 0):
             kin = K_IN if l == 0 else H
             src = X if l == 0 else h[l - 1]
             # weight gradient dW_l = dz_l^T src (split-K over rows, fixed-order reduction)
             F.check(self.gemm(1, 1, H, kin, rows, _p(dz), H, _p(src), kin, 0, None, None, None,
-                                         _p(part), None, kin, splits, st))
-            F.check(self.L.esr_reduce_splits(_p(part), splits, H * kin, H * kin, _p(self.gview(f"W{l}")), st))
-            F.check(self.L.esr_colsum_bf16(_p(dz), rows, H, rpb, _p(cpart), st))
-            F.check(self.L.esr_reduce_splits(_p(cpart), nblk, H, H, _p(self.gview(f"b{l}")), st))
+                                         _p(part[l]), None, kin, splits, st))
+            sums.append((part[l], splits, H * kin, H * kin, self.gview(f"W{l}")))
+            sums.append((cpart[l], nblk, H, H, self.gview(f"b{l}")))
             if l > 0:
-                dh_prev = self._buf(f"dh{l - 1}", (rows, H), torch.bfloat16)
-                dz_prev = self._buf(f"dz{l - 1}", (rows, H), torch.bfloat16)
+                dh_prev, dz_prev = self._buf(f"dh{l - 1}", (rows, H), torch.bfloat16), dzs[l - 1]
                 F.check(self.gemm(0, 1, rows, H, H, _p(dz), H, _p(self.view(f"W{l}", True)), H, 2,
                                              None, _p(dh), _p(z[l - 1]), _p(dh_prev), _p(dz_prev), H, 1, st))
                 dh, dz = dh_prev, dz_prev
+        if rows % rpb == 0:
+            F.check(self.L.esr_colsum_bf16(_p(dzs), 4 * rows, H, rpb, _p(cpart), st))
+        else:   # a row block would span two layers
+            for l in range(4):
+                F.check(self.L.esr_colsum_bf16(_p(dzs[l]), rows, H, rpb, _p(cpart[l]), st))
+        table = (F.Reduction * len(sums))(*[F.Reduction(p.data_ptr(), out.data_ptr(), stride, n, k, 0)
+                                            for p, k, stride, n, out in sums])
+        F.check(self.L.esr_reduce_many(table, len(sums), st))
 
     def loss(self, y, tgt, w, inv_den):
         rows = y.shape[0]

@@ -458,6 +458,15 @@ int esr_mlp_loss(const float* pred, const float* tgt, const float* w, int32_t ro
                  float* dpred, float* part, void* stream);
 /* fixed-order sums: out[i] = sum_s part[s*stride + i]; column sums of BF16 rows */
 int esr_reduce_splits(const float* part, int32_t splits, int64_t stride, int64_t n, float* out, void* stream);
+/* the same for up to 16 sets of partials in one launch (the table is host
+ * memory, read before the call returns) */
+typedef struct esr_reduction {
+    const float* part;
+    float* out;
+    int64_t stride, n;
+    int32_t splits, reserved;
+} esr_reduction;
+int esr_reduce_many(const esr_reduction* sets, int32_t n_sets, void* stream);
 int esr_colsum_bf16(const void* X, int32_t rows, int32_t C, int32_t rpb, float* part, void* stream);
 /* AdamW on FP32 master weights, refreshing an optional BF16 copy */
 int esr_adamw(float* p, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2, float eps,

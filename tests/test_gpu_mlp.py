@@ -235,3 +235,92 @@ def test_tcgen05_gemm_matches_mma_sync(ta, tb, epi, M, N, K, splits):
         if epi == 1:
             z = ref + bias.double().cpu()
             assert _rel(t1.double().cpu().numpy(), z.numpy()) < 4e-3
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 256), (7, 256), (129, 256), (1000, 256), (300, 40), (65, 7), (33, 264)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_column_sums_and_split_reduction_edges(rows, cols, shift):
+    """esr_colsum_bf16 and esr_reduce_splits at the edges of their row lanes,
+    column groups and split groups, on buffers aligned to 16 bytes and shifted
+    by one element. Tolerance: float32 sums of at most 1,000 BF16 values of
+    magnitude ~1 in 8 x 128 partial chains, 1e-5 of the sum of magnitudes."""
+    import torch
+    from eulersr_b200 import _ffi as F
+    g = torch.Generator().manual_seed(rows)
+    X = torch.randn(rows * cols + shift, generator=g).to(torch.bfloat16).cuda()[shift:]
+    rpb = 100
+    nb = (rows + rpb - 1) // rpb
+    part = torch.full((nb, cols), float("nan"), device="cuda")
+    out = torch.full((cols,), float("nan"), device="cuda")
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    F.check(F.lib().esr_colsum_bf16(p(X), rows, cols, rpb, p(part), st))
+    F.check(F.lib().esr_reduce_splits(p(part), nb, cols, cols, p(out), st))
+    x = X.view(rows, cols).double()
+    ref, mag = x.sum(0), x.abs().sum(0)
+    assert torch.all((out.double() - ref).abs() <= 1e-5 * mag + 1e-12)
+    for splits in (1, 7, 8, 9, 33):
+        q = torch.randn(splits, cols + 3, generator=g).cuda()
+        F.check(F.lib().esr_reduce_splits(p(q), splits, cols + 3, cols, p(out), st))
+        r = q[:, :cols].double()
+        assert torch.all((out.double() - r.sum(0)).abs() <= 1e-6 * r.abs().sum(0) + 1e-12)
+
+
+@pytest.mark.parametrize("rows", [1, 15, 128, 1001])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_head_kernels_edges(rows, shift):
+    """The head's forward and backward at row counts around its blocks and
+    warps, with aligned and shifted BF16 buffers, against float64. Tolerances:
+    float32 sums of 256 (forward) or `rows` (weight gradient) products, 1e-5
+    of the sum of magnitudes; dH and dZ are BF16 roundings, 2^-8 relative."""
+    import torch
+    from eulersr_b200 import _ffi as F
+    K, rpb = 256, 128
+    g = torch.Generator().manual_seed(rows + shift)
+    bf = lambda: torch.randn(rows * K + shift, generator=g).to(torch.bfloat16).cuda()[shift:].view(rows, K)
+    H, Z = bf(), bf()
+    dH = torch.zeros(rows * K + shift, dtype=torch.bfloat16, device="cuda")[shift:].view(rows, K)
+    dZ = torch.zeros_like(H) if not shift else torch.zeros(rows * K + 1, dtype=torch.bfloat16, device="cuda")[1:].view(rows, K)
+    W, b = torch.randn(4, K, generator=g).cuda(), torch.randn(4, generator=g).cuda()
+    dY, base = torch.randn(rows, 4, generator=g).cuda(), torch.randn(rows, 4, generator=g).cuda()
+    y = torch.empty(rows, 4, device="cuda")
+    nb = (rows + rpb - 1) // rpb
+    part = torch.full((nb, 4 * K + 4), float("nan"), device="cuda")
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    F.check(F.lib().esr_mlp_head_fwd(p(H), rows, K, p(W), p(b), p(base), p(y), st))
+    h, w = H.double(), W.double()
+    assert torch.all((y.double() - (h @ w.T + b + base)).abs() <= 1e-5 * (h.abs() @ w.abs().T + 1))
+    F.check(F.lib().esr_mlp_head_bwd(p(dY), p(H), p(Z), rows, K, p(W), p(dH), p(dZ), p(part), rpb, st))
+    dh = dY.double() @ w
+    tol = 2.0 ** -8 * dh.abs() + 1e-5 * (dY.double().abs() @ w.abs())
+    assert torch.all((dH.double() - dh).abs() <= tol)
+    assert torch.all((dZ.double() - dh * (Z > 0)).abs() <= tol)
+    tot = part.double().sum(0)
+    gw, mag = dY.double().T @ h, dY.double().abs().T @ h.abs()
+    assert torch.all((tot[:4 * K].view(4, K) - gw).abs() <= 1e-5 * mag + 1e-12)
+    assert torch.all((tot[4 * K:] - dY.double().sum(0)).abs() <= 1e-5 * dY.double().abs().sum(0) + 1e-12)
+
+
+def test_gemm_epilogue_aligned_and_shifted_buffers_agree():
+    """The 16-byte epilogue and the element-pair one (outputs 4 bytes off the
+    16-byte grid) write the same bits, forward and backward."""
+    import torch
+    from eulersr_b200 import _ffi as F
+    M, N, K = 384, 256, 128
+    g = torch.Generator().manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).cuda()
+    A, B, res, aux = rnd(M, K), rnd(N, K), rnd(M, N), rnd(M, N)
+    bias = torch.randn(N, generator=g).cuda()
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    for epi in (1, 2):
+        got = []
+        for off in (0, 2):
+            o0 = torch.zeros(M * N + off, dtype=torch.bfloat16, device="cuda")[off:]
+            o1 = torch.zeros(M * N + off, dtype=torch.bfloat16, device="cuda")[off:]
+            F.check(F.lib().esr_gemm_bf16(0, 0, M, N, K, p(A), K, p(B), K, epi, p(bias), p(res), p(aux), p(o0), p(o1),
+                                          N, 1, st))
+            got.append((o0.clone(), o1.clone()))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+        assert got[0][1].abs().sum() > 0
