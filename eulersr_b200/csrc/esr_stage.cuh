@@ -16,9 +16,9 @@
 // in single solves. The separate K1 / K2 pass 96 B of face states per item and
 // stage through memory and pay two launches; here a stage moves the state
 // alone, for about a third more reconstructions. Measured (us per SRK2 step,
-// separate kernels -> fused): 1 slot x 1,450 cells 20.0 -> 8.9, 1 x 25,968
-// 21.0 -> 10.6, 32 x 1,810 19.9 -> 13.9, 32 x 25,968 88 -> 62, 256 x 25,049
-// 569 -> 387; float64 1 x 19,384 37 -> 14, 24 x 25,968 282 -> 153; reference
+// separate kernels -> fused): 1 slot x 1,450 cells 20.0 -> 7.4, 1 x 25,968
+// 21.0 -> 9.1, 32 x 1,810 19.9 -> 12.4, 32 x 25,968 88 -> 60, 256 x 25,049
+// 569 -> 382; float64 1 x 19,384 37 -> 14, 24 x 25,968 282 -> 153; reference
 // fidelity 1 x 19,384 29 -> 24.
 //
 // CANON (float64 and fast float32): each face of the tile once, from its
@@ -32,6 +32,45 @@
 #include "esr_device.cuh"
 
 namespace esr {
+
+// Launches of k_stage overlap (programmatic dependent launch): a block may start
+// while the previous launch still runs, reads the tile tables, which never
+// change, and waits here until that launch has finished and its results are
+// visible. Everything a launch writes (states, control words, local steps) is
+// read after this, by loads that bypass the read-only cache. Worth 1.5 us per
+// step of a single solve (8.9 -> 7.4 at 1,450 cells, 10.6 -> 9.1 at 25,968).
+// k_stage_pair runs without it: its launches are long or its blocks' own
+// chains of dependent work dominate (32 x 1,810 cells 12.4 us either way).
+__device__ __forceinline__ void stage_begin() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+__device__ __forceinline__ float4 fresh(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double4 fresh(const double4* p) {
+  double4 v;
+  asm volatile("ld.global.cg.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  asm volatile("ld.global.cg.v2.f64 {%0,%1}, [%2+16];" : "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float fresh(const float* p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double fresh(const double* p) {
+  double v;
+  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int fresh(const int* p) {
+  int v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 
 template <typename T>
 struct StageMap {
@@ -123,28 +162,32 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
   const int slot = threadIdx.x & ((1 << sh) - 1), b = b0 + slot;
   const bool in_seg = b < s.B;
   const int g = s.case0 + (in_seg ? b : 0);
-  const int act = cs.active[g], done = cs.step[g], cap = cs.nmax[g];
-  const V inlet = cs.inlet[g];
   const int* list = s.tile_list + h.list;
+  const StageCell<T>* cells = s.tile_cells + h.cells;
+  StageCell<T> r = cells[min((int)threadIdx.x >> sh, h.n1 - 1)];
+  const int c0 = list[min((int)threadIdx.x >> sh, h.n2 - 1)];
+  stage_begin();
+  const int act = fresh(cs.active + g), done = fresh(cs.step + g), cap = fresh(cs.nmax + g);
+  const V inlet = fresh(cs.inlet + g);
   const bool live = in_seg && act && done + pos < cap;
   if (!__syncthreads_or(live)) return;          // every slot of the group idle
   const V* win = Win + s.off + (in_seg ? b : 0);
   // A: primitives of the tile, its two rings and its ghosts
-  for (int i = threadIdx.x; i < h.n2 << sh; i += nt) {
+  for (int i = threadIdx.x, c = c0; i < h.n2 << sh; i += nt) {
     T q[4];
-    cell_prim<T, FAST>(win[(long long)list[i >> sh] * s.B], kc, q);
+    const V w = fresh(win + (long long)c * s.B);
+    if (i + nt < h.n2 << sh) c = list[(i + nt) >> sh];
+    cell_prim<T, FAST>(w, kc, q);
     P[i] = mk4<T>(q[0], q[1], q[2], q[3]);
   }
   for (int i = threadIdx.x; i < h.n_ghosts << sh; i += nt) {
     const StageGhost<T> w = s.tile_ghosts[h.ghosts + (i >> sh)];
     T q[4];
-    ghost_prim<T, FAST>(w.kind, win[(long long)w.cell * s.B], w.nx, w.ny, inlet, kc, q);
+    ghost_prim<T, FAST>(w.kind, fresh(win + (long long)w.cell * s.B), w.nx, w.ny, inlet, kc, q);
     P[(h.n2 << sh) + i] = mk4<T>(q[0], q[1], q[2], q[3]);
   }
   // B: limited face states of the tile and its first ring. The first record
   // of each phase is on its way before the barrier.
-  const StageCell<T>* cells = s.tile_cells + h.cells;
-  StageCell<T> r = cells[min((int)threadIdx.x >> sh, h.n1 - 1)];
   __syncthreads();
   for (int i = threadIdx.x; i < h.n1 << sh; i += nt) {
     const int lc = i >> sh;
@@ -187,19 +230,25 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
     }
     if (i + nt < h.n_faces << sh) f = faces[(i + nt) >> sh];
   }
-  __syncthreads();
-  if (!live) return;
   // D: residual, sponge and stage update of the tile's own cells
   const V* G = CANON ? FV : FX;
-  const T strength = cs.strength[g];
-  const T case_dt = cs.dt[g];
+  const T strength = fresh(cs.strength + g);
+  const T case_dt = fresh(cs.dt + g);
   const StageOwn<T>* own = s.tile_own + h.own;
+  StageOwn<T> o = own[min((int)threadIdx.x >> sh, h.n_own - 1)];
+  const long long base = s.off + (in_seg ? b : 0);
+  V Wc = fresh(Win + base + (long long)o.cell * s.B), W0 = Wc;
+  if (STAGE != ST_FIRST) W0 = fresh(Wbase + base + (long long)o.cell * s.B);
+  __syncthreads();
+  if (!live) return;
   for (int i = threadIdx.x; i < h.n_own << sh; i += nt) {
     const int lc = i >> sh;
-    const StageOwn<T> o = own[lc];
-    const long long gi = s.off + (long long)o.cell * s.B + b;
-    const V Wc = Win[gi];
-    const V W0 = (STAGE == ST_FIRST) ? Wc : Wbase[gi];
+    if (i >= nt) {   // not the first
+      o = own[lc];
+      Wc = fresh(Win + base + (long long)o.cell * s.B);
+      W0 = STAGE == ST_FIRST ? Wc : fresh(Wbase + base + (long long)o.cell * s.B);
+    }
+    const long long gi = base + (long long)o.cell * s.B;
     T acc[4], dt = case_dt;
     if (LOCALDT) {   // dt holds the case's CFL number
       if (STAGE == ST_FIRST) {
@@ -208,7 +257,7 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
         dt = local_dt<T, FAST>(q, o.n, o.s, o.area, kc) * case_dt;
         dt_local[gi] = dt;
       } else {
-        dt = dt_local[gi];
+        dt = fresh(dt_local + gi);
       }
     }
 #pragma unroll
@@ -231,6 +280,18 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
     // density residual of the state the step starts from (density-L2 stop rule)
     if (STAGE == ST_FIRST && res_out != nullptr) res_out[gi] = R0;
     Wout[gi] = w;
+  }
+}
+
+// the states of two slots dB apart; wide: they are neighbours on a 32-byte
+// boundary, one access (as two 16-byte ones every sector is fetched twice)
+__device__ __forceinline__ void state_pair(const float4* p, int dB, bool wide, float4& a, float4& b) {
+  if (wide) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p));
+  } else {
+    a = p[0];
+    b = p[dB];
   }
 }
 
@@ -293,28 +354,30 @@ __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
   // slots b and b + 1; one past the segment repeats the last slot and is not stored
   const int bA = min(b0 + 2 * pr, s.B - 1), bB = min(b0 + 2 * pr + 1, s.B - 1);
   const int gA = s.case0 + bA, gB = s.case0 + bB;
-  const int actA = cs.active[gA], actB = cs.active[gB];
-  const int doneA = cs.step[gA], doneB = cs.step[gB], capA = cs.nmax[gA], capB = cs.nmax[gB];
   const int* list = s.tile_list + h.list;
+  const int n2 = h.n2 << SH;
+  int c[kLoads];
+#pragma unroll
+  for (int u = 0; u < kLoads; ++u) c[u] = list[min((int)threadIdx.x + u * kPairThreads, n2 - 1) >> SH];
+  const int actA = cs.active[gA], actB = cs.active[gB];
+  const int doneA = cs.step[gA], doneB = cs.step[gB];
+  const int capA = cs.nmax[gA], capB = cs.nmax[gB];
   const bool liveA = b0 + 2 * pr < s.B && actA && doneA + pos < capA;
   const bool liveB = b0 + 2 * pr + 1 < s.B && actB && doneB + pos < capB;
   if (!__syncthreads_or(liveA || liveB)) return;   // every slot of the group idle
   const float4* winA = Win + s.off + bA;
   const int dB = bB - bA;
+  // both slots in one 32-byte access: every row of the state starts on 32 bytes
+  const bool wide = dB == 1 && ((s.off | s.B) & 1) == 0;
   // A: primitives of the tile, its two rings and its ghosts; the states of
   // kLoads rows are requested before the first is used
-  const int n2 = h.n2 << SH;
   for (int i0 = threadIdx.x; i0 < n2; i0 += kLoads * kPairThreads) {
-    int c[kLoads];
     float4 a[kLoads], b[kLoads];
 #pragma unroll
-    for (int u = 0; u < kLoads; ++u) c[u] = list[min(i0 + u * kPairThreads, n2 - 1) >> SH];
+    for (int u = 0; u < kLoads; ++u) state_pair(winA + (long long)c[u] * s.B, dB, wide, a[u], b[u]);
+    if (i0 + kLoads * kPairThreads < n2)
 #pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      const float4* w = winA + (long long)c[u] * s.B;
-      a[u] = w[0];
-      b[u] = w[dB];
-    }
+      for (int u = 0; u < kLoads; ++u) c[u] = list[min(i0 + (kLoads + u) * kPairThreads, n2 - 1) >> SH];
 #pragma unroll
     for (int u = 0; u < kLoads; ++u) {
       const int i = i0 + u * kPairThreads;
@@ -395,7 +458,8 @@ __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
   // D: residual, sponge and stage update of the tile's own cells
   const StageOwn<float>* owns = s.tile_own + h.own;
   StageOwn<float> o = owns[min((int)threadIdx.x >> SH, h.n_own - 1)];
-  float4 wa = winA[(long long)o.cell * s.B], wb = winA[(long long)o.cell * s.B + dB];
+  float4 wa, wb;
+  state_pair(winA + (long long)o.cell * s.B, dB, wide, wa, wb);
   const float2 strength = make_float2(cs.strength[gA], cs.strength[gB]);
   const float2 case_dt = make_float2(cs.dt[gA], cs.dt[gB]);
   float2 inlet[4];
@@ -407,7 +471,11 @@ __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
     const long long gi = s.off + (long long)o.cell * s.B + bA;
     float2 Wc[4], W0[4], acc[4], w[4], R0;
     pair_of(wa, wb, Wc);
-    if (STAGE != ST_FIRST) pair_of(Wbase[gi], Wbase[gi + dB], W0);
+    if (STAGE != ST_FIRST) {
+      float4 a, b;
+      state_pair(Wbase + gi, dB, wide, a, b);
+      pair_of(a, b, W0);
+    }
     float2 dt = case_dt;
     if (LOCALDT) {   // dt holds the case's CFL number
       if (STAGE == ST_FIRST) {
@@ -430,16 +498,21 @@ __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
     xr::cell_update<STAGE, float2>(acc, o.area, sig, inlet, Wc, W0, dt, kc.half, &R0, w);
     if (i + kPairThreads < h.n_own << SH) {
       o = owns[(i + kPairThreads) >> SH];
-      wa = winA[(long long)o.cell * s.B];
-      wb = winA[(long long)o.cell * s.B + dB];
+      state_pair(winA + (long long)o.cell * s.B, dB, wide, wa, wb);
     }
     // density residual of the state the step starts from (density-L2 stop rule)
     if (STAGE == ST_FIRST && res_out != nullptr) {
       if (liveA) res_out[gi] = R0.x;
       if (liveB) res_out[gi + dB] = R0.y;
     }
-    if (liveA) Wout[gi] = make_float4(w[0].x, w[1].x, w[2].x, w[3].x);
-    if (liveB) Wout[gi + dB] = make_float4(w[0].y, w[1].y, w[2].y, w[3].y);
+    const float4 wA = make_float4(w[0].x, w[1].x, w[2].x, w[3].x), wB = make_float4(w[0].y, w[1].y, w[2].y, w[3].y);
+    if (wide && liveA && liveB) {
+      asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(Wout + gi), "f"(wA.x), "f"(wA.y),
+                   "f"(wA.z), "f"(wA.w), "f"(wB.x), "f"(wB.y), "f"(wB.z), "f"(wB.w) : "memory");
+    } else {
+      if (liveA) Wout[gi] = wA;
+      if (liveB) Wout[gi + dB] = wB;
+    }
   }
 }
 
@@ -474,20 +547,27 @@ auto pair_kernel(int sh) {
   return sh == 0 ? k_stage_pair<STAGE, LOCALDT, 0> : sh == 1 ? k_stage_pair<STAGE, LOCALDT, 1> : k_stage_pair<STAGE, LOCALDT, 2>;
 }
 template <typename T, bool FAST>
-void launch_stage(const StageLaunch<T>& L, bool rusanov, int stage, bool local, const V4<T>* win, const V4<T>* wbase,
-                  V4<T>* wout, const Cases<T>& cs, const Consts<T>& kc, int pos, T* dt_local, T* res, cudaStream_t st) {
+cudaError_t launch_stage(const StageLaunch<T>& L, bool rusanov, int stage, bool local, const V4<T>* win,
+                         const V4<T>* wbase, V4<T>* wout, const Cases<T>& cs, const Consts<T>& kc, int pos, T* dt_local,
+                         T* res, cudaStream_t st) {
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)L.blocks);
+  cfg.blockDim = dim3((unsigned)L.threads);
+  cfg.dynamicSmemBytes = (size_t)L.smem;
+  cfg.stream = st;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = L.pairs >= 0 ? 0 : 1;   // k_stage_pair does not wait for the previous launch by itself
+  cudaError_t e = cudaSuccess;
   stage_form(rusanov, stage, local, [&](auto f, auto s, auto l) {
-    if constexpr (kFastPath<T, FAST> && f() == 0) {
-      if (L.pairs >= 0) {
-        auto* k = pair_kernel<s(), l()>(L.pairs);
-        k<<<L.blocks, kPairThreads, L.smem, st>>>(L.map, win, wbase, wout, cs, kc, pos, dt_local, res, L.p_rows,
-                                                  L.fv_rows);
-        return;
-      }
-    }
-    k_stage<T, FAST, f(), s(), l()><<<L.blocks, L.threads, L.smem, st>>>(L.map, win, wbase, wout, cs, kc, pos, dt_local,
-                                                                         res, L.p_rows, L.fv_rows);
+    auto* k = &k_stage<T, FAST, f(), s(), l()>;
+    if constexpr (kFastPath<T, FAST> && f() == 0)
+      if (L.pairs >= 0) k = pair_kernel<s(), l()>(L.pairs);
+    e = cudaLaunchKernelEx(&cfg, k, L.map, win, wbase, wout, cs, kc, pos, dt_local, res, L.p_rows, L.fv_rows);
   });
+  return e;
 }
 // Raises the dynamic shared-memory limit of every form a solver of this flux
 // and time step launches, to what a block may hold at most: the limit is the
