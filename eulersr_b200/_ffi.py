@@ -95,6 +95,11 @@ class TuningVariant(C.Structure):
                 "k1_minb": int(self.k1_minb), "k2_minb": int(self.k2_minb), "step_ms": float(self.step_ms)}
 
 
+class MlpNet(C.Structure):
+    """esr_mlp_net"""
+    _fields_ = [("W", C.c_void_p * 4), ("b", C.c_void_p * 4), ("W4", C.c_void_p), ("b4", C.c_void_p)]
+
+
 class Reduction(C.Structure):
     """esr_reduction"""
     _fields_ = [("part", C.c_void_p), ("out", C.c_void_p), ("stride", C.c_int64), ("n", C.c_int64),
@@ -187,6 +192,8 @@ _SIGS = {
     "esr_mlp_loss": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p,
                                C.c_void_p]),
     "esr_reduce_splits": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
+    "esr_mlp_forward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                  C.c_void_p]),
     "esr_reduce_many": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p]),
     "esr_colsum_bf16": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]),
     "esr_adamw": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float,

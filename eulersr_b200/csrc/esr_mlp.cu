@@ -892,6 +892,226 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(int M, int N, int K_split, 
   }
 }
 
+// ---- the whole network forward in one kernel: a CTA owns TILES x 128 rows and
+// keeps their activations in shared memory from layer to layer.
+//   A   per tile 128 x 256 BF16 activations, K-major with the 128-byte swizzle
+//       (64 KB); layer l's MMAs read h_{l-1} there and its epilogue replaces
+//       it by h_l
+//   W   a ring of 64-wide K-blocks of the weights (32 KB each, by TMA): the 14
+//       blocks of the four layers run through it without a stop, so the next
+//       layer's first blocks arrive during the epilogue
+// One thread issues loads and tcgen05.mma; 8 warps per tile read the
+// accumulators back (warp w of a tile: rows 32 (w % 4) .., columns 128 (w / 4)
+// ..), add bias and residual and round as the layer-by-layer GEMM does; the
+// head ends in the summation order of k_head_fwd. Inference moves 272 B per
+// row instead of 4.4 KB and is one launch instead of five; a training forward
+// also writes h and z. What bounds it is bringing 448 KB of weights to every
+// CTA: two tiles share them once there are more tiles than SMs.
+struct MlpMaps { CUtensorMap x, w[4]; };
+struct MlpNet {
+  const float* b[4];
+  const float *w4, *b4, *base;
+  float* y;
+  bf16 *h[4], *z[4];       // null: not kept
+  int rows;
+};
+constexpr int FWD_BLOCKS = 14;                 // K-blocks of the four layers: 2 + 4 + 4 + 4
+template <bool KEEP, int TILES>
+struct Fwd {
+  static constexpr int STAGES = TILES == 1 ? 4 : KEEP ? 2 : 3;
+  static constexpr int W = TILES * 65536;                  // after the activations
+  static constexpr int BARS = W + STAGES * 32768;          // X, done, full and empty per stage, TMEM address
+  static constexpr int TURN = BARS + 128;                  // kept forward: 2 KB per warp to turn z's rows around
+  static constexpr int SMEM = 1024 + TURN + (KEEP ? TILES * 8 * 2048 : 0);
+  static constexpr int THREADS = TILES * 256;
+  static_assert(SMEM <= 227 * 1024, "one CTA per SM");
+};
+
+// byte offset of (row, 8-column chunk c8) in a tile's swizzled activations
+__device__ __forceinline__ uint32_t act_chunk(int row, int c8) {
+  return (uint32_t)((c8 >> 3) * 16384 + row * 128 + (((c8 & 7) ^ (row & 7)) << 4));
+}
+
+template <bool KEEP, int TILES>
+__global__ void __launch_bounds__((Fwd<KEEP, TILES>::THREADS)) k_mlp_fwd(const __grid_constant__ MlpMaps maps,
+                                                                         const __grid_constant__ MlpNet net) {
+  using C = Fwd<KEEP, TILES>;
+  constexpr int S = C::STAGES;
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t raw = saddr(smem_raw), A = (raw + 1023u) & ~1023u, Wt = A + C::W;
+  unsigned char* g = smem_raw + (A - raw);
+  const uint32_t xfull = A + C::BARS, done = xfull + 8, full = done + 8, empty = full + 8 * S;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g + C::BARS + 112);
+  __shared__ int s_abort;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, m0 = blockIdx.x * (TILES * 128);
+  if (tid == 0) {
+    s_abort = 0;
+    mbar_init(xfull, 1);
+    mbar_init(done, 1);
+    for (int k = 0; k < S; ++k) {
+      mbar_init(full + 8 * k, 1);
+      mbar_init(empty + 8 * k, 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(tmem_slot)),
+                 "n"(TILES * 256));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  constexpr uint32_t idesc = instr_desc<false, false, 256>();
+  // thread 0: K-block i of the 14 into its stage
+  int loaded = 0, landed = 0;
+  bool x_landed = false;
+  auto load = [&]() {
+    const int i = loaded++, l = i < 2 ? 0 : 1 + (i - 2) / 4, kb = i < 2 ? i : (i - 2) % 4;
+    mbar_expect_tx(full + 8 * (i % S), 32768);
+    tma_load_2d(Wt + (i % S) * 32768, &maps.w[l], kb * 64, 0, full + 8 * (i % S));
+  };
+  if (tid == 0) {
+    mbar_expect_tx(xfull, TILES * 32768);
+    for (int t = 0; t < TILES; ++t)
+      for (int kb = 0; kb < 2; ++kb) tma_load_2d(A + t * 65536 + kb * 16384, &maps.x, kb * 64, m0 + t * 128, xfull);
+    while (loaded < S) load();
+  }
+#pragma unroll 1
+  for (int l = 0; l < 4; ++l) {
+    const int KB = l == 0 ? 2 : 4, first = l == 0 ? 0 : 4 * l - 2;
+    bool ok = true;
+    if (tid == 0) {
+      if (l == 0) { ok = mbar_wait(xfull, 0); x_landed = ok; }
+      for (int kb = 0; kb < KB && ok; ++kb) {
+        const int i = first + kb, st = i % S;
+        ok = mbar_wait(full + 8 * st, (uint32_t)((i / S) & 1));
+        if (!ok) break;
+        landed = i + 1;
+        tc_fence_after();
+#pragma unroll
+        for (int t = 0; t < TILES; ++t)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma(tmem + t * 256, smem_desc(A + t * 65536 + kb * 16384 + j * 32, 16, 1024),
+                 smem_desc(Wt + st * 32768 + j * 32, 16, 1024), idesc, (kb | j) != 0);
+        umma_commit(empty + 8 * st);
+        // refill the stage that the previous K-block's MMAs read
+        if (kb >= 1 && loaded < FWD_BLOCKS && loaded == i - 1 + S) {
+          ok = mbar_wait(empty + 8 * ((i - 1) % S), (uint32_t)(((i - 1) / S) & 1));
+          if (ok) load();
+        }
+      }
+      umma_commit(done);   // completes once every MMA issued so far has
+    }
+    __syncwarp();
+    const bool mma_ok = mbar_wait(done, (uint32_t)(l & 1));
+    if (!ok || !mma_ok) atomicOr(&s_abort, 1);
+    __syncthreads();
+    if (s_abort) {
+      // A wait gave up: nothing more is written. Loads still landing in shared
+      // memory get a bounded wait each, the accumulators are released.
+      if (tid == 0) {
+        if (!x_landed) mbar_wait(xfull, 0);
+        for (int i = landed; i < loaded; ++i) mbar_wait(full + 8 * (i % S), (uint32_t)((i / S) & 1));
+      }
+      __syncthreads();
+      if (warp == 0) {
+        if (!mma_ok) mbar_wait(done, (uint32_t)(l & 1));
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TILES * 256));
+      }
+      return;
+    }
+    tc_fence_after();
+    if (tid == 0)   // every MMA so far is done: all stages are free
+      while (loaded < FWD_BLOCKS && loaded < first + KB + S) load();
+    const int t = warp >> 3, row = (warp & 3) * 32 + lane, col0 = ((warp >> 2) & 1) * 128;
+    const uint32_t acc = tmem + (uint32_t)(t * 256) + ((uint32_t)((warp & 3) * 32) << 16);
+    unsigned char* act = g + t * 65536;
+    unsigned char* turn = g + C::TURN + warp * 2048;
+    const float* bias = net.b[l];
+    const bool stored = KEEP && m0 + t * 128 < net.rows;
+#pragma unroll 1
+    for (int c32 = col0; c32 < col0 + 128; c32 += 32) {
+      uint32_t v[32];
+      tmem_ld16(acc + (uint32_t)c32, v);
+      tmem_ld16(acc + (uint32_t)(c32 + 16), v + 16);
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const int c = c32 + 8 * p;
+        bf16* a = reinterpret_cast<bf16*>(act + act_chunk(row, c >> 3));
+        const float4 b0 = __ldg(reinterpret_cast<const float4*>(bias + c));
+        const float4 b1 = __ldg(reinterpret_cast<const float4*>(bias + c) + 1);
+        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        float zv[8], hv[8];
+        if (l > 0) load8<true>(a, hv);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          zv[i] = __uint_as_float(v[8 * p + i]) + b[i];
+          hv[i] = (l > 0 ? hv[i] : 0.f) + fmaxf(zv[i], 0.f);
+        }
+        store8<true>(a, hv);
+        if (KEEP) store8<true>(reinterpret_cast<bf16*>(turn + lane * 64 + ((p ^ ((lane >> 1) & 3)) << 4)), zv);
+      }
+      if (KEEP) {
+        // 32 rows x 32 columns of this warp, eight rows (64 B each) per store:
+        // a lane writing its own row would touch 32 lines at a time
+        __syncwarp();
+        if (stored) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int r = q * 8 + (lane >> 2), ch = lane & 3, gr = (warp & 3) * 32 + r;
+            const size_t o = (size_t)(m0 + t * 128 + gr) * 256 + c32 + ch * 8;
+            *reinterpret_cast<uint4*>(net.z[l] + o) =
+                *reinterpret_cast<const uint4*>(turn + r * 64 + ((ch ^ ((r >> 1) & 3)) << 4));
+            *reinterpret_cast<uint4*>(net.h[l] + o) =
+                *reinterpret_cast<const uint4*>(act + act_chunk(gr, (c32 >> 3) + ch));
+          }
+        }
+        __syncwarp();
+      }
+    }
+    tc_fence_before();
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // h_l before the next layer's MMAs read it
+    __syncthreads();
+    tc_fence_after();
+  }
+  if (warp == 0)   // every tcgen05.ld has completed
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TILES * 256));
+  // head: a warp sums 16 rows, a lane the columns lane + 32 i in order
+  float w[4][8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[j][i] = net.w4[j * 256 + lane + 32 * i];
+  const float bias = net.b4[lane & 3];
+  const unsigned char* act = g + (warp >> 3) * 65536;
+#pragma unroll 2
+  for (int q = 0; q < 16; ++q) {
+    const int r = (warp & 7) * 16 + q;
+    const long long row = m0 + (warp >> 3) * 128 + r;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = lane + 32 * i;
+      const float v = __bfloat162float(reinterpret_cast<const bf16*>(act + act_chunk(r, k >> 3))[k & 7]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[j] += v * w[j][i];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+    if (lane < 4 && row < net.rows) {
+      const float v = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
+      net.y[row * 4 + lane] = v + bias + (net.base ? net.base[row * 4 + lane] : 0.f);
+    }
+  }
+}
+
 }  // namespace tc
 
 int mfail(int code, const std::string& msg) { return esr::report_error(code, msg); }
@@ -966,6 +1186,16 @@ int launch_gemm_tc(int M, int N, int K, int splits, const bf16* A, int lda, cons
   return ESR_OK;
 }
 
+template <bool KEEP, int TILES>
+int launch_fwd(const tc::MlpMaps& maps, const tc::MlpNet& n, void* stream) {
+  using C = tc::Fwd<KEEP, TILES>;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(tc::k_mlp_fwd<KEEP, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  if (attr != cudaSuccess) return mfail(ESR_ERR_CUDA, std::string("mlp_forward: ") + cudaGetErrorString(attr));
+  tc::k_mlp_fwd<KEEP, TILES><<<(n.rows / 128 + TILES - 1) / TILES, C::THREADS, C::SMEM, (cudaStream_t)stream>>>(maps, n);
+  return ESR_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1017,6 +1247,44 @@ int esr_gemm_bf16(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_
 #undef ESR_GEMM_CASE
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, std::string("gemm: ") + cudaGetErrorString(err));
+}
+
+int esr_mlp_forward(const esr_mlp_net* net, const void* X, int32_t rows, const float* base, float* y,
+                    void* const* h, void* const* z, void* stream) {
+  if (!net || !X || !y || rows <= 0 || rows % 128) return mfail(ESR_ERR_ARG, "mlp_forward: rows must be a multiple of 128");
+  if ((h == nullptr) != (z == nullptr)) return mfail(ESR_ERR_ARG, "mlp_forward: h and z are kept together");
+  for (int l = 0; l < 4; ++l) {
+    if (!net->W[l] || !net->b[l] || (h && (!h[l] || !z[l]))) return mfail(ESR_ERR_ARG, "mlp_forward: null operand");
+    if (!aligned16(net->W[l]) || !aligned16(net->b[l]) || (h && (!aligned16(h[l]) || !aligned16(z[l]))))
+      return mfail(ESR_ERR_ARG, "mlp_forward: operands must be 16-byte aligned");
+  }
+  if (!net->W4 || !net->b4 || !aligned16(X)) return mfail(ESR_ERR_ARG, "mlp_forward: bad operand");
+  tc::MlpMaps maps;
+  int rc = make_map(&maps.x, (const bf16*)X, 128, rows, 128, 64, 128);
+  for (int l = 0; l < 4 && rc == ESR_OK; ++l) {
+    const uint64_t k = l == 0 ? 128 : 256;
+    rc = make_map(&maps.w[l], (const bf16*)net->W[l], k, 256, k, 64, 256);
+  }
+  if (rc != ESR_OK) return rc;
+  tc::MlpNet n{};
+  for (int l = 0; l < 4; ++l) {
+    n.b[l] = net->b[l];
+    n.h[l] = h ? (bf16*)h[l] : nullptr;
+    n.z[l] = z ? (bf16*)z[l] : nullptr;
+  }
+  n.w4 = net->W4;
+  n.b4 = net->b4;
+  n.base = base;
+  n.y = y;
+  n.rows = rows;
+  // One tile per CTA while every tile gets an SM of its own; beyond that two
+  // tiles per CTA share the weights (a second round of CTAs would fetch them again).
+  const bool two = rows / 128 > 148;
+  if (h) rc = two ? launch_fwd<true, 2>(maps, n, stream) : launch_fwd<true, 1>(maps, n, stream);
+  else rc = two ? launch_fwd<false, 2>(maps, n, stream) : launch_fwd<false, 1>(maps, n, stream);
+  if (rc != ESR_OK) return rc;
+  cudaError_t err = cudaGetLastError();
+  return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, std::string("mlp_forward: ") + cudaGetErrorString(err));
 }
 
 int esr_gemm_bf16_mma_sync(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_t K, const void* A,

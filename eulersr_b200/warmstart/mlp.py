@@ -37,6 +37,11 @@ def _p(t):
     return C.c_void_p(t.data_ptr())
 
 
+def _array(tensors):
+    """Host array of four device addresses, or None."""
+    return (C.c_void_p * 4)(*[t.data_ptr() for t in tensors]) if tensors else None
+
+
 def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
@@ -51,6 +56,7 @@ class MLP:
             raise ValueError(f"the MLP runs on the library's CUDA kernels; device must be a CUDA device, not {device!r}")
         self.L = F.lib()
         # the 256-wide layers: tcgen05 kernel, or the mma.sync kernel kept as its cross-check
+        self.fused = gemm == "tcgen05"   # the forward as one kernel
         self.gemm = {"tcgen05": self.L.esr_gemm_bf16, "mma_sync": self.L.esr_gemm_bf16_mma_sync}[gemm]
         self.device = device
         self.launches = 0          # library kernels launched by forward()
@@ -113,6 +119,14 @@ class MLP:
         assert rows % ROW_TILE == 0 and X.shape[1] == K_IN and X.dtype == torch.bfloat16
         st = _stream()
         tag = "k" if keep else "f"
+        y = self._buf(f"{tag}y", (rows, N_OUT), torch.float32)
+        if self.fused:
+            h = z = None
+            if keep:
+                h, z = ([self._buf(f"k{n}{l}", (rows, H), torch.bfloat16) for l in range(4)] for n in "hz")
+            F.check(self.L.esr_mlp_forward(C.byref(self._net()), _p(X), rows, _p(base), _p(y), _array(h), _array(z), st))
+            self.launches += 1
+            return (y, dict(X=X, h=h, z=z)) if keep else y
         h = [self._buf(f"{tag}h{l}", (rows, H), torch.bfloat16) for l in range(4)]
         z = [self._buf(f"{tag}z{l}", (rows, H), torch.bfloat16) for l in range(4)]
         F.check(self.gemm(0, 0, rows, H, K_IN, _p(X), K_IN, _p(self.view("W0", True)), K_IN, 1,
@@ -120,13 +134,22 @@ class MLP:
         for l in range(1, 4):
             F.check(self.gemm(0, 0, rows, H, H, _p(h[l - 1]), H, _p(self.view(f"W{l}", True)), H, 1,
                                          _p(self.view(f"b{l}")), _p(h[l - 1]), None, _p(h[l]), _p(z[l]), H, 1, st))
-        y = self._buf(f"{tag}y", (rows, N_OUT), torch.float32)
         F.check(self.L.esr_mlp_head_fwd(_p(h[3]), rows, H, _p(self.view("W4")), _p(self.view("b4")),
                                         _p(base) if base is not None else None, _p(y), st))
         self.launches += 5
         if keep:
             return y, dict(X=X, h=h, z=z)
         return y
+
+    def _net(self):
+        """The network's device addresses (the flat vectors may be replaced between calls)."""
+        at = lambda name, bf16: (self.pb.data_ptr() + 2 * self.offsets[name][0] if bf16
+                                 else self.p.data_ptr() + 4 * self.offsets[name][0])
+        n = F.MlpNet()
+        n.W[:] = [at(f"W{l}", True) for l in range(4)]
+        n.b[:] = [at(f"b{l}", False) for l in range(4)]
+        n.W4, n.b4 = at("W4", False), at("b4", False)
+        return n
 
     # ----------------------------------------------------------- backward
     def backward(self, acts, dY, splits=None):

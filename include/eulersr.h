@@ -440,6 +440,21 @@ int esr_gemm_bf16_mma_sync(int32_t trans_a, int32_t trans_b, int32_t M, int32_t 
 /* Synchronous: 1 in *gave_up when a tcgen05 GEMM stopped waiting on its
  * pipeline barriers (bounded waits) since the last call, then clears it. */
 int esr_gemm_tc_status(int32_t* gave_up);
+/* The whole network forward in one launch (tcgen05): h0 = relu(W0 x + b0),
+ * h_l = h_{l-1} + relu(W_l h_{l-1} + b_l), y = W4 h3 + b4 (+ base), with the
+ * roundings and sums of the layer-by-layer calls below, bit for bit. X BF16
+ * [rows x 128], rows a multiple of 128; W0 BF16 [256 x 128], W1..3 BF16
+ * [256 x 256], W4 FP32 [4 x 256]. h and z: NULL, or four BF16 [rows x 256]
+ * outputs each (activations and pre-activations, for the backward pass).
+ * Its pipeline waits are bounded: esr_gemm_tc_status reports one that gave up. */
+typedef struct esr_mlp_net {
+    const void* W[4];
+    const float* b[4];
+    const float* W4;
+    const float* b4;
+} esr_mlp_net;
+int esr_mlp_forward(const esr_mlp_net* net, const void* X, int32_t rows, const float* base, float* y,
+                    void* const* h, void* const* z, void* stream);
 /* 4-wide output layer: y = H W^T + b (+ base), H BF16 [rows x K], W FP32 [4 x K] */
 int esr_mlp_head_fwd(const void* H, int32_t rows, int32_t K, const float* W, const float* b, const float* base,
                      float* y, void* stream);

@@ -324,3 +324,25 @@ def test_gemm_epilogue_aligned_and_shifted_buffers_agree():
             got.append((o0.clone(), o1.clone()))
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
         assert got[0][1].abs().sum() > 0
+
+
+@pytest.mark.parametrize("rows", [128, 384, 148 * 128, 149 * 128])
+@pytest.mark.parametrize("with_base", [True, False])
+def test_fused_forward_equals_layer_calls(rows, with_base):
+    """esr_mlp_forward (one tile, a few, one per SM, and an odd number in pairs) gives the bits
+    of the layer-by-layer GEMM and head calls: y, and h and z when kept."""
+    import torch
+    from eulersr_b200 import _ffi as F
+    m, X, base, *_ = _setup(rows=rows, seed=5)
+    base = base if with_base else None
+    got = []
+    for fused in (True, False):
+        m.fused = fused
+        y, acts = m.forward(X, base, keep=True)
+        y2 = m.forward(X, base)
+        assert torch.equal(y, y2)
+        got.append([y.clone()] + [t.clone() for t in acts["h"] + acts["z"]])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    bad = C.c_int32(-1)
+    F.check(F.lib().esr_gemm_tc_status(C.byref(bad)))
+    assert bad.value == 0
