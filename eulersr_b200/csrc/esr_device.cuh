@@ -1776,40 +1776,4 @@ __global__ void k_copy_out_device(const V4<T>* __restrict__ W, const int* __rest
   dst[c] = W[off + (long long)inv[c] * B + b];
 }
 
-// ------------------------------------------------------------------- IDW
-// eval/core.py:135-142 with utils/metrics.py:9-14: weights from float64
-// distances, float32 weighted sum over the k neighbours in order. A
-// neighbour index outside [0, n_src) is never read: the row becomes NaN and
-// *bad is set (the host reads it with esr_idw_status).
-__device__ int g_idw_bad = 0;
-
-static __global__ void k_idw(const float* __restrict__ src, int n_src, int n_vars, const int* __restrict__ idx,
-                             const float* __restrict__ dist, int n_dst, int k, float* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_dst) return;
-  double wsum = 0.0;
-  double w[16];
-  bool in_range = true;
-  for (int j = 0; j < k; ++j) {
-    const int q = idx[(size_t)i * k + j];
-    in_range = in_range && q >= 0 && q < n_src;
-    const double d = (double)dist[(size_t)i * k + j];
-    w[j] = 1.0 / (d * d + 1e-12);
-    wsum += w[j];
-  }
-  if (!in_range) {
-    atomicExch(&g_idw_bad, 1);
-    for (int v = 0; v < n_vars; ++v) out[(size_t)i * n_vars + v] = __int_as_float(0x7fc00000);
-    return;
-  }
-  for (int v = 0; v < n_vars; ++v) {
-    float acc = 0.0f;
-    for (int j = 0; j < k; ++j) {
-      const float wf = (float)(w[j] / wsum);
-      acc += wf * src[(size_t)idx[(size_t)i * k + j] * n_vars + v];
-    }
-    out[(size_t)i * n_vars + v] = acc;
-  }
-}
-
 }  // namespace esr

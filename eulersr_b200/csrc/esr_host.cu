@@ -23,6 +23,7 @@
 #include "esr_device.cuh"
 #include "esr_faithful.h"
 #include "esr_stage.cuh"
+#include "esr_warm.cuh"
 #include "esr_internal.h"
 
 namespace {
@@ -2426,6 +2427,20 @@ int esr_idw_apply(const float* d_src, int32_t n_src, int32_t n_vars, const int32
   if (n_dst == 0) return ESR_OK;
   const int tb = 128, nb = (n_dst + tb - 1) / tb;
   esr::k_idw<<<nb, tb, 0, (cudaStream_t)stream>>>(d_src, n_src, n_vars, d_idx, d_dist, n_dst, k, d_out);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? ESR_OK : fail(ESR_ERR_CUDA, cudaGetErrorString(e));
+}
+
+int esr_warm_inputs(const float* src_prim, const float* src_gradp, int32_t n_src, const int32_t* idx, const float* dist,
+                    const float* stat5, int32_t rows, int32_t rows_out, float mach_n, float aoa_n, const float* mu,
+                    const float* sig, int32_t ld, void* X, float* base, void* stream) {
+  if (!src_prim || !src_gradp || !idx || !dist || !stat5 || !mu || !sig || !X || !base || n_src <= 0 || rows <= 0 ||
+      rows_out < rows || ld < 16)
+    return fail(ESR_ERR_ARG, "warm_inputs: bad argument");
+  const bool vec = ld % 8 == 0 && ((uintptr_t)X & 15) == 0;
+  esr::k_warm_inputs<<<(rows_out + esr::kFeatureRows - 1) / esr::kFeatureRows, esr::kFeatureRows, 0, (cudaStream_t)stream>>>(
+      src_prim, src_gradp, n_src, idx, dist, stat5, rows, rows_out, mach_n, aoa_n, mu, sig, ld, (__nv_bfloat16*)X, base,
+      vec);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? ESR_OK : fail(ESR_ERR_CUDA, cudaGetErrorString(e));
 }

@@ -95,15 +95,12 @@ class WarmStart:
         n_lr = lr_prim.shape[0]
         lp = torch.as_tensor(lr_prim, dtype=torch.float32, device=self.device).contiguous()
         lg = torch.as_tensor(lr_gradp, dtype=torch.float32, device=self.device).contiguous()
-        idw = torch.empty((self.n_hr, 4), dtype=torch.float32, device=self.device)
-        idg = torch.empty((self.n_hr, 2), dtype=torch.float32, device=self.device)
-        F.check(self.L.esr_idw_apply(_p(lp), n_lr, 4, _p(self.idx), _p(self.dist), self.n_hr, 6, _p(idw), st))
-        F.check(self.L.esr_idw_apply(_p(lg), n_lr, 2, _p(self.idx), _p(self.dist), self.n_hr, 6, _p(idg), st))
-        X = torch.zeros((self.rows, K_IN), dtype=torch.bfloat16, device=self.device)
-        base = torch.zeros((self.rows, 4), dtype=torch.float32, device=self.device)
-        F.check(self.L.esr_mlp_features(_p(self.stat), _p(idw), _p(idg), self.n_hr, (mach - MACH_MID) / MACH_SCALE,
-                                        aoa / AOA_SCALE, _p(self.mu), _p(self.sig), K_IN, _p(X), _p(base), st))
-        self.launches += 3
+        X = torch.empty((self.rows, K_IN), dtype=torch.bfloat16, device=self.device)
+        base = torch.empty((self.rows, 4), dtype=torch.float32, device=self.device)
+        F.check(self.L.esr_warm_inputs(_p(lp), _p(lg), n_lr, _p(self.idx), _p(self.dist), _p(self.stat), self.n_hr,
+                                       self.rows, (mach - MACH_MID) / MACH_SCALE, aoa / AOA_SCALE, _p(self.mu),
+                                       _p(self.sig), K_IN, _p(X), _p(base), st))
+        self.launches += 1
         return X, base
 
     def predict_state(self, lr_prim, lr_gradp, mach, aoa, use_mlp=True, gamma=1.4):

@@ -413,7 +413,15 @@ int esr_rel_change_noalloc(const void* d_A, const void* d_B, int64_t n_rows, int
 int esr_idw_apply(const float* d_src, int32_t n_src, int32_t n_vars,
                   const int32_t* d_idx, const float* d_dist, int32_t n_dst, int32_t k,
                   float* d_out, void* stream);
-/* Synchronous: 1 in *bad when an esr_idw_apply since the last call met an
+/* The warm start's input rows of one case in one launch: esr_idw_apply (k = 6)
+ * of the coarse primitives [n_src x 4] and pressure gradients [n_src x 2] and
+ * esr_mlp_features of the result, bit for bit: X BF16 [rows_out x ld] (ld >=
+ * 16) and base FP32 [rows_out x 4], rows from `rows` on zero. An out-of-range
+ * neighbour makes its row NaN and raises the IDW error flag. */
+int esr_warm_inputs(const float* src_prim, const float* src_gradp, int32_t n_src, const int32_t* idx, const float* dist,
+                    const float* stat5, int32_t rows, int32_t rows_out, float mach_n, float aoa_n, const float* mu,
+                    const float* sig, int32_t ld, void* X, float* base, void* stream);
+/* Synchronous: 1 in *bad when an esr_idw_apply or esr_warm_inputs since the last call met an
  * out-of-range neighbour index, then clears the flag. */
 int esr_idw_status(int32_t* bad);
 

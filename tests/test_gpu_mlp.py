@@ -346,3 +346,41 @@ def test_fused_forward_equals_layer_calls(rows, with_base):
     bad = C.c_int32(-1)
     F.check(F.lib().esr_gemm_tc_status(C.byref(bad)))
     assert bad.value == 0
+
+
+@pytest.mark.parametrize("rows,rows_out", [(1, 128), (127, 128), (128, 128), (300, 384)])
+def test_warm_inputs_equal_separate_calls(rows, rows_out):
+    """esr_warm_inputs gives the bits of two esr_idw_apply calls and
+    esr_mlp_features, zero rows after the last, and the same NaN row and error
+    flag for an out-of-range neighbour."""
+    import torch
+    from eulersr_b200 import _ffi as F
+    L, n_src, ld = F.lib(), 50, 128
+    g = torch.Generator().manual_seed(rows)
+    f = lambda *s: torch.randn(*s, generator=g).cuda()
+    prim, gradp, stat = f(n_src, 4), f(n_src, 2), f(rows, 5)
+    idx = torch.randint(0, n_src, (rows, 6), generator=g, dtype=torch.int32).cuda()
+    dist = torch.rand(rows, 6, generator=g).cuda()
+    mu, sig = f(4), torch.rand(4, generator=g).cuda() + 0.5
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    bad = C.c_int32(0)
+    for wrong in (False, True):
+        if wrong:
+            idx[rows // 2, 3] = n_src
+        ip, ig = torch.empty(rows, 4, device="cuda"), torch.empty(rows, 2, device="cuda")
+        X0 = torch.zeros(rows_out, ld, dtype=torch.bfloat16, device="cuda")
+        b0 = torch.zeros(rows_out, 4, device="cuda")
+        F.check(L.esr_idw_apply(p(prim), n_src, 4, p(idx), p(dist), rows, 6, p(ip), st))
+        F.check(L.esr_idw_apply(p(gradp), n_src, 2, p(idx), p(dist), rows, 6, p(ig), st))
+        F.check(L.esr_mlp_features(p(stat), p(ip), p(ig), rows, 0.3, -0.2, p(mu), p(sig), ld, p(X0), p(b0), st))
+        F.check(L.esr_idw_status(C.byref(bad)))
+        assert bad.value == int(wrong)
+        X1 = torch.full((rows_out, ld), 7.0, dtype=torch.bfloat16, device="cuda")
+        b1 = torch.full((rows_out, 4), 7.0, device="cuda")
+        F.check(L.esr_warm_inputs(p(prim), p(gradp), n_src, p(idx), p(dist), p(stat), rows, rows_out, 0.3, -0.2, p(mu),
+                                  p(sig), ld, p(X1), p(b1), st))
+        F.check(L.esr_idw_status(C.byref(bad)))
+        assert bad.value == int(wrong)
+        assert torch.equal(X0.view(torch.int16), X1.view(torch.int16))
+        assert torch.equal(torch.nan_to_num(b0, 99.0), torch.nan_to_num(b1, 99.0))
