@@ -490,6 +490,14 @@ typedef struct esr_reduction {
     int32_t splits, reserved;
 } esr_reduction;
 int esr_reduce_many(const esr_reduction* sets, int32_t n_sets, void* stream);
+/* Weight and bias gradients of the four 256-wide layers in one launch
+ * (tcgen05), as partials over `splits` ranges of rows (1 <= splits <= rows /
+ * 64, rows a multiple of 128): dw[l] FP32 [splits x 256 x kin] = dz[l]^T
+ * src[l] and db FP32 [4 x splits x 256] = column sums of dz[l]. dz[l] BF16
+ * [rows x 256]; src[0] BF16 [rows x 128] (kin 128), src[1..3] BF16 [rows x 256]
+ * (kin 256). Its pipeline waits are bounded (esr_gemm_tc_status). */
+int esr_mlp_wgrad(const void* const* dz, const void* const* src, int32_t rows, int32_t splits, float* const* dw,
+                  float* db, void* stream);
 int esr_colsum_bf16(const void* X, int32_t rows, int32_t C, int32_t rpb, float* part, void* stream);
 /* AdamW on FP32 master weights, refreshing an optional BF16 copy */
 int esr_adamw(float* p, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2, float eps,

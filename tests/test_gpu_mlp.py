@@ -384,3 +384,32 @@ def test_warm_inputs_equal_separate_calls(rows, rows_out):
         assert bad.value == int(wrong)
         assert torch.equal(X0.view(torch.int16), X1.view(torch.int16))
         assert torch.equal(torch.nan_to_num(b0, 99.0), torch.nan_to_num(b1, 99.0))
+
+
+@pytest.mark.parametrize("rows,splits", [(128, 1), (128, 2), (384, 1), (640, 3), (1152, 5), (4224, 10), (4224, 66)])
+def test_batched_weight_gradients_match_float64(rows, splits):
+    """esr_mlp_wgrad at one K-block per range, fewer K-blocks than accumulators,
+    ranges of unequal length and rings that wrap: dW_l = dz_l^T src_l and db_l
+    against float64 sums of the same BF16 values. A float32 sum of n products
+    is within n ulp (2^-23, whatever the order) of the sum of magnitudes."""
+    import torch
+    from eulersr_b200 import _ffi as F
+    g = torch.Generator().manual_seed(rows + splits)
+    rnd = lambda *s: (torch.randn(*s, generator=g) + 0.25).to(torch.bfloat16).cuda()
+    dz = [rnd(rows, 256) for _ in range(4)]
+    src = [rnd(rows, 128)] + [rnd(rows, 256) for _ in range(3)]
+    dw = [torch.full((splits, 256, s.shape[1]), float("nan"), device="cuda") for s in src]
+    db = torch.full((4, splits, 256), float("nan"), device="cuda")
+    arr = lambda ts: (C.c_void_p * 4)(*[t.data_ptr() for t in ts])
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    F.check(F.lib().esr_mlp_wgrad(arr(dz), arr(src), rows, splits, arr(dw), C.c_void_p(db.data_ptr()), st))
+    tol = rows * 2.0 ** -23
+    for l in range(4):
+        a, b = dz[l].double(), src[l].double()
+        assert torch.all((dw[l].double().sum(0) - a.T @ b).abs() <= tol * (a.abs().T @ b.abs()))
+        assert torch.all((db[l].double().sum(0) - a.sum(0)).abs() <= tol * a.abs().sum(0))
+    bad = C.c_int32(-1)
+    F.check(F.lib().esr_gemm_tc_status(C.byref(bad)))
+    assert bad.value == 0
+    for bad_rows, bad_splits in ((rows + 64, 1), (rows, 0), (rows, rows // 64 + 1)):
+        assert F.lib().esr_mlp_wgrad(arr(dz), arr(src), bad_rows, bad_splits, arr(dw), C.c_void_p(db.data_ptr()), st) != 0
