@@ -96,7 +96,7 @@ class TuningVariant(C.Structure):
 
 
 class MlpNet(C.Structure):
-    """esr_mlp_net"""
+    """esr_mlp_net; esr_mlp_grads has the same fields"""
     _fields_ = [("W", C.c_void_p * 4), ("b", C.c_void_p * 4), ("W4", C.c_void_p), ("b4", C.c_void_p)]
 
 
@@ -195,6 +195,9 @@ _SIGS = {
     "esr_mlp_forward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                   C.c_void_p]),
     "esr_mlp_wgrad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "esr_mlp_backward_workspace": (C.c_int64, [C.c_int32]),
+    "esr_mlp_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                   C.c_void_p, C.c_void_p]),
     "esr_reduce_many": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p]),
     "esr_colsum_bf16": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]),
     "esr_adamw": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float,

@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(int M, int N, int K_split, 
             if (e.res)
 #pragma unroll
               for (int i = 0; i < 8; ++i) v[i] += res[u][i];
-            store8<true>(static_cast<bf16*>(e.out0) + o, v);
+            if (e.out0) store8<true>(static_cast<bf16*>(e.out0) + o, v);
             if (e.aux) {
 #pragma unroll
               for (int i = 0; i < 8; ++i) v[i] = aux[u][i] > 0.f ? v[i] : 0.f;
@@ -881,7 +881,8 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(int M, int N, int K_split, 
           d0 += __bfloat162float(rr.x);
           d1 += __bfloat162float(rr.y);
         }
-        *reinterpret_cast<__nv_bfloat162*>(static_cast<bf16*>(e.out0) + o) = __floats2bfloat162_rn(d0, d1);
+        if (e.out0)
+          *reinterpret_cast<__nv_bfloat162*>(static_cast<bf16*>(e.out0) + o) = __floats2bfloat162_rn(d0, d1);
         if (e.aux) {
           const __nv_bfloat162 zz = *reinterpret_cast<const __nv_bfloat162*>(e.aux + o);
           *reinterpret_cast<__nv_bfloat162*>(e.out1 + o) = __floats2bfloat162_rn(
@@ -1113,53 +1114,50 @@ __global__ void __launch_bounds__((Fwd<KEEP, TILES>::THREADS)) k_mlp_fwd(const _
 }
 
 // ---- the weight and bias gradients of the four layers in one launch:
-// dW_l = dz_l^T src_l (src_0 = X, src_l = h_{l-1}) and db_l = sum of dz_l's
-// rows, as partials over `splits` ranges of rows. A CTA owns one 128 x 128
-// tile of one layer's dW (14 tiles) and one range; with 10 ranges that is one
-// CTA per SM, so a launch's start and its epilogue are paid once instead of
-// four times, and the partials are 9 MB instead of 33. Warp 1 loads, warp 0
-// issues the MMAs, warps 4-7 of the tiles with n = 0 add up dz's columns from
-// the same shared-memory tiles (no pass of their own over dz). K-blocks go to
-// four accumulators in turn, which keeps each float32 chain below the 1,024
-// rows it had at 32 splits. Bound by the operands' way through L2 (twice 134 MB at
-// 32,768 rows). Training step at 32,768 rows 271 -> 233 us (four GEMMs 64 us,
-// column sums 19, reductions 12 before); error of dW against 64-bit sums of
-// the same values 8.8e-7..1.2e-6 -> 6.8e-7..9.3e-7, of db 1.7e-7 -> 5e-8
-// (512 to 12,800 rows: 5 to 25 times smaller).
-constexpr int WG_TILES = 14, WG_STAGES = 6, WG_ACC = 4;
+// dW_l = dz_l^T src_l (src_0 = X, src_l = h_{l-1}) as `splits` partials, each
+// one accumulator over an equal range of rows, and db_l = sum of dz_l's rows
+// as partials of 256 rows, row by row: the sums and their order are those of
+// one split-K GEMM and one column sum per layer, bit for bit. A CTA owns one
+// 128 x 128 tile of one layer's dW (14 tiles) and up to four ranges, each with
+// an accumulator of its own, so that a launch's start is paid once and one
+// range's partial goes out while the next one's MMAs run. Warp 1 loads, warp 0
+// issues the MMAs, warps 2-3 of the tiles with n = 0 add up dz's columns from
+// the same shared-memory tiles (no pass of their own over dz), warps 4-7 write
+// the partials. Bound by the operands' way through L2 (134 MB,
+// twice) and the partials (33 MB) at 32,768 rows: 43 us, against four GEMMs of
+// 16 us and 19 us of column sums.
+constexpr int WG_TILES = 14, WG_STAGES = 4, WG_ACC = 4;
 struct WgradMaps { CUtensorMap dz[4], src[4]; };
-struct WgradOut { float *dw[4], *db; };   // dw[l]: splits x 256 x (l ? 256 : 128); db: 4 x splits x 256
+struct WgradOut { float *dw[4], *db; };   // dw[l]: splits x 256 x (l ? 256 : 128); db: 4 x blocks of 256 rows x 256, or null
 struct Wg {
   static constexpr int STAGE_BYTES = 32768;
-  static constexpr int BARS = WG_STAGES * STAGE_BYTES;    // full and empty per stage, done, TMEM address
-  static constexpr int SUMS = BARS + 128;                 // 8 x 128 column sums
-  static constexpr int SMEM = 1024 + SUMS + 8 * 128 * 4;
-  static_assert(BM * SLD * 4 <= BARS, "the epilogue's tile takes the stages' place");
+  static constexpr int TILE = WG_STAGES * STAGE_BYTES;    // 4 x 32 rows of a partial on their way out
+  static constexpr int BARS = TILE + BM * SLD * 4;        // full and empty per stage, done per accumulator, TMEM address
+  static constexpr int SMEM = 1024 + BARS + 128;
   static_assert(SMEM <= 227 * 1024 && 2 * SMEM > 227 * 1024, "one CTA per SM: it takes all of TMEM");
 };
 
 __global__ void __launch_bounds__(THREADS) k_mlp_wgrad(const __grid_constant__ WgradMaps maps, const WgradOut out,
-                                                       int k_blocks) {
+                                                       int rows, int splits, int per_cta) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = saddr(smem_raw), tiles = (raw + 1023u) & ~1023u;
   unsigned char* g = smem_raw + (tiles - raw);
   const uint32_t full = tiles + Wg::BARS, empty = full + 8 * WG_STAGES, done = empty + 8 * WG_STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g + Wg::BARS + 112);
-  float* sums = reinterpret_cast<float*>(g + Wg::SUMS);
   __shared__ int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t = blockIdx.x, l = t < 12 ? 1 + (t >> 2) : 0;
   const int m_blk = (t < 12 ? (t >> 1) & 1 : t - 12) * BM, n_blk = t < 12 ? (t & 1) * 128 : 0, kin = l ? 256 : 128;
-  const int kb0 = (int)((long long)k_blocks * blockIdx.y / gridDim.y);
-  const int KT = (int)((long long)k_blocks * (blockIdx.y + 1) / gridDim.y) - kb0;   // at least 1
-  const bool bias = n_blk == 0;
+  const int c0 = blockIdx.y * per_cta, nc = min(per_cta, splits - c0);   // this CTA's ranges
+  const int KC = rows / splits / BK, kb0 = c0 * KC, KT = nc * KC;
+  const bool bias = n_blk == 0 && out.db != nullptr;
   if (tid == 0) {
     s_abort = 0;
     for (int s = 0; s < WG_STAGES; ++s) {
       mbar_init(full + 8 * s, 1);
-      mbar_init(empty + 8 * s, bias ? 5 : 1);   // the MMAs, and the four summing warps
+      mbar_init(empty + 8 * s, bias ? 3 : 1);   // the MMAs, and the two summing warps
     }
-    mbar_init(done, 1);
+    for (int q = 0; q < WG_ACC; ++q) mbar_init(done + 8 * q, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 0) {
@@ -1172,7 +1170,6 @@ __global__ void __launch_bounds__(THREADS) k_mlp_wgrad(const __grid_constant__ W
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  float col[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   int issued = 0;   // K-blocks whose loads have been issued (warp 1)
   if (warp == 1) {
     if (lane == 0) {
@@ -1194,96 +1191,94 @@ __global__ void __launch_bounds__(THREADS) k_mlp_wgrad(const __grid_constant__ W
   } else if (warp == 0) {
     if (lane == 0) {
       constexpr uint32_t idesc = instr_desc<true, true, 128>();
+      int kt = 0;
+      bool ok = true;
+      for (int q = 0; q < nc; ++q) {
+        for (int k = 0; k < KC && ok; ++k, ++kt) {
+          const int s = kt % WG_STAGES;
+          if (!mbar_wait(full + 8 * s, (uint32_t)((kt / WG_STAGES) & 1))) {
+            atomicOr(&s_abort, 1);
+            __threadfence_block();
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a = tiles + s * Wg::STAGE_BYTES, b = a + 16384;
+#pragma unroll
+          for (int j = 0; j < BK / 16; ++j)
+            umma(tmem + (uint32_t)(q * 128), smem_desc(a + j * 2048, 8192, 1024), smem_desc(b + j * 2048, 8192, 1024),
+                 idesc, (k | j) != 0);
+          umma_commit(empty + 8 * s);
+        }
+        umma_commit(done + 8 * q);   // its one phase completes when every MMA issued so far has
+      }
+    }
+    __syncwarp();
+  } else if (warp < 4) {
+    if (bias) {
+      // a thread adds two columns row by row; a warp reads the 128 bytes of one row
+      const int u = tid - 64, nblk = (rows + 255) / 256;
+      const unsigned char* col = g + (u >> 5) * 8192 + (u & 3) * 4;
+      float s0 = 0.f, s1 = 0.f;
       for (int kt = 0; kt < KT; ++kt) {
         const int s = kt % WG_STAGES;
         if (!mbar_wait(full + 8 * s, (uint32_t)((kt / WG_STAGES) & 1))) { atomicOr(&s_abort, 1); break; }
-        tc_fence_after();
-        const uint32_t a = tiles + s * Wg::STAGE_BYTES, b = a + 16384;
+        const unsigned char* p = col + s * Wg::STAGE_BYTES;
+        uint32_t v[BK];   // all on their way before the chain of additions
 #pragma unroll
-        for (int j = 0; j < BK / 16; ++j)
-          umma(tmem + (uint32_t)((kt % WG_ACC) * 128), smem_desc(a + j * 2048, 8192, 1024),
-               smem_desc(b + j * 2048, 8192, 1024), idesc, kt >= WG_ACC || j != 0);
-        umma_commit(empty + 8 * s);
+        for (int k = 0; k < BK; ++k)
+          v[k] = *reinterpret_cast<const uint32_t*>(p + (k >> 3) * 1024 + (k & 7) * 128 + ((((u >> 2) & 7) ^ (k & 7)) << 4));
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(empty + 8 * s) : "memory");
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+          s0 += __uint_as_float(v[k] << 16);
+          s1 += __uint_as_float(v[k] & 0xFFFF0000u);
+        }
+        const int kb = kb0 + kt;
+        if ((kb & 3) == 3 || kb == rows / BK - 1) {
+          *reinterpret_cast<float2*>(out.db + ((size_t)l * nblk + (kb >> 2)) * 256 + m_blk + 2 * u) = make_float2(s0, s1);
+          s0 = s1 = 0.f;
+        }
       }
-      umma_commit(done);   // its one phase completes when every MMA issued so far has
     }
-    __syncwarp();
-  } else if (warp >= 4 && bias) {
-    // thread: columns 8 (2-group, chunk) .. + 7 and the rows k % 8 of each K-block,
-    // summed per K-block first; a warp reads 512 consecutive bytes
-    const int u = tid - 128, r8 = (u >> 3) & 7, c = u & 7;
-    for (int kt = 0; kt < KT; ++kt) {
-      const int s = kt % WG_STAGES;
-      if (!mbar_wait(full + 8 * s, (uint32_t)((kt / WG_STAGES) & 1))) { atomicOr(&s_abort, 1); break; }
-      const unsigned char* p = g + s * Wg::STAGE_BYTES + (u >> 6) * 8192 + r8 * 128 + ((c ^ r8) << 4);
-      float b[8];
+  } else {
+    const int wq = warp & 3;
+    float* stile = reinterpret_cast<float*>(g + Wg::TILE) + wq * 32 * SLD;
+    for (int q = 0; q < nc; ++q) {
+      if (!mbar_wait(done + 8 * q, 0)) atomicOr(&s_abort, 1);
+      if (__any_sync(0xffffffffu, *(volatile int*)&s_abort)) break;
+      tc_fence_after();
+#pragma unroll 2
+      for (int cc = 0; cc < 128; cc += 16) {
+        uint32_t v[16];
+        tmem_ld16(tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(q * 128 + cc), v);
+        uint4* dst = reinterpret_cast<uint4*>(stile + lane * SLD + cc);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        float v[8];
-        load8<true>(reinterpret_cast<const bf16*>(p + k * 1024), v);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) b[i] = k ? b[i] + v[i] : v[i];
+        for (int i = 0; i < 4; ++i) dst[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
       }
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(empty + 8 * s) : "memory");
-#pragma unroll
-      for (int i = 0; i < 8; ++i) col[i] += b[i];
+      float* dw = out.dw[l] + ((size_t)(c0 + q) * 256 + m_blk + wq * 32) * kin + n_blk + lane * 4;
+#pragma unroll 8
+      for (int r = 0; r < 32; ++r)
+        *reinterpret_cast<float4*>(dw + (size_t)r * kin) = *reinterpret_cast<const float4*>(stile + r * SLD + lane * 4);
+      __syncwarp();
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sums[r8 * 128 + (u >> 6) * 64 + c * 8 + i] = col[i];
+    tc_fence_before();
   }
-  const bool done_ok = mbar_wait(done, 0);
-  if (!done_ok) atomicOr(&s_abort, 1);
   __syncthreads();
+  // A wait gave up: loads that may still be landing and the MMAs issued get a
+  // bounded wait each; the partials are not complete and the host sees the flag.
   if (s_abort) {
-    // A wait gave up: nothing is written. Loads that may still be landing get
-    // a bounded wait each; the accumulators are released once the MMAs issued
-    // have finished.
     if (warp == 1 && lane == 0)
       for (int j = max(0, issued - WG_STAGES); j < issued; ++j)
         mbar_wait(full + 8 * (j % WG_STAGES), (uint32_t)((j / WG_STAGES) & 1));
+    if (warp == 0) mbar_wait(done + 8 * (nc - 1), 0);
     __syncthreads();
-    if (warp == 0) {
-      if (!done_ok) mbar_wait(done, 0);
-      __syncwarp();
-      tc_fence_after();
-      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(WG_ACC * 128));
-    }
-    return;
   }
-  tc_fence_after();
-  float* stile = reinterpret_cast<float*>(g);
-  {
-    const int wq = warp & 3, r = wq * 32 + lane, na = min(KT, WG_ACC);
-#pragma unroll 1
-    for (int cc = (warp >> 2) * 64; cc < (warp >> 2) * 64 + 64; cc += 16) {
-      uint32_t v[16];
-      float x[16];
-      for (int q = 0; q < na; ++q) {
-        tmem_ld16(tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(q * 128 + cc), v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = q ? x[i] + __uint_as_float(v[i]) : __uint_as_float(v[i]);
-      }
-      float4* dst = reinterpret_cast<float4*>(stile + r * SLD + cc);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) dst[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
   if (warp == 0) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(WG_ACC * 128));
-  }
-  float* dw = out.dw[l] + (size_t)blockIdx.y * 256 * kin + (size_t)m_blk * kin + n_blk;
-#pragma unroll 4
-  for (int q = tid; q < BM * 32; q += THREADS)
-    *reinterpret_cast<float4*>(dw + (size_t)(q >> 5) * kin + (q & 31) * 4) =
-        *reinterpret_cast<const float4*>(stile + (q >> 5) * SLD + (q & 31) * 4);
-  if (bias && tid < 128) {
-    float v = sums[tid];
-    for (int k = 1; k < 8; ++k) v += sums[k * 128 + tid];
-    out.db[((size_t)l * gridDim.y + blockIdx.y) * 256 + m_blk + tid] = v;
   }
 }
 
@@ -1464,10 +1459,12 @@ int esr_mlp_forward(const esr_mlp_net* net, const void* X, int32_t rows, const f
 
 int esr_mlp_wgrad(const void* const* dz, const void* const* src, int32_t rows, int32_t splits, float* const* dw, float* db,
                   void* stream) {
-  if (!dz || !src || !dw || !db || rows <= 0 || rows % 128)
+  if (!dz || !src || !dw || rows <= 0 || rows % 128)
     return mfail(ESR_ERR_ARG, "mlp_wgrad: rows must be a multiple of 128");
-  if (splits < 1 || splits > rows / tc::BK || splits > 65535)
-    return mfail(ESR_ERR_ARG, "mlp_wgrad: between 1 and rows / 64 splits");
+  if (splits < 1 || splits > 65535 || rows % (tc::BK * (int64_t)splits))
+    return mfail(ESR_ERR_ARG, "mlp_wgrad: rows must be a multiple of 64 x splits");
+  if (db && (splits > 1 && rows / splits % 256 || !aligned16(db)))
+    return mfail(ESR_ERR_ARG, "mlp_wgrad: column sums need splits of whole 256-row blocks");
   tc::WgradMaps maps;
   tc::WgradOut out{};
   out.db = db;
@@ -1484,7 +1481,10 @@ int esr_mlp_wgrad(const void* const* dz, const void* const* src, int32_t rows, i
   static const cudaError_t attr =
       cudaFuncSetAttribute(tc::k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::Wg::SMEM);
   if (attr != cudaSuccess) return mfail(ESR_ERR_CUDA, std::string("mlp_wgrad: ") + cudaGetErrorString(attr));
-  tc::k_mlp_wgrad<<<dim3(tc::WG_TILES, splits), tc::THREADS, tc::Wg::SMEM, (cudaStream_t)stream>>>(maps, out, rows / tc::BK);
+  // as many ranges per CTA as keep the launch to one CTA per SM, at most one per accumulator
+  const int per = std::min(tc::WG_ACC, (splits + 148 / tc::WG_TILES - 1) / (148 / tc::WG_TILES));
+  tc::k_mlp_wgrad<<<dim3(tc::WG_TILES, (splits + per - 1) / per), tc::THREADS, tc::Wg::SMEM, (cudaStream_t)stream>>>(
+      maps, out, rows, splits, per);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, std::string("mlp_wgrad: ") + cudaGetErrorString(err));
 }
@@ -1590,6 +1590,80 @@ int esr_reduce_many(const esr_reduction* sets, int32_t n_sets, void* stream) {
   k_reduce_splits<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(q);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, cudaGetErrorString(err));
+}
+
+// Workspace of esr_mlp_backward, each part on 256 bytes
+struct BackwardWork {
+  static constexpr int RPB = 256;   // rows per partial of the head's gradients and of the bias gradients
+  int splits = 1, head_blocks;
+  bool sums_with_wgrad;             // a range is whole 256-row blocks
+  size_t dz[4], dh, dw[4], db, head, bytes;
+  explicit BackwardWork(int rows) {
+    // ranges of at least 1,024 rows
+    while (splits < 64 && rows % (tc::BK * splits * 2) == 0 && rows / (splits * 2) >= 1024) splits *= 2;
+    sums_with_wgrad = splits == 1 || rows / splits % RPB == 0;
+    head_blocks = (rows + RPB - 1) / RPB;
+    size_t at = 0;
+    auto take = [&](size_t n) { const size_t o = at; at += (n + 255) / 256 * 256; return o; };
+    for (auto& o : dz) o = take((size_t)rows * 256 * sizeof(bf16));
+    dh = take((size_t)rows * 256 * sizeof(bf16));
+    for (int l = 0; l < 4; ++l) dw[l] = take((size_t)splits * 256 * (l ? 256 : 128) * sizeof(float));
+    db = take((size_t)4 * head_blocks * 256 * sizeof(float));
+    head = take((size_t)head_blocks * (4 * 256 + 4) * sizeof(float));
+    bytes = at;
+  }
+};
+
+int64_t esr_mlp_backward_workspace(int32_t rows) {
+  return rows > 0 && rows % 128 == 0 ? (int64_t)BackwardWork(rows).bytes : -1;
+}
+
+int esr_mlp_backward(const esr_mlp_net* net, const void* X, int32_t rows, const float* dY, const void* const* h,
+                     const void* const* z, void* work, const esr_mlp_grads* out, void* stream) {
+  if (!net || !X || !dY || !h || !z || !work || !out || !net->W4 || !out->W4 || !out->b4)
+    return mfail(ESR_ERR_ARG, "mlp_backward: null operand");
+  if (rows <= 0 || rows % 128) return mfail(ESR_ERR_ARG, "mlp_backward: rows must be a multiple of 128");
+  for (int l = 0; l < 4; ++l) {
+    if (!h[l] || !z[l] || !out->W[l] || !out->b[l] || (l && !net->W[l])) return mfail(ESR_ERR_ARG, "mlp_backward: null operand");
+    if (!aligned16(h[l]) || !aligned16(z[l]) || (l && !aligned16(net->W[l])))
+      return mfail(ESR_ERR_ARG, "mlp_backward: operands must be 16-byte aligned");
+  }
+  if (!aligned16(work)) return mfail(ESR_ERR_ARG, "mlp_backward: the workspace must be 16-byte aligned");
+  const BackwardWork at(rows);
+  char* base = static_cast<char*>(work);
+  auto f32 = [&](size_t o) { return reinterpret_cast<float*>(base + o); };
+  void* dz[4];
+  for (int l = 0; l < 4; ++l) dz[l] = base + at.dz[l];
+  bf16* dh = reinterpret_cast<bf16*>(base + at.dh);
+  int rc = esr_mlp_head_bwd(dY, h[3], z[3], rows, 256, net->W4, dh, dz[3], f32(at.head), BackwardWork::RPB, stream);
+  // dh_{l-1} = dh_l + dz_l W_l, in place: an element is read and written by one
+  // thread. dh_0 has no reader, only its dz_0 is written.
+  for (int l = 3; l > 0 && rc == ESR_OK; --l) {
+    const Epi e{nullptr, dh, (const bf16*)z[l - 1], l > 1 ? dh : nullptr, (bf16*)dz[l - 1], 256, (long long)rows * 256, true};
+    rc = launch_gemm_tc<false, true, EPI_BWD>(rows, 256, 256, 1, (const bf16*)dz[l], 256, (const bf16*)net->W[l], 256, e,
+                                              (cudaStream_t)stream);
+  }
+  if (rc != ESR_OK) return rc;
+  const void* src[4] = {X, h[0], h[1], h[2]};
+  float* dw[4];
+  for (int l = 0; l < 4; ++l) dw[l] = f32(at.dw[l]);
+  rc = esr_mlp_wgrad(dz, src, rows, at.splits, dw, at.sums_with_wgrad ? f32(at.db) : nullptr, stream);
+  const size_t db_layer = (size_t)at.head_blocks * 256;
+  if (!at.sums_with_wgrad)
+    for (int l = 0; l < 4 && rc == ESR_OK; ++l)
+      rc = esr_colsum_bf16(dz[l], rows, 256, BackwardWork::RPB, f32(at.db) + l * db_layer, stream);
+  if (rc != ESR_OK) return rc;
+  esr_reduction sums[10];
+  int n = 0;
+  const int64_t hs = 4 * 256 + 4;
+  sums[n++] = {f32(at.head), out->W4, hs, 4 * 256, at.head_blocks, 0};
+  sums[n++] = {f32(at.head) + 4 * 256, out->b4, hs, 4, at.head_blocks, 0};
+  for (int l = 0; l < 4; ++l) {
+    const int64_t m = 256 * (l ? 256 : 128);
+    sums[n++] = {dw[l], out->W[l], m, m, at.splits, 0};
+    sums[n++] = {f32(at.db) + l * db_layer, out->b[l], 256, 256, at.head_blocks, 0};
+  }
+  return esr_reduce_many(sums, n, stream);
 }
 
 int esr_colsum_bf16(const void* X, int32_t rows, int32_t C, int32_t rpb, float* part, void* stream) {

@@ -25,9 +25,6 @@ K_IN = 128      # padded input width (13 features used)
 H = 256
 N_OUT = 4
 ROW_TILE = 128  # the GEMM tiles rows by 128
-# ranges of rows of the batched weight gradients: with 14 tiles per range, one
-# block per SM; fewer where a range would have less than 256 rows
-WGRAD_SPLITS = 10
 
 
 def _p(t):
@@ -146,12 +143,15 @@ class MLP:
 
     def _net(self):
         """The network's device addresses (the flat vectors may be replaced between calls)."""
-        at = lambda name, bf16: (self.pb.data_ptr() + 2 * self.offsets[name][0] if bf16
-                                 else self.p.data_ptr() + 4 * self.offsets[name][0])
+        return self._addresses(self.p, self.pb)
+
+    def _addresses(self, flat, weights=None):
+        """Device addresses of every weight and bias in `flat`; those of W0..W3 in the BF16 copy, if given."""
+        p, w = flat.data_ptr(), (4, flat.data_ptr()) if weights is None else (2, weights.data_ptr())
         n = F.MlpNet()
-        n.W[:] = [at(f"W{l}", True) for l in range(4)]
-        n.b[:] = [at(f"b{l}", False) for l in range(4)]
-        n.W4, n.b4 = at("W4", False), at("b4", False)
+        n.W[:] = [w[1] + w[0] * self.offsets[f"W{l}"][0] for l in range(4)]
+        n.b[:] = [p + 4 * self.offsets[f"b{l}"][0] for l in range(4)]
+        n.W4, n.b4 = p + 4 * self.offsets["W4"][0], p + 4 * self.offsets["b4"][0]
         return n
 
     # ----------------------------------------------------------- backward
@@ -160,11 +160,13 @@ class MLP:
         X, h, z = acts["X"], acts["h"], acts["z"]
         rows = X.shape[0]
         st = _stream()
-        # the weight gradients of all layers in one launch, unless a caller sets the split of each GEMM
-        batched = self.fused and splits is None
-        if batched:
-            splits = max(1, min(WGRAD_SPLITS, rows // 256))
-        elif splits is None:
+        if self.fused and splits is None:
+            work = self._buf("backward", (self.L.esr_mlp_backward_workspace(rows),), torch.uint8)
+            F.check(self.L.esr_mlp_backward(C.byref(self._net()), _p(X), rows, _p(dY), _array(h), _array(z), _p(work),
+                                            C.byref(self._addresses(self.g)), st))
+            return
+        # layer by layer: the mma.sync kernel, or a split of the weight gradients set by the caller
+        if splits is None:
             splits = 1
             while splits < 64 and rows % (64 * splits * 2) == 0 and rows // (splits * 2) >= 1024:
                 splits *= 2
@@ -179,25 +181,21 @@ class MLP:
         # W4 and b4 are contiguous in the flat layout, as in the partials
         sums = [(part_head, nblk, 4 * H + 4, 4 * H + 4, self.gview("W4"))]
         part = self._buf("part_w", (4, splits, H, H), torch.float32)
-        n_col = splits if batched else nblk
-        cpart = self._buf("part_c", (4, n_col, H), torch.float32)
+        cpart = self._buf("part_c", (4, nblk, H), torch.float32)
         for l in (3, 2, 1, 0):
             kin = K_IN if l == 0 else H
             src = X if l == 0 else h[l - 1]
             # weight gradient dW_l = dz_l^T src (split-K over rows, fixed-order reduction)
-            if not batched:
-                F.check(self.gemm(1, 1, H, kin, rows, _p(dz), H, _p(src), kin, 0, None, None, None,
-                                  _p(part[l]), None, kin, splits, st))
+            F.check(self.gemm(1, 1, H, kin, rows, _p(dz), H, _p(src), kin, 0, None, None, None,
+                                         _p(part[l]), None, kin, splits, st))
             sums.append((part[l], splits, H * kin, H * kin, self.gview(f"W{l}")))
-            sums.append((cpart[l], n_col, H, H, self.gview(f"b{l}")))
+            sums.append((cpart[l], nblk, H, H, self.gview(f"b{l}")))
             if l > 0:
                 dh_prev, dz_prev = self._buf(f"dh{l - 1}", (rows, H), torch.bfloat16), dzs[l - 1]
                 F.check(self.gemm(0, 1, rows, H, H, _p(dz), H, _p(self.view(f"W{l}", True)), H, 2,
                                              None, _p(dh), _p(z[l - 1]), _p(dh_prev), _p(dz_prev), H, 1, st))
                 dh, dz = dh_prev, dz_prev
-        if batched:
-            F.check(self.L.esr_mlp_wgrad(_array(dzs), _array([X, *h[:3]]), rows, splits, _array(part), _p(cpart), st))
-        elif rows % rpb == 0:
+        if rows % rpb == 0:
             F.check(self.L.esr_colsum_bf16(_p(dzs), 4 * rows, H, rpb, _p(cpart), st))
         else:   # a row block would span two layers
             for l in range(4):

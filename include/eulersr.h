@@ -491,13 +491,29 @@ typedef struct esr_reduction {
 } esr_reduction;
 int esr_reduce_many(const esr_reduction* sets, int32_t n_sets, void* stream);
 /* Weight and bias gradients of the four 256-wide layers in one launch
- * (tcgen05), as partials over `splits` ranges of rows (1 <= splits <= rows /
- * 64, rows a multiple of 128): dw[l] FP32 [splits x 256 x kin] = dz[l]^T
- * src[l] and db FP32 [4 x splits x 256] = column sums of dz[l]. dz[l] BF16
- * [rows x 256]; src[0] BF16 [rows x 128] (kin 128), src[1..3] BF16 [rows x 256]
- * (kin 256). Its pipeline waits are bounded (esr_gemm_tc_status). */
+ * (tcgen05): dw[l] FP32 [splits x 256 x kin] = dz[l]^T src[l] over `splits`
+ * equal ranges of rows (rows a multiple of 128 and of 64 x splits), the sums of
+ * esr_gemm_bf16; db, unless NULL, FP32 [4 x ceil(rows / 256) x 256] = column
+ * sums of dz[l] per 256 rows, the sums of esr_colsum_bf16 (splits 1, or ranges
+ * of whole 256-row blocks). dz[l] BF16 [rows x 256]; src[0] BF16 [rows x 128]
+ * (kin 128), src[1..3] BF16 [rows x 256] (kin 256). Its pipeline waits are
+ * bounded (esr_gemm_tc_status). */
 int esr_mlp_wgrad(const void* const* dz, const void* const* src, int32_t rows, int32_t splits, float* const* dw,
                   float* db, void* stream);
+/* The whole backward pass in one call: from dY = d loss / d y (FP32 [rows x 4])
+ * and the h, z that esr_mlp_forward kept, the gradients of every weight and
+ * bias (FP32, the shapes of esr_mlp_net). `work`: esr_mlp_backward_workspace
+ * bytes of device memory (-1 for rows that are not a multiple of 128), owned by
+ * one call at a time. */
+typedef struct esr_mlp_grads {
+    float* W[4];
+    float* b[4];
+    float* W4;
+    float* b4;
+} esr_mlp_grads;
+int64_t esr_mlp_backward_workspace(int32_t rows);
+int esr_mlp_backward(const esr_mlp_net* net, const void* X, int32_t rows, const float* dY, const void* const* h,
+                     const void* const* z, void* work, const esr_mlp_grads* out, void* stream);
 int esr_colsum_bf16(const void* X, int32_t rows, int32_t C, int32_t rpb, float* part, void* stream);
 /* AdamW on FP32 master weights, refreshing an optional BF16 copy */
 int esr_adamw(float* p, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2, float eps,

@@ -386,30 +386,57 @@ def test_warm_inputs_equal_separate_calls(rows, rows_out):
         assert torch.equal(torch.nan_to_num(b0, 99.0), torch.nan_to_num(b1, 99.0))
 
 
-@pytest.mark.parametrize("rows,splits", [(128, 1), (128, 2), (384, 1), (640, 3), (1152, 5), (4224, 10), (4224, 66)])
-def test_batched_weight_gradients_match_float64(rows, splits):
-    """esr_mlp_wgrad at one K-block per range, fewer K-blocks than accumulators,
-    ranges of unequal length and rings that wrap: dW_l = dz_l^T src_l and db_l
-    against float64 sums of the same BF16 values. A float32 sum of n products
-    is within n ulp (2^-23, whatever the order) of the sum of magnitudes."""
+@pytest.mark.parametrize("rows,splits", [(128, 1), (384, 1), (640, 2), (1024, 4), (1152, 9), (2816, 11), (5632, 22), (2688, 42)])
+def test_batched_weight_gradients_equal_layer_calls(rows, splits):
+    """esr_mlp_wgrad at one K-block per range, one to four ranges per block, a
+    block with fewer, more ranges than fit one wave, and rings that wrap: the
+    bits of the split-K GEMM and of the column sums of each layer."""
     import torch
     from eulersr_b200 import _ffi as F
     g = torch.Generator().manual_seed(rows + splits)
     rnd = lambda *s: (torch.randn(*s, generator=g) + 0.25).to(torch.bfloat16).cuda()
     dz = [rnd(rows, 256) for _ in range(4)]
     src = [rnd(rows, 128)] + [rnd(rows, 256) for _ in range(3)]
-    dw = [torch.full((splits, 256, s.shape[1]), float("nan"), device="cuda") for s in src]
-    db = torch.full((4, splits, 256), float("nan"), device="cuda")
+    nblk = (rows + 255) // 256
+    sums = splits == 1 or rows // splits % 256 == 0
+    new = lambda: ([torch.full((splits, 256, s.shape[1]), float("nan"), device="cuda") for s in src],
+                   torch.full((4, nblk, 256), float("nan"), device="cuda"))
+    dw, db = new()
+    want, wantb = new()
     arr = lambda ts: (C.c_void_p * 4)(*[t.data_ptr() for t in ts])
+    p = lambda t: C.c_void_p(t.data_ptr())
     st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
-    F.check(F.lib().esr_mlp_wgrad(arr(dz), arr(src), rows, splits, arr(dw), C.c_void_p(db.data_ptr()), st))
-    tol = rows * 2.0 ** -23
+    L = F.lib()
+    F.check(L.esr_mlp_wgrad(arr(dz), arr(src), rows, splits, arr(dw), p(db) if sums else None, st))
     for l in range(4):
-        a, b = dz[l].double(), src[l].double()
-        assert torch.all((dw[l].double().sum(0) - a.T @ b).abs() <= tol * (a.abs().T @ b.abs()))
-        assert torch.all((db[l].double().sum(0) - a.sum(0)).abs() <= tol * a.abs().sum(0))
+        kin = src[l].shape[1]
+        F.check(L.esr_gemm_bf16(1, 1, 256, kin, rows, p(dz[l]), 256, p(src[l]), kin, 0, None, None, None, p(want[l]), None,
+                                kin, splits, st))
+        F.check(L.esr_colsum_bf16(p(dz[l]), rows, 256, 256, p(wantb[l]), st))
+        assert torch.equal(dw[l], want[l])
+    assert torch.equal(db, wantb) if sums else True
     bad = C.c_int32(-1)
-    F.check(F.lib().esr_gemm_tc_status(C.byref(bad)))
+    F.check(L.esr_gemm_tc_status(C.byref(bad)))
     assert bad.value == 0
-    for bad_rows, bad_splits in ((rows + 64, 1), (rows, 0), (rows, rows // 64 + 1)):
-        assert F.lib().esr_mlp_wgrad(arr(dz), arr(src), bad_rows, bad_splits, arr(dw), C.c_void_p(db.data_ptr()), st) != 0
+    for r, s in ((rows + 64, 1), (rows, 0), (rows, rows // 64 + 1)):
+        assert L.esr_mlp_wgrad(arr(dz), arr(src), r, s, arr(dw), None, st) != 0
+
+
+@pytest.mark.parametrize("rows", [128, 384, 2048, 2688, 4352])
+def test_backward_in_one_call_equals_layer_calls(rows):
+    """esr_mlp_backward (in-place dh, one weight-gradient launch, with the
+    column sums in it or, where a range is no whole number of 256-row blocks,
+    beside it) gives the bits of the layer-by-layer calls."""
+    import torch
+    m, X, base, tgt, w, inv_den = _setup(rows=rows, seed=9)
+    y, acts = m.forward(X, base, keep=True)
+    _, dpred = m.loss(y, tgt, w, inv_den)
+    splits = 1
+    while rows % (128 * splits) == 0 and rows // (splits * 2) >= 1024:
+        splits *= 2
+    m.backward(acts, dpred, splits=splits)
+    want = m.g.clone()
+    m.g.fill_(float("nan"))
+    m.backward(acts, dpred)
+    assert torch.equal(m.g, want)
+    assert m.L.esr_mlp_backward_workspace(rows + 64) == -1
