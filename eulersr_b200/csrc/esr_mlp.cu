@@ -921,16 +921,18 @@ __global__ void __launch_bounds__(THREADS) k_gemm_tc(int M, int N, int K_split, 
 //   A   per tile 128 x 256 BF16 activations, K-major with the 128-byte swizzle
 //       (64 KB); layer l's MMAs read h_{l-1} there and its epilogue replaces
 //       it by h_l
-//   W   a ring of 64-wide K-blocks of the weights (32 KB each, by TMA): the 14
-//       blocks of the four layers run through it without a stop, so the next
-//       layer's first blocks arrive during the epilogue
-// One thread issues loads and tcgen05.mma; 8 warps per tile read the
+//   W   a ring of 64-wide K-blocks of the weights (32 KB each, by TMA), streamed
+//       through for every layer of every tile
+// One warp loads, one issues tcgen05.mma, 8 warps per tile read the
 // accumulators back (warp w of a tile: rows 32 (w % 4) .., columns 128 (w / 4)
 // ..), add bias and residual and round as the layer-by-layer GEMM does; the
 // head ends in the summation order of k_head_fwd. Inference moves 272 B per
 // row instead of 4.4 KB and is one launch instead of five; a training forward
-// also writes h and z. What bounds it is bringing 448 KB of weights to every
-// CTA: two tiles share them once there are more tiles than SMs.
+// also writes h and z. Two tiles take turns: one's MMAs (2,400 cycles a layer)
+// run while the other's epilogue (6,000; 15,000 with h and z on their way to
+// memory) does. Inference of 25,984 rows takes 36 us and a training
+// forward of 32,768 rows 58, 40 and 63 with both tiles in step and a head of
+// 160 shuffles per 8 rows (14,400 of 61,000 cycles), 98 and 84 layer by layer.
 struct MlpMaps { CUtensorMap x, w[4]; };
 struct MlpNet {
   const float* b[4];
@@ -939,15 +941,14 @@ struct MlpNet {
   bf16 *h[4], *z[4];       // null: not kept
   int rows;
 };
-constexpr int FWD_BLOCKS = 14;                 // K-blocks of the four layers: 2 + 4 + 4 + 4
 template <bool KEEP, int TILES>
 struct Fwd {
   static constexpr int STAGES = TILES == 1 ? 4 : KEEP ? 2 : 3;
   static constexpr int W = TILES * 65536;                  // after the activations
-  static constexpr int BARS = W + STAGES * 32768;          // X, done, full and empty per stage, TMEM address
+  static constexpr int BARS = W + STAGES * 32768;          // X, done and ready per tile, full and empty per stage, TMEM address
   static constexpr int TURN = BARS + 128;                  // kept forward: 2 KB per warp to turn z's rows around
   static constexpr int SMEM = 1024 + TURN + (KEEP ? TILES * 8 * 2048 : 0);
-  static constexpr int THREADS = TILES * 256;
+  static constexpr int THREADS = TILES * 256 + 64;         // epilogues, MMA issuer, loader
   static_assert(SMEM <= 227 * 1024, "one CTA per SM");
 };
 
@@ -964,14 +965,18 @@ __global__ void __launch_bounds__((Fwd<KEEP, TILES>::THREADS)) k_mlp_fwd(const _
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = saddr(smem_raw), A = (raw + 1023u) & ~1023u, Wt = A + C::W;
   unsigned char* g = smem_raw + (A - raw);
-  const uint32_t xfull = A + C::BARS, done = xfull + 8, full = done + 8, empty = full + 8 * S;
+  const uint32_t xfull = A + C::BARS, done = xfull + 8, ready = done + 8 * TILES, full = ready + 8 * TILES;
+  const uint32_t empty = full + 8 * S;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(g + C::BARS + 112);
-  __shared__ int s_abort;
+  __shared__ int s_abort;   // set when a wait gave up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, m0 = blockIdx.x * (TILES * 128);
   if (tid == 0) {
     s_abort = 0;
     mbar_init(xfull, 1);
-    mbar_init(done, 1);
+    for (int t = 0; t < TILES; ++t) {
+      mbar_init(done + 8 * t, 1);
+      mbar_init(ready + 8 * t, 8);
+    }
     for (int k = 0; k < S; ++k) {
       mbar_init(full + 8 * k, 1);
       mbar_init(empty + 8 * k, 1);
@@ -987,72 +992,65 @@ __global__ void __launch_bounds__((Fwd<KEEP, TILES>::THREADS)) k_mlp_fwd(const _
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  constexpr uint32_t idesc = instr_desc<false, false, 256>();
-  // thread 0: K-block i of the 14 into its stage
-  int loaded = 0, landed = 0;
-  bool x_landed = false;
-  auto load = [&]() {
-    const int i = loaded++, l = i < 2 ? 0 : 1 + (i - 2) / 4, kb = i < 2 ? i : (i - 2) % 4;
-    mbar_expect_tx(full + 8 * (i % S), 32768);
-    tma_load_2d(Wt + (i % S) * 32768, &maps.w[l], kb * 64, 0, full + 8 * (i % S));
-  };
-  if (tid == 0) {
-    mbar_expect_tx(xfull, TILES * 32768);
-    for (int t = 0; t < TILES; ++t)
-      for (int kb = 0; kb < 2; ++kb) tma_load_2d(A + t * 65536 + kb * 16384, &maps.x, kb * 64, m0 + t * 128, xfull);
-    while (loaded < S) load();
-  }
-#pragma unroll 1
-  for (int l = 0; l < 4; ++l) {
-    const int KB = l == 0 ? 2 : 4, first = l == 0 ? 0 : 4 * l - 2;
-    bool ok = true;
-    if (tid == 0) {
-      if (l == 0) { ok = mbar_wait(xfull, 0); x_landed = ok; }
-      for (int kb = 0; kb < KB && ok; ++kb) {
-        const int i = first + kb, st = i % S;
-        ok = mbar_wait(full + 8 * st, (uint32_t)((i / S) & 1));
-        if (!ok) break;
-        landed = i + 1;
-        tc_fence_after();
-#pragma unroll
-        for (int t = 0; t < TILES; ++t)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            umma(tmem + t * 256, smem_desc(A + t * 65536 + kb * 16384 + j * 32, 16, 1024),
-                 smem_desc(Wt + st * 32768 + j * 32, 16, 1024), idesc, (kb | j) != 0);
-        umma_commit(empty + 8 * st);
-        // refill the stage that the previous K-block's MMAs read
-        if (kb >= 1 && loaded < FWD_BLOCKS && loaded == i - 1 + S) {
-          ok = mbar_wait(empty + 8 * ((i - 1) % S), (uint32_t)(((i - 1) / S) & 1));
-          if (ok) load();
+  int issued = 0;   // K-blocks whose loads have been issued (loader)
+  auto gave_up = [&]() { return *(volatile int*)&s_abort != 0; };
+  if (warp == TILES * 8 + 1) {   // loader: X, then the K-blocks of every layer, tile by tile
+    if (lane == 0) {
+      mbar_expect_tx(xfull, TILES * 32768);
+      for (int t = 0; t < TILES; ++t)
+        for (int kb = 0; kb < 2; ++kb) tma_load_2d(A + t * 65536 + kb * 16384, &maps.x, kb * 64, m0 + t * 128, xfull);
+      bool ok = true;
+      for (int l = 0; l < 4 && ok; ++l)
+        for (int i = 0; i < TILES * (l ? 4 : 2); ++i) {
+          const int st = issued % S;
+          if (issued >= S && (!mbar_wait(empty + 8 * st, (uint32_t)((issued / S - 1) & 1)) || gave_up())) {
+            atomicOr(&s_abort, 1);
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(full + 8 * st, 32768);
+          tma_load_2d(Wt + st * 32768, &maps.w[l], (i & (l ? 3 : 1)) * 64, 0, full + 8 * st);
+          ++issued;
         }
-      }
-      umma_commit(done);   // completes once every MMA issued so far has
     }
     __syncwarp();
-    const bool mma_ok = mbar_wait(done, (uint32_t)(l & 1));
-    if (!ok || !mma_ok) atomicOr(&s_abort, 1);
-    __syncthreads();
-    if (s_abort) {
-      // A wait gave up: nothing more is written. Loads still landing in shared
-      // memory get a bounded wait each, the accumulators are released.
-      if (tid == 0) {
-        if (!x_landed) mbar_wait(xfull, 0);
-        for (int i = landed; i < loaded; ++i) mbar_wait(full + 8 * (i % S), (uint32_t)((i / S) & 1));
-      }
-      __syncthreads();
-      if (warp == 0) {
-        if (!mma_ok) mbar_wait(done, (uint32_t)(l & 1));
-        __syncwarp();
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TILES * 256));
-      }
-      return;
+  } else if (warp == TILES * 8) {   // MMA issuer
+    if (lane == 0) {
+      constexpr uint32_t idesc = instr_desc<false, false, 256>();
+      bool ok = mbar_wait(xfull, 0);
+      int i = 0;
+      for (int l = 0; l < 4; ++l)
+        for (int t = 0; t < TILES; ++t) {
+          // h_{l-1} is in place and the accumulator has been read
+          if (ok && l > 0) ok = mbar_wait(ready + 8 * t, (uint32_t)((l - 1) & 1)) && !gave_up();
+          tc_fence_after();
+          for (int kb = 0; kb < (l ? 4 : 2) && ok; ++kb, ++i) {
+            const int st = i % S;
+            ok = mbar_wait(full + 8 * st, (uint32_t)((i / S) & 1));
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              umma(tmem + t * 256, smem_desc(A + t * 65536 + kb * 16384 + j * 32, 16, 1024),
+                   smem_desc(Wt + st * 32768 + j * 32, 16, 1024), idesc, (kb | j) != 0);
+            umma_commit(empty + 8 * st);
+          }
+          if (!ok) {
+            atomicOr(&s_abort, 1);
+            __threadfence_block();
+          }
+          umma_commit(done + 8 * t);   // completes once every MMA issued so far has
+        }
     }
+    __syncwarp();
+  } else {
+  const int t = warp >> 3;
+#pragma unroll 1
+  for (int l = 0; l < 4; ++l) {
+    if (!mbar_wait(done + 8 * t, (uint32_t)(l & 1))) atomicOr(&s_abort, 1);
+    if (__any_sync(0xffffffffu, gave_up())) break;
     tc_fence_after();
-    if (tid == 0)   // every MMA so far is done: all stages are free
-      while (loaded < FWD_BLOCKS && loaded < first + KB + S) load();
-    const int t = warp >> 3, row = (warp & 3) * 32 + lane, col0 = ((warp >> 2) & 1) * 128;
+    const int row = (warp & 3) * 32 + lane, col0 = ((warp >> 2) & 1) * 128;
     const uint32_t acc = tmem + (uint32_t)(t * 256) + ((uint32_t)((warp & 3) * 32) << 16);
     unsigned char* act = g + t * 65536;
     unsigned char* turn = g + C::TURN + warp * 2048;
@@ -1100,39 +1098,72 @@ __global__ void __launch_bounds__((Fwd<KEEP, TILES>::THREADS)) k_mlp_fwd(const _
     }
     tc_fence_before();
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // h_l before the next layer's MMAs read it
-    __syncthreads();
-    tc_fence_after();
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(ready + 8 * t) : "memory");
   }
-  if (warp == 0)   // every tcgen05.ld has completed
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TILES * 256));
-  // head: a warp sums 16 rows, a lane the columns lane + 32 i in order
-  float w[4][8];
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) w[j][i] = net.w4[j * 256 + lane + 32 * i];
-  const float bias = net.b4[lane & 3];
-  const unsigned char* act = g + (warp >> 3) * 65536;
-#pragma unroll 2
-  for (int q = 0; q < 16; ++q) {
-    const int r = (warp & 7) * 16 + q;
-    const long long row = m0 + (warp >> 3) * 128 + r;
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
+  // h_3 of the tile is in place once its 8 warps are here
+  asm volatile("bar.sync %0, 256;\n" ::"r"(1 + t) : "memory");
+  // head: a warp sums 16 rows, 8 at a time; a lane the columns lane + 32 i in
+  // order. The 32 sums over lanes of a pass (8 rows x 4 outputs) halve their
+  // number at each step of the butterfly (31 shuffles instead of 160; the
+  // pairs added are those of k_head_fwd), so that each lane ends with one.
+  if (!__any_sync(0xffffffffu, gave_up())) {
+    float2 w01[8], w23[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int k = lane + 32 * i;
-      const float v = __bfloat162float(reinterpret_cast<const bf16*>(act + act_chunk(r, k >> 3))[k & 7]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s[j] += v * w[j][i];
+      const int c = lane + 32 * i;
+      w01[i] = make_float2(net.w4[c], net.w4[256 + c]);
+      w23[i] = make_float2(net.w4[512 + c], net.w4[768 + c]);
     }
+    const float bias = net.b4[lane & 3];
+    const unsigned char* act = g + t * 65536;
+#pragma unroll 1
+    for (int q = 0; q < 16; q += 8) {
+      float s[32];   // row q + (k >> 2), output k & 3
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+      for (int k = 0; k < 8; ++k) {
+        const int r = (warp & 7) * 16 + q + k;
+        float2 a = make_float2(0.f, 0.f), b = a;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
-    if (lane < 4 && row < net.rows) {
-      const float v = lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3];
-      net.y[row * 4 + lane] = v + bias + (net.base ? net.base[row * 4 + lane] : 0.f);
+        for (int i = 0; i < 8; ++i) {
+          const int c = lane + 32 * i;
+          const float v = __bfloat162float(reinterpret_cast<const bf16*>(act + act_chunk(r, c >> 3))[c & 7]);
+          a = __ffma2_rn(make_float2(v, v), w01[i], a);
+          b = __ffma2_rn(make_float2(v, v), w23[i], b);
+        }
+        s[4 * k] = a.x; s[4 * k + 1] = a.y; s[4 * k + 2] = b.x; s[4 * k + 3] = b.y;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;   // keeps the upper half of the sums
+#pragma unroll
+        for (int k = 0; k < o; ++k) {
+          const float keep = up ? s[k + o] : s[k], send = up ? s[k] : s[k + o];
+          s[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      const long long row = m0 + t * 128 + (warp & 7) * 16 + q + (lane >> 2);
+      if (row < net.rows) net.y[row * 4 + (lane & 3)] = s[0] + bias + (net.base ? net.base[row * 4 + (lane & 3)] : 0.f);
     }
+  }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (s_abort) {
+    // A wait gave up: the outputs are not complete and the host sees the flag.
+    // Loads still landing in shared memory and the MMAs issued get a bounded
+    // wait each, the accumulators are released.
+    if (warp == TILES * 8 + 1 && lane == 0) {
+      mbar_wait(xfull, 0);
+      for (int j = max(0, issued - S); j < issued; ++j) mbar_wait(full + 8 * (j % S), (uint32_t)((j / S) & 1));
+    }
+    if (warp == 0)
+      for (int t = 0; t < TILES; ++t) mbar_wait(done + 8 * t, 1);   // the last layer's commit
+    __syncthreads();
+  }
+  if (warp == 0) {   // every tcgen05.ld has completed
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TILES * 256));
   }
 }
 
