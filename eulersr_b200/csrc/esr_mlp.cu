@@ -1061,116 +1061,117 @@ __global__ void __launch_bounds__((Fwd<KEEP, TILES>::THREADS)) k_mlp_fwd(const _
     }
     __syncwarp();
   } else {
-  const int t = warp >> 3;
+    const int t = warp >> 3;
 #pragma unroll 1
-  for (int l = 0; l < 4; ++l) {
-    if (!mbar_wait(done + 8 * t, (uint32_t)(l & 1))) atomicOr(&s_abort, 1);
-    if (__any_sync(0xffffffffu, gave_up())) break;
-    tc_fence_after();
-    const int row = (warp & 3) * 32 + lane, col0 = ((warp >> 2) & 1) * 128;
-    const uint32_t acc = tmem + (uint32_t)(t * 256) + ((uint32_t)((warp & 3) * 32) << 16);
-    unsigned char* act = g + t * 65536;
-    unsigned char* turn = g + C::TURN + warp * 2048;
-    const float* bias = net.b[l];
-    const bool stored = KEEP && m0 + t * 128 < net.rows;
+    for (int l = 0; l < 4; ++l) {
+      if (!mbar_wait(done + 8 * t, (uint32_t)(l & 1))) atomicOr(&s_abort, 1);
+      if (__any_sync(0xffffffffu, gave_up())) break;
+      tc_fence_after();
+      const int row = (warp & 3) * 32 + lane, col0 = ((warp >> 2) & 1) * 128;
+      const uint32_t acc = tmem + (uint32_t)(t * 256) + ((uint32_t)((warp & 3) * 32) << 16);
+      unsigned char* act = g + t * 65536;
+      unsigned char* turn = g + C::TURN + warp * 2048;
+      const float* bias = net.b[l];
+      const bool stored = KEEP && m0 + t * 128 < net.rows;
 #pragma unroll 1
-    for (int c32 = col0; c32 < col0 + 128; c32 += 32) {
-      // everything the chunk needs is requested before the one wait (36 -> 33 us, 58 -> 55)
-      uint32_t v[32];
-      tmem_ld32(acc + (uint32_t)c32, v);
-      uint4 res[4];
-      float4 bv[8];
+      for (int c32 = col0; c32 < col0 + 128; c32 += 32) {
+        // everything the chunk needs is requested before the one wait (36 -> 33 us, 58 -> 55)
+        uint32_t v[32];
+        tmem_ld32(acc + (uint32_t)c32, v);
+        uint4 res[4];
+        float4 bv[8];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        if (l > 0) res[p] = *reinterpret_cast<const uint4*>(act + act_chunk(row, (c32 >> 3) + p));
-        bv[2 * p] = __ldg(reinterpret_cast<const float4*>(bias + c32) + 2 * p);
-        bv[2 * p + 1] = __ldg(reinterpret_cast<const float4*>(bias + c32) + 2 * p + 1);
-      }
-      tmem_wait(v);
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const int c = c32 + 8 * p;
-        bf16* a = reinterpret_cast<bf16*>(act + act_chunk(row, c >> 3));
-        const float4 b0 = bv[2 * p], b1 = bv[2 * p + 1];
-        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        float zv[8], hv[8];
-        if (l > 0) load8<true>(reinterpret_cast<const bf16*>(&res[p]), hv);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          zv[i] = __uint_as_float(v[8 * p + i]) + b[i];
-          hv[i] = (l > 0 ? hv[i] : 0.f) + fmaxf(zv[i], 0.f);
+        for (int p = 0; p < 4; ++p) {
+          if (l > 0) res[p] = *reinterpret_cast<const uint4*>(act + act_chunk(row, (c32 >> 3) + p));
+          bv[2 * p] = __ldg(reinterpret_cast<const float4*>(bias + c32) + 2 * p);
+          bv[2 * p + 1] = __ldg(reinterpret_cast<const float4*>(bias + c32) + 2 * p + 1);
         }
-        store8<true>(a, hv);
-        if (KEEP) store8<true>(reinterpret_cast<bf16*>(turn + lane * 64 + ((p ^ ((lane >> 1) & 3)) << 4)), zv);
-      }
-      if (KEEP) {
-        // 32 rows x 32 columns of this warp, eight rows (64 B each) per store:
-        // a lane writing its own row would touch 32 lines at a time
-        __syncwarp();
-        if (stored) {
+        tmem_wait(v);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int r = q * 8 + (lane >> 2), ch = lane & 3, gr = (warp & 3) * 32 + r;
-            const size_t o = (size_t)(m0 + t * 128 + gr) * 256 + c32 + ch * 8;
-            *reinterpret_cast<uint4*>(net.z[l] + o) =
-                *reinterpret_cast<const uint4*>(turn + r * 64 + ((ch ^ ((r >> 1) & 3)) << 4));
-            *reinterpret_cast<uint4*>(net.h[l] + o) =
-                *reinterpret_cast<const uint4*>(act + act_chunk(gr, (c32 >> 3) + ch));
+        for (int p = 0; p < 4; ++p) {
+          const int c = c32 + 8 * p;
+          bf16* a = reinterpret_cast<bf16*>(act + act_chunk(row, c >> 3));
+          const float4 b0 = bv[2 * p], b1 = bv[2 * p + 1];
+          const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+          float zv[8], hv[8];
+          if (l > 0) load8<true>(reinterpret_cast<const bf16*>(&res[p]), hv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            zv[i] = __uint_as_float(v[8 * p + i]) + b[i];
+            hv[i] = (l > 0 ? hv[i] : 0.f) + fmaxf(zv[i], 0.f);
+          }
+          store8<true>(a, hv);
+          if (KEEP) store8<true>(reinterpret_cast<bf16*>(turn + lane * 64 + ((p ^ ((lane >> 1) & 3)) << 4)), zv);
+        }
+        if (KEEP) {
+          // 32 rows x 32 columns of this warp, eight rows (64 B each) per store:
+          // a lane writing its own row would touch 32 lines at a time
+          __syncwarp();
+          if (stored) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int r = q * 8 + (lane >> 2), ch = lane & 3, gr = (warp & 3) * 32 + r;
+              const size_t o = (size_t)(m0 + t * 128 + gr) * 256 + c32 + ch * 8;
+              *reinterpret_cast<uint4*>(net.z[l] + o) =
+                  *reinterpret_cast<const uint4*>(turn + r * 64 + ((ch ^ ((r >> 1) & 3)) << 4));
+              *reinterpret_cast<uint4*>(net.h[l] + o) =
+                  *reinterpret_cast<const uint4*>(act + act_chunk(gr, (c32 >> 3) + ch));
+            }
+          }
+          __syncwarp();
+        }
+      }
+      tc_fence_before();
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // h_l before the next layer's MMAs read it
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(ready + 8 * t) : "memory");
+    }
+    // h_3 of the tile is in place once its 8 warps are here
+    asm volatile("bar.sync %0, 256;\n" ::"r"(1 + t) : "memory");
+    // head: a warp sums 16 rows, 8 at a time; a lane the columns lane + 32 i in
+    // order. The 32 sums over lanes of a pass (8 rows x 4 outputs) halve their
+    // number at each step of the butterfly (31 shuffles instead of 160; the
+    // pairs added are those of k_head_fwd), so that each lane ends with one.
+    if (!__any_sync(0xffffffffu, gave_up())) {
+      float2 w01[8], w23[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int c = lane + 32 * i;
+        w01[i] = make_float2(net.w4[c], net.w4[256 + c]);
+        w23[i] = make_float2(net.w4[512 + c], net.w4[768 + c]);
+      }
+      const float bias = net.b4[lane & 3];
+      const unsigned char* act = g + t * 65536;
+#pragma unroll 1
+      for (int q = 0; q < 16; q += 8) {
+        float s[32];   // row q + (k >> 2), output k & 3
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = (warp & 7) * 16 + q + k;
+          float2 a = make_float2(0.f, 0.f), b = a;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int c = lane + 32 * i;
+            const float v = __bfloat162float(reinterpret_cast<const bf16*>(act + act_chunk(r, c >> 3))[c & 7]);
+            a = __ffma2_rn(make_float2(v, v), w01[i], a);
+            b = __ffma2_rn(make_float2(v, v), w23[i], b);
+          }
+          s[4 * k] = a.x; s[4 * k + 1] = a.y; s[4 * k + 2] = b.x; s[4 * k + 3] = b.y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const bool up = (lane & o) != 0;   // keeps the upper half of the sums
+#pragma unroll
+          for (int k = 0; k < o; ++k) {
+            const float keep = up ? s[k + o] : s[k], send = up ? s[k] : s[k + o];
+            s[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
           }
         }
-        __syncwarp();
+        const long long row = m0 + t * 128 + (warp & 7) * 16 + q + (lane >> 2);
+        if (row < net.rows)
+          net.y[row * 4 + (lane & 3)] = s[0] + bias + (net.base ? net.base[row * 4 + (lane & 3)] : 0.f);
       }
     }
-    tc_fence_before();
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // h_l before the next layer's MMAs read it
-    __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(ready + 8 * t) : "memory");
-  }
-  // h_3 of the tile is in place once its 8 warps are here
-  asm volatile("bar.sync %0, 256;\n" ::"r"(1 + t) : "memory");
-  // head: a warp sums 16 rows, 8 at a time; a lane the columns lane + 32 i in
-  // order. The 32 sums over lanes of a pass (8 rows x 4 outputs) halve their
-  // number at each step of the butterfly (31 shuffles instead of 160; the
-  // pairs added are those of k_head_fwd), so that each lane ends with one.
-  if (!__any_sync(0xffffffffu, gave_up())) {
-    float2 w01[8], w23[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int c = lane + 32 * i;
-      w01[i] = make_float2(net.w4[c], net.w4[256 + c]);
-      w23[i] = make_float2(net.w4[512 + c], net.w4[768 + c]);
-    }
-    const float bias = net.b4[lane & 3];
-    const unsigned char* act = g + t * 65536;
-#pragma unroll 1
-    for (int q = 0; q < 16; q += 8) {
-      float s[32];   // row q + (k >> 2), output k & 3
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int r = (warp & 7) * 16 + q + k;
-        float2 a = make_float2(0.f, 0.f), b = a;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int c = lane + 32 * i;
-          const float v = __bfloat162float(reinterpret_cast<const bf16*>(act + act_chunk(r, c >> 3))[c & 7]);
-          a = __ffma2_rn(make_float2(v, v), w01[i], a);
-          b = __ffma2_rn(make_float2(v, v), w23[i], b);
-        }
-        s[4 * k] = a.x; s[4 * k + 1] = a.y; s[4 * k + 2] = b.x; s[4 * k + 3] = b.y;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const bool up = (lane & o) != 0;   // keeps the upper half of the sums
-#pragma unroll
-        for (int k = 0; k < o; ++k) {
-          const float keep = up ? s[k + o] : s[k], send = up ? s[k] : s[k + o];
-          s[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-      }
-      const long long row = m0 + t * 128 + (warp & 7) * 16 + q + (lane >> 2);
-      if (row < net.rows) net.y[row * 4 + (lane & 3)] = s[0] + bias + (net.base ? net.base[row * 4 + (lane & 3)] : 0.f);
-    }
-  }
   }
   tc_fence_before();
   __syncthreads();
