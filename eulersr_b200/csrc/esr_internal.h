@@ -41,6 +41,8 @@ struct HostMesh {
   // tile sets built so far (tiles_of), a few per mesh
   mutable std::mutex tile_mutex;
   mutable std::map<std::array<int, 3>, std::shared_ptr<const TileSet>> tiles;
+  // their device tables (StageTables), by device, precision, fidelity and tile size
+  mutable std::map<std::array<int, 4>, std::shared_ptr<void>> device_tiles;
 };
 
 int prepare_mesh(const esr_mesh_desc& d, HostMesh& hm, std::string& err);

@@ -581,3 +581,33 @@ def test_fused_stage_equals_separate_kernels(diamond02, naca02, slots, dt_mode):
             s.close()
         for g, (a, b) in enumerate(zip(*states)):
             assert np.all(np.isfinite(a)) and np.array_equal(a, b), (slots, g)
+
+
+@pytest.mark.parametrize("precision,fidelity", [("f32", "fast"), ("f32", "reference"), ("f64", "fast")])
+def test_solvers_share_a_mesh_and_outlive_it(diamond02, precision, fidelity):
+    """The stage kernel's tables belong to the mesh: a second solver (another
+    slot count, the same tile size), one that outlives the first and the mesh
+    handle, and the same tables under another precision in between give the
+    states of a solver with a mesh of its own."""
+    from eulersr_b200.solver import DeviceMesh, FlowCase, Solver
+    dtype = np.float64 if precision == "f64" else np.float32
+    case = FlowCase(mach=2.0, aoa_deg=3.0, cfl=0.6, tf=10.0, dtype=dtype)
+
+    def states(mesh, slots, before_step=lambda: None):
+        s = Solver(mesh, slots, precision=precision, fidelity=fidelity)
+        s.set_case(slots - 1, case)
+        before_step()
+        s.step(12)
+        return s, s.get_state(slots - 1)
+
+    own = states(diamond02, 1)[1]
+    dm = DeviceMesh(diamond02)
+    other = Solver(dm, 1, precision="f32" if precision == "f64" else "f64")
+    first, a = states(dm, 1)
+
+    def drop():
+        first.close()
+        other.close()
+        dm.close()
+    _, b = states(dm, 2, drop)
+    assert np.array_equal(a, own) and np.array_equal(b, own)
