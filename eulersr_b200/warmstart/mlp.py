@@ -38,8 +38,8 @@ def _p(t):
 
 
 def _array(tensors):
-    """Host array of four device addresses, or None."""
-    return (C.c_void_p * 4)(*[t.data_ptr() for t in tensors]) if tensors is not None else None
+    """Host array of four device addresses, or None; host tensors are refused as in _p."""
+    return (C.c_void_p * 4)(*[_p(t) for t in tensors]) if tensors is not None else None
 
 
 def _stream():
@@ -146,8 +146,13 @@ class MLP:
         return self._addresses(self.p, self.pb)
 
     def _addresses(self, flat, weights=None):
-        """Device addresses of every weight and bias in `flat`; those of W0..W3 in the BF16 copy, if given."""
-        p, w = flat.data_ptr(), (4, flat.data_ptr()) if weights is None else (2, weights.data_ptr())
+        """Device addresses of every weight and bias in `flat`; those of W0..W3 in the BF16 copy, if given.
+        A flat vector in host memory or too short for the layout is refused: kernels use these addresses."""
+        for t in (flat,) if weights is None else (flat, weights):
+            if t.numel() < self.n_params:
+                raise ValueError(f"a flat vector of {t.numel()} values cannot hold the network's {self.n_params}")
+        p = _p(flat).value
+        w = (4, p) if weights is None else (2, _p(weights).value)
         n = F.MlpNet()
         n.W[:] = [w[1] + w[0] * self.offsets[f"W{l}"][0] for l in range(4)]
         n.b[:] = [p + 4 * self.offsets[f"b{l}"][0] for l in range(4)]
