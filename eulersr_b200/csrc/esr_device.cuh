@@ -850,11 +850,12 @@ __global__ void k_grad_export(const Seg<T>* __restrict__ segs, int seg, int b, c
 
 // ----------------------------------------------------------------- K2 flux
 // euler_solver.py:602-628 residual = sum_k F_k s_k / area - sponge (helper.py:262-295),
-// then the stage update of :630-653.
+// then the stage update of :630-653. A second stage runs in place (Wbase =
+// Wout): those two may alias and Wbase is not read through the read-only cache.
 template <typename T, bool FAST, int FLUX, bool MUSCL, int STAGE, bool LOCALDT, int MINB = 0>
 __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, ESR_K2_MINB>)) k_flux(const BlockMap<T> bm,
-                                              const V4<T>* __restrict__ Win, const V4<T>* __restrict__ Wbase,
-                                              V4<T>* __restrict__ Wout, const V4<T>* __restrict__ FV,
+                                              const V4<T>* __restrict__ Win, const V4<T>* Wbase,
+                                              V4<T>* Wout, const V4<T>* __restrict__ FV,
                                               long long total, Cases<T> cs, Consts<T> kc, int pos,
                                               const T* __restrict__ dt_local, T* __restrict__ res_out) {
   Seg<T> s;
@@ -984,8 +985,8 @@ template <int STAGE, bool LOCALDT, int MINB = ESR_PATCH_MINB>
 __global__ void __launch_bounds__(32 * kPatchWarps, MINB) k_flux_patch(const Seg<float>* __restrict__ segs,
                                                                   const int4* __restrict__ pblk,
                                                                   const float4* __restrict__ Win,
-                                                                  const float4* __restrict__ Wbase,
-                                                                  float4* __restrict__ Wout,
+                                                                  const float4* Wbase,
+                                                                  float4* Wout,
                                                                   const float4* __restrict__ FV, long long total,
                                                                   Cases<float> cs, Consts<float> kc, int pos,
                                                                   const float* __restrict__ dt_local,

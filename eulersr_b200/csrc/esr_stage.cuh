@@ -118,6 +118,9 @@ __device__ __forceinline__ V4<T> stage_update(const T acc[4], T area, T sig, con
   }
 }
 
+// A second stage runs in place (Wbase = Wout = the state): both kernels read a
+// cell's Wbase before they write it, in the thread that writes it, and declare
+// neither pointer __restrict__.
 // threads of a block (most) and resident blocks per SM a kernel is compiled for
 #ifndef ESR_STAGE_MINB
 #define ESR_STAGE_MINB 3
@@ -136,7 +139,7 @@ template <typename T, bool FAST> constexpr bool kCanon = FAST || sizeof(T) == 8;
 
 template <typename T, bool FAST, int FLUX, int STAGE, bool LOCALDT>
 __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
-    const StageMap<T> sm, const V4<T>* __restrict__ Win, const V4<T>* __restrict__ Wbase, V4<T>* __restrict__ Wout,
+    const StageMap<T> sm, const V4<T>* __restrict__ Win, const V4<T>* Wbase, V4<T>* Wout,
     Cases<T> cs, Consts<T> kc, int pos, T* __restrict__ dt_local, T* __restrict__ res_out, int p_rows, int fv_rows) {
   using V = V4<T>;
   constexpr bool CANON = kCanon<T, FAST>;
@@ -284,11 +287,24 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
 }
 
 // the states of two slots dB apart; wide: they are neighbours on a 32-byte
-// boundary, one access (as two 16-byte ones every sector is fetched twice)
+// boundary, one access (as two 16-byte ones every sector is fetched twice).
+// For Win alone, which no launch writes: the read-only path.
 __device__ __forceinline__ void state_pair(const float4* p, int dB, bool wide, float4& a, float4& b) {
   if (wide) {
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p));
+  } else {
+    a = p[0];
+    b = p[dB];
+  }
+}
+// the same for Wbase, which a second stage overwrites in place (Wbase = Wout):
+// the ordinary path, and never moved past a store
+__device__ __forceinline__ void base_pair(const float4* p, int dB, bool wide, float4& a, float4& b) {
+  if (wide) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p) : "memory");
   } else {
     a = p[0];
     b = p[dB];
@@ -328,9 +344,8 @@ __device__ __forceinline__ void pair_of(const float4& a, const float4& b, float2
 
 template <int STAGE, bool LOCALDT, int SH>
 __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
-    const StageMap<float> sm, const float4* __restrict__ Win, const float4* __restrict__ Wbase,
-    float4* __restrict__ Wout, Cases<float> cs, Consts<float> kc, int pos, float* __restrict__ dt_local,
-    float* __restrict__ res_out, int p_rows, int fv_rows) {
+    const StageMap<float> sm, const float4* __restrict__ Win, const float4* Wbase, float4* Wout, Cases<float> cs,
+    Consts<float> kc, int pos, float* __restrict__ dt_local, float* __restrict__ res_out, int p_rows, int fv_rows) {
   constexpr int NP = 1 << SH;
   extern __shared__ __align__(16) unsigned char stage_smem[];
   float4* P0 = reinterpret_cast<float4*>(stage_smem);   // primitives: (rho, u) and (v, p) of both slots
@@ -473,7 +488,7 @@ __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
     pair_of(wa, wb, Wc);
     if (STAGE != ST_FIRST) {
       float4 a, b;
-      state_pair(Wbase + gi, dB, wide, a, b);
+      base_pair(Wbase + gi, dB, wide, a, b);
       pair_of(a, b, W0);
     }
     float2 dt = case_dt;
