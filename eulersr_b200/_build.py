@@ -18,7 +18,8 @@ INCLUDE = PKG.parent / "include"
 LIB = PKG / "libeulersr.so"
 
 SOURCES = ["esr_host.cu", "esr_mesh.cpp", "esr_noalloc.cu", "esr_mlp.cu", "esr_faithful.cu"]
-HEADERS = ["esr_device.cuh", "esr_stage.cuh", "esr_internal.h", "esr_layout.h", "esr_mlp.cuh", "esr_warm.cuh", "esr_faithful.h"]
+HEADERS = ["esr_device.cuh", "esr_stage.cuh", "esr_internal.h", "esr_layout.h", "esr_mlp.cuh", "esr_warm.cuh", "esr_faithful.h",
+           "esr_per_device.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # per-source flags: the reference-fidelity kernels round every float32
 # product and sum separately, as the reference's float32 arithmetic does

@@ -24,6 +24,7 @@
 
 #include "esr_internal.h"
 #include "esr_mlp.cuh"
+#include "esr_per_device.h"
 
 namespace {
 
@@ -1366,17 +1367,26 @@ __global__ void __launch_bounds__(THREADS) k_mlp_wgrad(const __grid_constant__ W
 
 int mfail(int code, const std::string& msg) { return esr::report_error(code, msg); }
 
+// Raises KERNEL's dynamic shared-memory limit on the current device
+template <auto KERNEL>
+cudaError_t allow_smem(int bytes) {
+  static PerDevice set;
+  int device = 0;
+  const cudaError_t err = cudaGetDevice(&device);
+  if (err != cudaSuccess) return err;
+  return (cudaError_t)set.once(device, [&](int) {
+    return (int)cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  });
+}
+
 template <bool AT, bool BT, int EPI>
 int launch_gemm(int M, int N, int K, int splits, const bf16* A, int lda, const bf16* B, int ldb, const Epi& e,
                 cudaStream_t st) {
   constexpr int A_ELEMS = AT ? BK * LD_MN : BM * LD_K;
   constexpr int B_ELEMS = BT ? BK * LD_MN : BN * LD_K;
   const int smem = STAGES * (A_ELEMS + B_ELEMS) * (int)sizeof(bf16);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_gemm<AT, BT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attr_set = true;
-  }
+  const cudaError_t err = allow_smem<&k_gemm<AT, BT, EPI>>(smem);
+  if (err != cudaSuccess) return mfail(ESR_ERR_CUDA, std::string("gemm: ") + cudaGetErrorString(err));
   dim3 grid(N / BN, M / BM, splits);
   k_gemm<AT, BT, EPI><<<grid, THREADS, smem, st>>>(M, N, K / splits, A, lda, B, ldb, e);
   return ESR_OK;
@@ -1410,14 +1420,6 @@ int make_map(CUtensorMap* map, const bf16* base, uint64_t inner, uint64_t outer,
 template <bool AT, bool BT, int EPI>
 int launch_gemm_tc(int M, int N, int K, int splits, const bf16* A, int lda, const bf16* B, int ldb, const Epi& e,
                    cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(tc::k_gemm_tc<AT, BT, EPI, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         tc::Cfg<128>::SMEM);
-    cudaFuncSetAttribute(tc::k_gemm_tc<AT, BT, EPI, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         tc::Cfg<256>::SMEM);
-    attr_set = true;
-  }
   // 256-wide tiles (A read once per row block) when there are still enough
   // of them to give every SM one; otherwise 128-wide tiles for parallelism
   const int tbn = (N % 256 == 0 && (long long)(M / tc::BM) * (N / 256) * splits >= 148) ? 256 : 128;
@@ -1426,6 +1428,9 @@ int launch_gemm_tc(int M, int N, int K, int splits, const bf16* A, int lda, cons
   if (rc != ESR_OK) return rc;
   rc = BT ? make_map(&mb, B, N, K, ldb, 64, 64) : make_map(&mb, B, K, N, ldb, 64, tbn);
   if (rc != ESR_OK) return rc;
+  const cudaError_t err = tbn == 256 ? allow_smem<&tc::k_gemm_tc<AT, BT, EPI, 256>>(tc::Cfg<256>::SMEM)
+                                     : allow_smem<&tc::k_gemm_tc<AT, BT, EPI, 128>>(tc::Cfg<128>::SMEM);
+  if (err != cudaSuccess) return mfail(ESR_ERR_CUDA, std::string("gemm: ") + cudaGetErrorString(err));
   if (tbn == 256) {
     dim3 grid(N / 256, M / tc::BM, splits);
     tc::k_gemm_tc<AT, BT, EPI, 256><<<grid, tc::THREADS, tc::Cfg<256>::SMEM, st>>>(M, N, K / splits, ma, mb, e);
@@ -1439,8 +1444,7 @@ int launch_gemm_tc(int M, int N, int K, int splits, const bf16* A, int lda, cons
 template <bool KEEP, int TILES>
 int launch_fwd(const tc::MlpMaps& maps, const tc::MlpNet& n, void* stream) {
   using C = tc::Fwd<KEEP, TILES>;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(tc::k_mlp_fwd<KEEP, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  const cudaError_t attr = allow_smem<&tc::k_mlp_fwd<KEEP, TILES>>(C::SMEM);
   if (attr != cudaSuccess) return mfail(ESR_ERR_CUDA, std::string("mlp_forward: ") + cudaGetErrorString(attr));
   tc::k_mlp_fwd<KEEP, TILES><<<(n.rows / 128 + TILES - 1) / TILES, C::THREADS, C::SMEM, (cudaStream_t)stream>>>(maps, n);
   return ESR_OK;
@@ -1477,7 +1481,7 @@ int gemm_check(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_t K
 int esr_gemm_bf16(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_t K, const void* A, int32_t lda,
                   const void* B, int32_t ldb, int32_t epi, const float* bias, const void* res, const void* aux,
                   void* out0, void* out1, int32_t ldo, int32_t splits, void* stream) {
-  const int rc = gemm_check(trans_a, trans_b, M, N, K, A, lda, B, ldb, epi, bias, aux, out0, out1, ldo, splits, tc::BK);
+  int rc = gemm_check(trans_a, trans_b, M, N, K, A, lda, B, ldb, epi, bias, aux, out0, out1, ldo, splits, tc::BK);
   if (rc != ESR_OK) return rc;
   // rows and buffers aligned for the 16-byte epilogue (a null one is not touched)
   const bool vec = ldo % 8 == 0 && aligned16(bias) && aligned16(res) && aligned16(aux) && aligned16(out0) && aligned16(out1);
@@ -1486,7 +1490,7 @@ int esr_gemm_bf16(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_
   const bf16* a = (const bf16*)A;
   const bf16* b = (const bf16*)B;
 #define ESR_GEMM_CASE(TA, TB, E) \
-  if (!!trans_a == TA && !!trans_b == TB && epi == E) launch_gemm_tc<TA, TB, E>(M, N, K, splits, a, lda, b, ldb, e, st); else
+  if (!!trans_a == TA && !!trans_b == TB && epi == E) rc = launch_gemm_tc<TA, TB, E>(M, N, K, splits, a, lda, b, ldb, e, st); else
   ESR_GEMM_CASE(false, false, EPI_FWD)
   ESR_GEMM_CASE(false, true, EPI_BWD)
   ESR_GEMM_CASE(true, true, EPI_F32)
@@ -1495,6 +1499,7 @@ int esr_gemm_bf16(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_
   ESR_GEMM_CASE(false, false, EPI_BWD)
   return mfail(ESR_ERR_ARG, "gemm: unsupported layout/epilogue combination");
 #undef ESR_GEMM_CASE
+  if (rc != ESR_OK) return rc;
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, std::string("gemm: ") + cudaGetErrorString(err));
 }
@@ -1558,8 +1563,7 @@ int esr_mlp_wgrad(const void* const* dz, const void* const* src, int32_t rows, i
     if (rc != ESR_OK) return rc;
     out.dw[l] = dw[l];
   }
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(tc::k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::Wg::SMEM);
+  const cudaError_t attr = allow_smem<&tc::k_mlp_wgrad>(tc::Wg::SMEM);
   if (attr != cudaSuccess) return mfail(ESR_ERR_CUDA, std::string("mlp_wgrad: ") + cudaGetErrorString(attr));
   // as many ranges per CTA as keep the launch to one CTA per SM, at most one per accumulator
   const int per = std::min(tc::WG_ACC, (splits + 148 / tc::WG_TILES - 1) / (148 / tc::WG_TILES));
@@ -1572,14 +1576,14 @@ int esr_mlp_wgrad(const void* const* dz, const void* const* src, int32_t rows, i
 int esr_gemm_bf16_mma_sync(int32_t trans_a, int32_t trans_b, int32_t M, int32_t N, int32_t K, const void* A,
                            int32_t lda, const void* B, int32_t ldb, int32_t epi, const float* bias, const void* res,
                            const void* aux, void* out0, void* out1, int32_t ldo, int32_t splits, void* stream) {
-  const int rc = gemm_check(trans_a, trans_b, M, N, K, A, lda, B, ldb, epi, bias, aux, out0, out1, ldo, splits, BK);
+  int rc = gemm_check(trans_a, trans_b, M, N, K, A, lda, B, ldb, epi, bias, aux, out0, out1, ldo, splits, BK);
   if (rc != ESR_OK) return rc;
   Epi e{bias, (const bf16*)res, (const bf16*)aux, out0, (bf16*)out1, ldo, (long long)M * ldo, false};
   cudaStream_t st = (cudaStream_t)stream;
   const bf16* a = (const bf16*)A;
   const bf16* b = (const bf16*)B;
 #define ESR_GEMM_CASE(TA, TB, E) \
-  if (!!trans_a == TA && !!trans_b == TB && epi == E) launch_gemm<TA, TB, E>(M, N, K, splits, a, lda, b, ldb, e, st); else
+  if (!!trans_a == TA && !!trans_b == TB && epi == E) rc = launch_gemm<TA, TB, E>(M, N, K, splits, a, lda, b, ldb, e, st); else
   ESR_GEMM_CASE(false, false, EPI_FWD)
   ESR_GEMM_CASE(false, true, EPI_BWD)
   ESR_GEMM_CASE(true, true, EPI_F32)
@@ -1588,6 +1592,7 @@ int esr_gemm_bf16_mma_sync(int32_t trans_a, int32_t trans_b, int32_t M, int32_t 
   ESR_GEMM_CASE(false, false, EPI_BWD)
   return mfail(ESR_ERR_ARG, "gemm: unsupported layout/epilogue combination");
 #undef ESR_GEMM_CASE
+  if (rc != ESR_OK) return rc;
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, std::string("gemm: ") + cudaGetErrorString(err));
 }
