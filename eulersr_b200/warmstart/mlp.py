@@ -42,6 +42,11 @@ def _array(tensors):
     return (C.c_void_p * 4)(*[_p(t) for t in tensors]) if tensors is not None else None
 
 
+def _aligned(*tensors):
+    """Every address is a multiple of 16: what the one-call kernels' vector accesses need."""
+    return all(t.data_ptr() % 16 == 0 for t in tensors)
+
+
 def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
@@ -120,7 +125,8 @@ class MLP:
         st = _stream()
         tag = "k" if keep else "f"
         y = self._buf(f"{tag}y", (rows, N_OUT), torch.float32)
-        if self.fused:
+        # the layer calls take biases at any address (flat vectors that are views of a larger one)
+        if self.fused and _aligned(self.p):
             h = z = None
             if keep:
                 h, z = ([self._buf(f"k{n}{l}", (rows, H), torch.bfloat16) for l in range(4)] for n in "hz")
@@ -165,12 +171,13 @@ class MLP:
         X, h, z = acts["X"], acts["h"], acts["z"]
         rows = X.shape[0]
         st = _stream()
-        if self.fused and splits is None:
+        if self.fused and splits is None and _aligned(*h, *z):
             work = self._buf("backward", (self.L.esr_mlp_backward_workspace(rows),), torch.uint8)
             F.check(self.L.esr_mlp_backward(C.byref(self._net()), _p(X), rows, _p(dY), _array(h), _array(z), _p(work),
                                             C.byref(self._addresses(self.g)), st))
             return
-        # layer by layer: the mma.sync kernel, or a split of the weight gradients set by the caller
+        # layer by layer: the mma.sync kernel, a split of the weight gradients set by the caller, or
+        # activations at addresses that the one-call form cannot take
         if splits is None:
             splits = 1
             while splits < 64 and rows % (64 * splits * 2) == 0 and rows // (splits * 2) >= 1024:

@@ -440,3 +440,35 @@ def test_backward_in_one_call_equals_layer_calls(rows):
     m.backward(acts, dpred)
     assert torch.equal(m.g, want)
     assert m.L.esr_mlp_backward_workspace(rows + 64) == -1
+
+
+@pytest.mark.parametrize("rows", [128, 2688])
+def test_views_of_larger_buffers_run(rows):
+    """Flat parameters and kept activations that are views into a larger
+    buffer, at 4-byte addresses, give the bits of buffers of their own: the
+    layer calls take them where the one-call kernels' 16-byte accesses cannot."""
+    import torch
+    m, X, base, tgt, w, inv_den = _setup(rows=rows, seed=11)
+
+    def passes(acts_of=lambda acts: acts):
+        y, acts = m.forward(X, base, keep=True)
+        _, dpred = m.loss(y, tgt, w, inv_den)
+        m.backward(acts_of(acts), dpred)
+        return y.clone(), m.g.clone()
+
+    def shifted(acts):
+        z = []
+        for t in acts["z"]:
+            big = torch.zeros(t.numel() + 2, dtype=t.dtype, device=t.device)
+            big[2:].copy_(t.reshape(-1))
+            z.append(big[2:].view(t.shape))
+        return dict(acts, z=z)
+
+    want = passes()
+    assert all(torch.equal(a, b) for a, b in zip(passes(shifted), want))
+    big = torch.zeros(m.n_params + 1, device=m.p.device)
+    big[1:].copy_(m.p)
+    m.p = big[1:]
+    assert m.p.data_ptr() % 16 == 4
+    assert all(torch.equal(a, b) for a, b in zip(passes(), want))
+    assert torch.equal(m.forward(X, base), want[0])
