@@ -742,9 +742,9 @@ __device__ __forceinline__ void limited_faces(const T Pc[4], const T Pk[3][4], c
 }
 
 // per-cell CFL time step over the case's CFL number (helper.py:8-18)
-template <typename T, bool FAST>
+template <typename T, bool FAST, bool XR = kXr<T, FAST>>
 __device__ __forceinline__ T local_dt(const T P[4], const T n[6], const T len[3], T area, const Consts<T>& kc) {
-  if constexpr (kXr<T, FAST>) {
+  if constexpr (XR) {
     return xr::local_dt<T>(P, n, len, area, kc);
   } else {
     const T cel = sqrt(fabs(kc.gamma * P[3] / P[0]));
@@ -764,7 +764,8 @@ __device__ __forceinline__ T local_dt(const T P[4], const T n[6], const T len[3]
 // gradient (helper.py:136-153), limiter (euler_solver.py:45-67) and the cell's
 // own MUSCL face states (euler_solver.py:69-98). Writes FV[k][item] (primitive).
 // With LOCALDT it also writes the per-cell CFL time step of the state.
-// MUSCL=false only computes the local dt (constant reconstruction needs no face states).
+// MUSCL=false only computes the local dt (constant reconstruction needs no
+// face states), with IEEE division and square root as its flux kernel.
 template <typename T, bool FAST, bool MUSCL, bool LOCALDT, int MINB = 0>
 __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, LOCALDT ? ESR_K1_MINB_LOCAL : ESR_K1_MINB>)) k_recon(const BlockMap<T> bm,
                                                const V4<T>* __restrict__ W, V4<T>* __restrict__ FV,
@@ -780,11 +781,12 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, LOCALDT ? ESR_
   const long long gi = s.off + (long long)c * s.B + b;
   const V4<T> Wc = W[gi];
   T Pc[4];
-  cell_prim<T, FAST>(Wc, kc, Pc);
+  if constexpr (MUSCL) cell_prim<T, FAST>(Wc, kc, Pc);
+  else prim<T, FAST>(Wc, kc.gm1, kc.half, Pc);
   if (LOCALDT) {
     T gn[12];
     geo_groups<T, 3>(s, c, 0, gn);
-    dt_local[gi] = local_dt<T, FAST>(Pc, gn + G_N0X, gn + G_S0, gn[G_AREA], kc) * cs.dt[g];   // cs.dt holds the case CFL in local mode
+    dt_local[gi] = local_dt<T, FAST, MUSCL && kXr<T, FAST>>(Pc, gn + G_N0X, gn + G_S0, gn[G_AREA], kc) * cs.dt[g];   // cs.dt holds the case CFL in local mode
   }
   if (!MUSCL) return;
   const int4 nb = __ldg(s.nbr + c);
