@@ -594,8 +594,9 @@ __device__ __forceinline__ V4<T> cell_update4(const T acc[4], T area, T sig, con
 // With hi = max(P_k - P_c, 0) and lo = min(P_k - P_c, 0) (exact: subtraction
 // is monotonic) a face of increment d has
 // phi = (a a + 2 a d) / (a a + 2 d d + a d + eps), a = hi or lo by d's sign.
-// NV variables at a time: each is independent of the others.
-template <typename V, int NV>
+// NV variables at a time: each is independent of the others. FAR (float64):
+// the values may be large enough for products of four differences to overflow.
+template <typename V, int NV, bool FAR = false>
 __device__ __forceinline__ void limited_faces(const V Pc[NV], const V Pk[3][NV], const Scalar<V> gc[12],
                                               const Consts<Scalar<V>>& k, V out[3][NV]) {
   const V zero = splat<V>(0), one = splat<V>(1), veps = splat<V>(k.venk_eps), leps = splat<V>(k.eps_lim);
@@ -627,14 +628,18 @@ __device__ __forceinline__ void limited_faces(const V Pc[NV], const V Pk[3][NV],
     if constexpr (sizeof(Scalar<V>) == 8) {
       // A float64 division costs as much as the rest of a face's limiter, so
       // the smallest of the three fractions (denominators positive) is found
-      // by cross-multiplication and divided once.
+      // by cross-multiplication and divided once, unless FAR.
+      if constexpr (FAR) {
+        least = lower(phi[0] / dens[0], phi[1] / dens[1], phi[2] / dens[2]);
+      } else {
 #pragma unroll
-      for (int f = 1; f < 3; ++f) {
-        const auto less = gt(mul(phi[0], dens[f]), mul(phi[f], dens[0]));
-        phi[0] = pick(less, phi[f], phi[0]);
-        dens[0] = pick(less, dens[f], dens[0]);
+        for (int f = 1; f < 3; ++f) {
+          const auto less = gt(mul(phi[0], dens[f]), mul(phi[f], dens[0]));
+          phi[0] = pick(less, phi[f], phi[0]);
+          dens[0] = pick(less, dens[f], dens[0]);
+        }
+        least = phi[0] / dens[0];
       }
-      least = phi[0] / dens[0];
     } else {
       least = lower(phi[0], phi[1], phi[2]);
     }
@@ -675,11 +680,11 @@ __device__ __forceinline__ void ghost_prim(int kind, const V4<T>& Wc, T nx, T ny
 // from its own and its neighbours' (or ghosts') primitives: LSQ gradient
 // (helper.py:136-153), limiter (euler_solver.py:45-67), face states
 // (euler_solver.py:69-98). gc: LSQ coefficients and face offsets.
-template <typename T, bool FAST>
+template <typename T, bool FAST, bool FAR = false>
 __device__ __forceinline__ void limited_faces(const T Pc[4], const T Pk[3][4], const T gc[12], const LsqRef* lsq, int c,
                                               const Consts<T>& kc, T out[3][4]) {
   if constexpr (kXr<T, FAST>) {
-    xr::limited_faces<T, 4>(Pc, Pk, gc, kc, out);
+    xr::limited_faces<T, 4, FAR>(Pc, Pk, gc, kc, out);
   } else {
   T gx[4], gy[4];
   if constexpr (!FAST && sizeof(T) == 4) {

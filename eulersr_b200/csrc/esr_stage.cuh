@@ -27,6 +27,8 @@
 // side of every cell from its own perspective, as the reference evaluates
 // them, into a buffer of its own.
 #pragma once
+#include <limits.h>
+
 #include <type_traits>
 
 #include "esr_device.cuh"
@@ -79,6 +81,43 @@ struct StageMap {
   Seg<T> seg0;
   int groups;         // one mesh: slot groups per tile, else 0
 };
+
+// Exponent word of the largest of four primitives and `top`. From 2^200
+// (kFarWord) a block's limiter divides three times (xr::limited_faces): its
+// cross products, of the order of the fourth power, overflow at 2^256. Looked
+// at here, in integers and once a block, it costs 0.7 % of a float64 stage (32 x
+// 25,968 cells 164.7 -> 166.1 us per step); a branch in the limiter 4 %.
+constexpr int kFarWord = (1023 + 200) << 20;
+__device__ __forceinline__ int top_word(const double q[4], int top) {
+#pragma unroll
+  for (int v = 0; v < 4; ++v) top = max(top, __double2hiint(q[v]) & 0x7fffffff);
+  return top;
+}
+
+// Phase B of a block with such values, out of line: the loop that every other
+// block runs keeps its size and its registers.
+static __device__ __noinline__ void far_faces(const V4<double>* P, V4<double>* FV, const StageCell<double>* cells,
+                                              int n1, int sh, int slot, double venk_eps, double eps_lim) {
+  Consts<double> kc;
+  kc.venk_eps = venk_eps;
+  kc.eps_lim = eps_lim;
+  for (int i = threadIdx.x; i < n1 << sh; i += blockDim.x) {
+    const StageCell<double> r = cells[i >> sh];
+    double Pk[3][4], q[3][4];
+    const V4<double> pc = P[i];
+    const double Pc[4] = {pc.x, pc.y, pc.z, pc.w};
+    for (int k = 0; k < 3; ++k) {
+      const V4<double> p = P[((int)r.nbr[k] << sh) + slot];
+      Pk[k][0] = p.x; Pk[k][1] = p.y; Pk[k][2] = p.z; Pk[k][3] = p.w;
+    }
+    xr::limited_faces<double, 4, true>(Pc, Pk, r.gc, kc, q);
+    for (int k = 0; k < 3; ++k) {
+      if (r.slot[k] == kNoSlot) continue;
+      const bool inner = slot_kind((int)r.kinds, k) == K_INTERIOR;
+      FV[((int)r.slot[k] << sh) + slot] = inner ? mk4<double>(q[k][0], q[k][1], q[k][2], q[k][3]) : pc;
+    }
+  }
+}
 
 // value of face state `q`'s flux through the unit normal n, in the run's rounding
 template <typename T, bool FAST, int FLUX>
@@ -176,23 +215,29 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
   if (!__syncthreads_or(live)) return;          // every slot of the group idle
   const V* win = Win + s.off + (in_seg ? b : 0);
   // A: primitives of the tile, its two rings and its ghosts
+  constexpr bool SCALED = kXr<T, FAST> && sizeof(T) == 8;   // the limiter's products have a range (limited_faces)
+  int top = 0;                                              // largest exponent word of the primitives
   for (int i = threadIdx.x, c = c0; i < h.n2 << sh; i += nt) {
     T q[4];
     const V w = fresh(win + (long long)c * s.B);
     if (i + nt < h.n2 << sh) c = list[(i + nt) >> sh];
     cell_prim<T, FAST>(w, kc, q);
+    if constexpr (SCALED) if (live) top = top_word(q, top);
     P[i] = mk4<T>(q[0], q[1], q[2], q[3]);
   }
   for (int i = threadIdx.x; i < h.n_ghosts << sh; i += nt) {
     const StageGhost<T> w = s.tile_ghosts[h.ghosts + (i >> sh)];
     T q[4];
     ghost_prim<T, FAST>(w.kind, fresh(win + (long long)w.cell * s.B), w.nx, w.ny, inlet, kc, q);
+    if constexpr (SCALED) if (live) top = top_word(q, top);
     P[(h.n2 << sh) + i] = mk4<T>(q[0], q[1], q[2], q[3]);
   }
   // B: limited face states of the tile and its first ring. The first record
   // of each phase is on its way before the barrier.
-  __syncthreads();
-  for (int i = threadIdx.x; i < h.n1 << sh; i += nt) {
+  bool far = false;
+  if constexpr (SCALED) far = __syncthreads_or(top >= kFarWord);
+  else __syncthreads();
+  for (int i = (SCALED && far) ? INT_MAX : (int)threadIdx.x; i < h.n1 << sh; i += nt) {
     const int lc = i >> sh;
     StageCell<T> rn = r;
     if (kFastPath<T, FAST> && i + nt < h.n1 << sh) rn = cells[(i + nt) >> sh];   // the next one meanwhile
@@ -214,6 +259,7 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
     if (!kFastPath<T, FAST> && i + nt < h.n1 << sh) rn = cells[(i + nt) >> sh];
     r = rn;
   }
+  if constexpr (SCALED) if (far) far_faces(P, FV, cells, h.n1, sh, slot, kc.venk_eps, kc.eps_lim);
   const StageFace<T>* faces = s.tile_faces + h.faces;
   StageFace<T> f = faces[min((int)threadIdx.x >> sh, h.n_faces - 1)];
   __syncthreads();

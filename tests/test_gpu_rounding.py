@@ -41,3 +41,27 @@ def test_constant_reconstruction_local_time_step(diamond02, precision):
     want = np.load(GOLDEN / "constant_local_dt.npz")[precision]
     got = _steps(diamond02, precision=precision, reconstruction="constant", dt_mode="local")[0]
     assert np.array_equal(got, want.astype(np.float64))
+
+
+@pytest.mark.parametrize("exponent", [-60, 240, 280])
+def test_float64_limiter_far_from_unit_scale(diamond02, exponent):
+    """Density and pressure in units 2^exponent: the limiter's fractions have
+    squares of state differences above and below, whose cross products leave
+    float64's range from 2^256 on although each fraction is ordinary. Held to
+    the float64 parity tolerance against the oracle (field-scaled 1e-12)."""
+    from conftest import oracle_mesh, rel_err
+    from eulersr_b200.solver import FlowCase, Solver
+    from oracle import euler_oracle as O
+    scale = 2.0 ** exponent
+    om = oracle_mesh(diamond02, np.float64)
+    W, inlet = O.initialize(diamond02.n_cells, dict(rho_inf=scale, p_inf=scale, gamma=1.4, Mach=2.5, aoa=5.0,
+                                                    case=diamond02.metadata["case"]), np.float64)
+    dt = O.get_dt(W, om, CFL=0.6)
+    for _ in range(20):
+        W = O.time_step_srk2(W, om, dt, inlet)
+    s = Solver(diamond02, 1, precision="f64")
+    s.set_case(0, FlowCase(mach=2.5, aoa_deg=5.0, cfl=0.6, tf=100.0, rho_inf=scale, p_inf=scale))
+    assert abs(s.dt()[0] - dt) <= 1e-14 * dt
+    s.step(20)
+    assert rel_err(s.get_state(0), W) <= 1e-12
+    s.close()
