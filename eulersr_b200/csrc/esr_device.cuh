@@ -13,8 +13,8 @@
 //              (geo[cell * G_COUNT + field], esr_layout.h), read as float4/double4 groups
 //   stage      one Runge-Kutta stage of a MUSCL solve in one kernel
 //              (esr_stage.cuh); the separate pair below remains for fast
-//              float32 HLLC at a requested launch shape, K2 also for constant
-//              reconstruction
+//              float32 HLLC at a requested launch shape and for float64 in
+//              the reference's sequence, K2 also for constant reconstruction
 //   K1 recon   cell + 3 neighbour primitives, LSQ gradient, Venkatakrishnan
 //              limiter, the 3 MUSCL face states of the cell -> FV[k][item]
 //   K2 flux    per cell: the 3 face fluxes (HLLC or Rusanov) from its own
@@ -147,14 +147,18 @@ __device__ __forceinline__ void block_origin(const BlockMap<T>& bm, Seg<T>& s, i
   }
 }
 
-// Precision policy. The float32 kernels of the reference-fidelity mode (FAST =
-// false, compiled without FMA contraction in their own translation unit,
-// esr_faithful.cu) keep the reference's exact operation sequence. FAST float32
-// (the default) uses approximate reciprocals and square roots (1 ulp); float64
-// uses IEEE division and square root, with the formulas of xr:: below.
+// Precision policy. FAST = false (fidelity reference) keeps the reference's
+// operation sequence with IEEE division and square root: the conserved round
+// trip of the face states, Fc - (Fc - F_HLLC), every side of a face from its
+// own cell. In float32 those kernels are compiled without FMA contraction in
+// their own translation unit (esr_faithful.cu). FAST (the default) uses the
+// formulas of xr:: below: in float32 with approximate reciprocals and square
+// roots (1 ulp), in float64 with IEEE ones and a reciprocal where the sequence
+// divides. Constant reconstruction keeps the sequence in every mode, with
+// __fdividef in fast float32.
 template <typename T, bool FAST> constexpr bool kFastPath = FAST && sizeof(T) == 4;
-// kernels whose numerics are the xr:: functions: fast float32 and float64 MUSCL + HLLC
-template <typename T, bool FAST> constexpr bool kXr = FAST || sizeof(T) == 8;
+// MUSCL kernels whose numerics are the xr:: functions (the Rusanov flux itself has none)
+template <typename T, bool FAST> constexpr bool kXr = FAST;
 template <typename T, bool FAST = (sizeof(T) == 4)>
 __device__ __forceinline__ T dv(T a, T b) {
   if constexpr (kFastPath<T, FAST>) return __fdividef(a, b);
@@ -801,10 +805,17 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, LOCALDT ? ESR_
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const int kind = slot_kind(nb.w, k);
-    if (kind == K_INTERIOR)
-      cell_prim<T, FAST>(W[s.off + (long long)nbk[k] * s.B + b], kc, Pk[k]);
-    else
-      ghost_prim<T, FAST>(kind, Wc, geo(s, G_N0X + 2 * k, c), geo(s, G_N0Y + 2 * k, c), inlet, kc, Pk[k]);
+    if constexpr (kXr<T, FAST>) {
+      if (kind == K_INTERIOR)
+        cell_prim<T, FAST>(W[s.off + (long long)nbk[k] * s.B + b], kc, Pk[k]);
+      else
+        ghost_prim<T, FAST>(kind, Wc, geo(s, G_N0X + 2 * k, c), geo(s, G_N0Y + 2 * k, c), inlet, kc, Pk[k]);
+    } else {   // one conversion for both: its divisions are not worth a branch
+      V4<T> Wk;
+      if (kind == K_INTERIOR) Wk = W[s.off + (long long)nbk[k] * s.B + b];
+      else Wk = ghost_cons<T, FAST>(kind, Wc, geo(s, G_N0X + 2 * k, c), geo(s, G_N0Y + 2 * k, c), inlet, kc);
+      prim<T, FAST>(Wk, kc.gm1, kc.half, Pk[k]);
+    }
   }
   T gc[12];   // LSQ coefficients and face offsets (groups 3-5)
   geo_groups<T, 3>(s, c, 3, gc);
@@ -909,14 +920,35 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, ESR_K2_MINB>))
     Wout[gi] = o;
   } else {
     T acc[4];
+    // The step's first state, on its way before the fluxes (float64 48 x 25,968
+    // cells 443 -> 434 us per step) except in fast float32, which is short of
+    // registers (constant reconstruction 32 x 25,968 43.1 -> 44.6 with it)
+    constexpr bool EARLY = STAGE != ST_FIRST && !kFastPath<T, FAST>;
+    V4<T> W0 = Wc;
+    if (EARLY) W0 = Wbase[gi];
   #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const int kind = slot_kind(nb.w, k);
       const T nx = gk[G_N0X + 2 * k], ny = gk[G_N0Y + 2 * k];
+      V4<T> WL, WR;
       T PL[4], PR[4];
-      const V4<T> WL = Wc;
-      const V4<T> WR = (kind == K_INTERIOR) ? Win[s.off + (long long)nbk[k] * s.B + b]
-                                            : ghost_cons<T, FAST>(kind, Wc, nx, ny, inlet, kc);
+      if constexpr (MUSCL) {   // the face states, through the reference's conserved round trip
+        const V4<T> fl = FV[(long long)k * total + gi];
+        const T qL[4] = {fl.x, fl.y, fl.z, fl.w};
+        T qR[4];
+        if (kind == K_INTERIOR) {
+          const V4<T> fr = FV[(long long)slot_opp(nb.w, k) * total + s.off + (long long)nbk[k] * s.B + b];
+          qR[0] = fr.x; qR[1] = fr.y; qR[2] = fr.z; qR[3] = fr.w;
+        } else {
+          prim<T, FAST>(ghost_cons<T, FAST>(kind, Wc, nx, ny, inlet, kc), kc.gm1, kc.half, qR);
+        }
+        WL = cons<T, FAST>(qL, kc.gm1, kc.inv_gm1, kc.half);
+        WR = cons<T, FAST>(qR, kc.gm1, kc.inv_gm1, kc.half);
+      } else {
+        WL = Wc;
+        WR = (kind == K_INTERIOR) ? Win[s.off + (long long)nbk[k] * s.B + b]
+                                  : ghost_cons<T, FAST>(kind, Wc, nx, ny, inlet, kc);
+      }
       prim<T, FAST>(WL, kc.gm1, kc.half, PL);
       prim<T, FAST>(WR, kc.gm1, kc.half, PR);
       T F[4];
@@ -938,15 +970,14 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, ESR_K2_MINB>))
     const T dt = LOCALDT ? dt_local[gi] : cs.dt[g];
     // density residual of the state the step starts from (density-L2 stop rule)
     if (STAGE == ST_FIRST && res_out != nullptr) res_out[gi] = R0;
+    if (STAGE != ST_FIRST && !EARLY) W0 = Wbase[gi];
     V4<T> o;
     if (STAGE == ST_FIRST) {
       o = mk4<T>(Wc.x - dt * R0, Wc.y - dt * R1, Wc.z - dt * R2, Wc.w - dt * R3);
     } else if (STAGE == ST_SRK2_SECOND) {
-      const V4<T> W0 = Wbase[gi];
       o = mk4<T>(kc.half * (W0.x + Wc.x - dt * R0), kc.half * (W0.y + Wc.y - dt * R1),
                  kc.half * (W0.z + Wc.z - dt * R2), kc.half * (W0.w + Wc.w - dt * R3));
     } else {
-      const V4<T> W0 = Wbase[gi];
       o = mk4<T>(kc.half * (W0.x - dt * R0 + Wc.x), kc.half * (W0.y - dt * R1 + Wc.y),
                  kc.half * (W0.z - dt * R2 + Wc.z), kc.half * (W0.w - dt * R3 + Wc.w));
     }

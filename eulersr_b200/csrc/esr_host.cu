@@ -156,7 +156,8 @@ struct SolverT : SolverBase {
   // second register budget of each fast float32 kernel (autotuned)
   bool k1_alt = false, k2_alt = false, kp_alt = false;
   // MUSCL stages by the fused kernel (esr_stage.cuh); the separate K1 / K2
-  // remain for fast float32 HLLC at launch shapes that ask for them
+  // remain for fast float32 HLLC at launch shapes that ask for them and for
+  // float64 in the reference's sequence
   bool fused = false;
   DevBuf<int4> d_sblk;   // several meshes: (segment, tile, first slot) per block
   StageLaunch<T> stage{};
@@ -247,7 +248,11 @@ struct SolverT : SolverBase {
   BlockMap<T> bmap() { return BlockMap<T>{d_segs.p, d_blk.p, hseg0, meshes.size() == 1 ? 1 : 0}; }
   // float32 with esr_params.fidelity = ESR_FIDELITY_REFERENCE: the kernels of esr_faithful.cu
   bool faithful() const { return sizeof(T) == 4 && P.fidelity == ESR_FIDELITY_REFERENCE; }
-  static constexpr bool kF = sizeof(T) == 4;   // FAST flag of the kernels this file instantiates
+  static constexpr bool kF = sizeof(T) == 4;   // FAST flag of the separate kernels this file instantiates
+  // Float64 in the reference's operation sequence (fidelity reference) runs the
+  // separate kernels: they are that sequence and no fused stage computes it
+  bool sequence64() const { return sizeof(T) == 8 && P.fidelity == ESR_FIDELITY_REFERENCE; }
+  bool stage_form() const { return muscl() && !sequence64(); }   // the fused stage kernel applies
   // K2 by patches applies to float32 fast-fidelity HLLC + MUSCL solves
   bool patch_eligible() const {
     return sizeof(T) == 4 && !faithful() && P.flux == ESR_FLUX_HLLC && P.reconstruction == ESR_RECON_MUSCL;
@@ -363,7 +368,7 @@ struct SolverT : SolverBase {
       s.lsq = md.lsq.p;
       s.patch_start = md.patch.p;
       s.n_patches = (int)hm.patch_start.size() - 1;
-      if (muscl()) ESR_TRY(upload_tiles(md, s, g));
+      if (stage_form()) ESR_TRY(upload_tiles(md, s, g));
       ESR_TRY(set_divider(s));
       h_live_full.push_back(make_int4(s.B, (int)s.b_magic, s.b_shift, 0));
       hsegs.push_back(s);
@@ -377,7 +382,7 @@ struct SolverT : SolverBase {
     hseg0 = hsegs[0];
     ESR_TRY(build_blocks(block));
     ESR_TRY(build_patch_blocks());
-    if (muscl()) ESR_TRY(build_stage_blocks());
+    if (stage_form()) ESR_TRY(build_stage_blocks());
     ESR_TRY(d_case_seg.alloc(n_slots));
     ESR_TRY(d_case_slot.alloc(n_slots));
     ESR_TRY(d_ncells.alloc(n_slots));
@@ -420,10 +425,8 @@ struct SolverT : SolverBase {
     ESR_CUDA(cudaMemsetAsync(inlet.p, 0, n_slots * sizeof(V), stream));
     hcase_index.assign(n_slots, -1);
     ESR_CUDA(cudaStreamSynchronize(stream));
-    if (p->block_size != 0 && patch_eligible()) {   // a launch shape was asked for
-      fused = false;
-      ESR_TRY(FV.reserve(3 * total));
-    }
+    if (p->block_size != 0 && patch_eligible()) fused = false;   // a launch shape was asked for
+    if (muscl() && !fused) ESR_TRY(FV.reserve(3 * total));
     if (p->block_size == 0) ESR_TRY(autotune());
     return ESR_OK;
   }
@@ -606,7 +609,7 @@ struct SolverT : SolverBase {
     if (faithful()) {
       if constexpr (sizeof(T) == 4) ESR_CUDA(faithful_allow_stage(rus, local));
     } else {
-      ESR_CUDA((allow_stage<T, kF>(rus, local)));
+      ESR_CUDA((allow_stage<T, true>(rus, local)));
     }
     fused = true;
     return ESR_OK;
@@ -670,7 +673,7 @@ struct SolverT : SolverBase {
   int apply_choice(const TuneChoice& c) {
     ESR_TRY(build_blocks(c.block));
     use_patch = c.patches && patch_eligible();
-    fused = muscl() && (c.fused || !patch_eligible());
+    fused = stage_form() && (c.fused || !patch_eligible());
     if (muscl() && !fused) ESR_TRY(FV.reserve(3 * total));
     k1_alt = c.k1;
     k2_alt = c.k2;
@@ -700,7 +703,7 @@ struct SolverT : SolverBase {
   esr_tuning tuning{};
   TuneChoice chosen;
   int autotune() {
-    if (muscl() && !patch_eligible()) return ESR_OK;   // the fused stage kernel alone: nothing to choose
+    if (stage_form() && !patch_eligible()) return ESR_OK;   // the fused stage kernel alone: nothing to choose
     const std::string key = tune_key();
     {
       std::lock_guard<std::mutex> lock(tune_mutex());
@@ -901,11 +904,15 @@ struct SolverT : SolverBase {
         ++launches;
         return;
       }
-      if (muscl()) {   // fast HLLC; every other MUSCL solve runs fused
+      if (muscl()) {   // fast HLLC; every other float32 MUSCL solve runs fused
         if (local) launch_flux<0, true, STAGE, true>(win, wbase, wout, cs, pos);
         else launch_flux<0, true, STAGE, false>(win, wbase, wout, cs, pos);
         return;
       }
+    } else if (muscl()) {   // the reference's sequence
+#define ESR_FLUX_CASE(F, L) if (rus == (F == 1) && local == L) { launch_flux<F, true, STAGE, L>(win, wbase, wout, cs, pos); return; }
+      ESR_FLUX_CASE(0, false) ESR_FLUX_CASE(0, true) ESR_FLUX_CASE(1, false) ESR_FLUX_CASE(1, true)
+#undef ESR_FLUX_CASE
     }
 #define ESR_FLUX_CASE(F, L) if (rus == (F == 1) && local == L) { launch_flux<F, false, STAGE, L>(win, wbase, wout, cs, pos); return; }
     ESR_FLUX_CASE(0, false) ESR_FLUX_CASE(0, true) ESR_FLUX_CASE(1, false) ESR_FLUX_CASE(1, true)
@@ -927,18 +934,17 @@ struct SolverT : SolverBase {
       ++launches;
       return;
     }
-    if constexpr (sizeof(T) == 4) {
-      tap_begin(0);
-      if (write_dt)   // the local-dt K1 keeps its one budget
-        k_recon<T, kF, true, true><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
-      else if (k1_alt)
-        k_recon<T, kF, true, false, ESR_K1_MINB_ALT><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos,
-                                                                                  dt_local.p);
-      else
-        k_recon<T, kF, true, false><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
-      tap_end();
-      ++launches;
+    tap_begin(0);
+    if (write_dt) {   // the local-dt K1 keeps its one budget
+      k_recon<T, kF, true, true><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
+    } else if (sizeof(T) == 4 && k1_alt) {
+      k_recon<T, kF, true, false, (sizeof(T) == 4 ? ESR_K1_MINB_ALT : 0)><<<n_blk, block, 0, stream>>>(
+          bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
+    } else {
+      k_recon<T, kF, true, false><<<n_blk, block, 0, stream>>>(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p);
     }
+    tap_end();
+    ++launches;
   }
   // one Runge-Kutta stage of every live slot: wout from win (and wbase, the
   // state the step started from)
@@ -955,7 +961,7 @@ struct SolverT : SolverBase {
       if constexpr (sizeof(T) == 4)
         faithful_stage(stage, rus, STAGE, local, win, wbase, wout, cs, kc, pos, dt_local.p, res.p, stream);
     } else {
-      launch_stage<T, kF>(stage, rus, STAGE, local, win, wbase, wout, cs, kc, pos, dt_local.p, res.p, stream);
+      launch_stage<T, true>(stage, rus, STAGE, local, win, wbase, wout, cs, kc, pos, dt_local.p, res.p, stream);
     }
     tap_end();
     ++launches;

@@ -21,9 +21,9 @@
 // 569 -> 382; float64 1 x 19,384 37 -> 14, 24 x 25,968 282 -> 153; reference
 // fidelity 1 x 19,384 29 -> 24.
 //
-// CANON (float64 and fast float32): each face of the tile once, from its
-// owner (the lower cell), the flux stored over the two face states it came
-// from, negated for the other cell. Otherwise (reference fidelity): every
+// CANON (fast fidelity): each face of the tile once, from its owner (the
+// lower cell), the flux stored over the two face states it came from, negated
+// for the other cell. Otherwise (reference fidelity): every
 // side of every cell from its own perspective, as the reference evaluates
 // them, into a buffer of its own.
 #pragma once
@@ -174,14 +174,13 @@ template <typename T>
 constexpr int kStageThreads = sizeof(T) == 8 ? ESR_STAGE_THREADS_F64 : 256;
 template <typename T>
 constexpr int kStageBlocks = sizeof(T) == 8 ? ESR_STAGE_MINB_F64 : ESR_STAGE_MINB;
-template <typename T, bool FAST> constexpr bool kCanon = FAST || sizeof(T) == 8;
 
 template <typename T, bool FAST, int FLUX, int STAGE, bool LOCALDT>
 __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
     const StageMap<T> sm, const V4<T>* __restrict__ Win, const V4<T>* Wbase, V4<T>* Wout,
     Cases<T> cs, Consts<T> kc, int pos, T* __restrict__ dt_local, T* __restrict__ res_out, int p_rows, int fv_rows) {
   using V = V4<T>;
-  constexpr bool CANON = kCanon<T, FAST>;
+  constexpr bool CANON = FAST;
   extern __shared__ __align__(16) unsigned char stage_smem[];
   V* P = reinterpret_cast<V*>(stage_smem);      // primitives
   V* FV = P + p_rows;                           // face states; then, when CANON, the fluxes
@@ -215,7 +214,8 @@ __global__ void __launch_bounds__(kStageThreads<T>, kStageBlocks<T>) k_stage(
   if (!__syncthreads_or(live)) return;          // every slot of the group idle
   const V* win = Win + s.off + (in_seg ? b : 0);
   // A: primitives of the tile, its two rings and its ghosts
-  constexpr bool SCALED = kXr<T, FAST> && sizeof(T) == 8;   // the limiter's products have a range (limited_faces)
+  static_assert(FAST || sizeof(T) == 4, "float64 in the reference's sequence runs the separate kernels");
+  constexpr bool SCALED = sizeof(T) == 8;   // the limiter's products have a range (limited_faces)
   int top = 0;                                              // largest exponent word of the primitives
   for (int i = threadIdx.x, c = c0; i < h.n2 << sh; i += nt) {
     T q[4];

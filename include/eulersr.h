@@ -84,14 +84,21 @@ extern "C" {
                                   * face's flux evaluated once and exchanged in shared memory
                                   * (float32 fast fidelity, HLLC + MUSCL; the fluxes are bitwise
                                   * those of the per-cell K2) */
-#define ESR_FIDELITY_FAST 0      /* geometry formed in float64 and rounded once; float32 kernels
-                                  * with approximate division and the direct HLLC flux */
+/* Fidelity of MUSCL solves. Both meet the parity tolerances of their precision
+ * (float64 1e-12 after 100 steps); the mode decides how each operation rounds. */
+#define ESR_FIDELITY_FAST 0      /* geometry formed in float64 and rounded once. float32: approximate
+                                  * reciprocals and square roots (1 ulp). float64: IEEE division and
+                                  * square root. In both the HLLC flux of the selected state itself,
+                                  * each face once (from its owner), explicit multiply-adds and
+                                  * reciprocals in place of repeated divisions */
 #define ESR_FIDELITY_REFERENCE 1 /* the reference's rounding: geometry formed in the run's
                                   * precision in its operation order (mesh.py:223-240,
-                                  * euler_solver.py:49,74,79, helper.py:136-150), the
-                                  * least-squares gradient solved per call (helper.py:136-153)
-                                  * and float32 kernels with IEEE division, the central-flux
-                                  * identity and no fused multiply-add */
+                                  * euler_solver.py:49,74,79, helper.py:136-150). float32: the
+                                  * least-squares gradient solved per call (helper.py:136-153), IEEE
+                                  * division, the central-flux identity, every side of a face from
+                                  * its own cell and no fused multiply-add. float64: the same
+                                  * sequence with the gradient's coefficients formed once per mesh
+                                  * and multiply-adds where the compiler fuses them */
 
 /* Mesh description; all host arrays are owned by the caller and copied. */
 typedef struct esr_mesh_desc {

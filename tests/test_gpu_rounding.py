@@ -65,3 +65,13 @@ def test_float64_limiter_far_from_unit_scale(diamond02, exponent):
     s.step(20)
     assert rel_err(s.get_state(0), W) <= 1e-12
     s.close()
+
+
+@pytest.mark.parametrize("run", ["diamond_hllc_global_SRK2", "naca0012_rusanov_local_RK2", "naca0012_hllc_local_EE"])
+def test_float64_reference_fidelity_keeps_the_sequence(diamond02, naca02, run):
+    """Float64 with fidelity 'reference' computes the reference's sequence of
+    operations, not the fast mode's formulas (third slot of three)."""
+    geom, flux, dt_mode, scheme = run.split("_")
+    got = _steps(diamond02 if geom == "diamond" else naca02, slots=3, precision="f64", fidelity="reference", flux=flux,
+                 dt_mode=dt_mode, time_scheme=scheme)[2]
+    assert np.array_equal(got, np.load(GOLDEN / "float64_sequence.npz")[run])
