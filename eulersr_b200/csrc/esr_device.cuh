@@ -13,8 +13,9 @@
 //              (geo[cell * G_COUNT + field], esr_layout.h), read as float4/double4 groups
 //   stage      one Runge-Kutta stage of a MUSCL solve in one kernel
 //              (esr_stage.cuh); the separate pair below remains for fast
-//              float32 HLLC at a requested launch shape and for float64 in
-//              the reference's sequence, K2 also for constant reconstruction
+//              float32 HLLC at a requested launch shape and for reference
+//              fidelity (float64, and float32 batches), K2 also for constant
+//              reconstruction
 //   K1 recon   cell + 3 neighbour primitives, LSQ gradient, Venkatakrishnan
 //              limiter, the 3 MUSCL face states of the cell -> FV[k][item]
 //   K2 flux    per cell: the 3 face fluxes (HLLC or Rusanov) from its own
@@ -920,10 +921,11 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, FAST, MINB, ESR_K2_MINB>))
     Wout[gi] = o;
   } else {
     T acc[4];
-    // The step's first state, on its way before the fluxes (float64 48 x 25,968
-    // cells 443 -> 434 us per step) except in fast float32, which is short of
-    // registers (constant reconstruction 32 x 25,968 43.1 -> 44.6 with it)
-    constexpr bool EARLY = STAGE != ST_FIRST && !kFastPath<T, FAST>;
+    // The step's first state, on its way before the fluxes where registers allow:
+    // float64 48 x 25,968 cells 443 -> 434 us per step, reference fidelity with
+    // constant reconstruction 256 x 25,968 572 -> 555; not in fast float32 (32 x
+    // 25,968 43.1 -> 44.6) nor with float32 face states (64 x 1,810 43.7 -> 45.6)
+    constexpr bool EARLY = STAGE != ST_FIRST && !kFastPath<T, FAST> && (sizeof(T) == 8 || !MUSCL);
     V4<T> W0 = Wc;
     if (EARLY) W0 = Wbase[gi];
   #pragma unroll

@@ -5,9 +5,12 @@
 
 namespace esr {
 
-void faithful_local_dt(const BlockMap<float>& bm, const float4* W, const Cases<float>& cs, const Consts<float>& kc,
-                       int pos, float* dt_local, int n_blk, int block, cudaStream_t st) {
-  k_recon<float, false, false, true><<<n_blk, block, 0, st>>>(bm, W, nullptr, 0, cs, kc, pos, dt_local);
+void faithful_recon(const BlockMap<float>& bm, const float4* W, float4* FV, long long total, const Cases<float>& cs,
+                    const Consts<float>& kc, int pos, float* dt_local, bool muscl, bool localdt, int n_blk, int block,
+                    cudaStream_t st) {
+  if (!muscl) k_recon<float, false, false, true><<<n_blk, block, 0, st>>>(bm, W, nullptr, 0, cs, kc, pos, dt_local);
+  else if (localdt) k_recon<float, false, true, true><<<n_blk, block, 0, st>>>(bm, W, FV, total, cs, kc, pos, dt_local);
+  else k_recon<float, false, true, false><<<n_blk, block, 0, st>>>(bm, W, FV, total, cs, kc, pos, dt_local);
 }
 
 void faithful_stage(const StageLaunch<float>& L, bool rusanov, int stage, bool local, const float4* win,
@@ -18,30 +21,37 @@ void faithful_stage(const StageLaunch<float>& L, bool rusanov, int stage, bool l
 cudaError_t faithful_allow_stage(bool rusanov, bool local) {
   return allow_stage<float, false>(rusanov, local);
 }
+cudaError_t faithful_stage_residents(const StageLaunch<float>& L, bool rusanov, bool local, int* blocks) {
+  cudaError_t e = cudaSuccess;
+  stage_form(rusanov, ST_FIRST, local, [&](auto f, auto s, auto l) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_stage<float, false, f(), s(), l()>, L.threads, L.smem);
+  });
+  return e;
+}
 
 template <int STAGE>
 static void flux_stage(const BlockMap<float>& bm, const float4* win, const float4* wbase, float4* wout,
-                       const Cases<float>& cs, const Consts<float>& kc, int pos, const float* dt_local, float* res,
-                       bool rus, bool local, int n_blk, int block, cudaStream_t st) {
-#define ESR_FF(F, L)                                                                                          \
-  if (rus == (F == 1) && local == L) {                                                                        \
-    k_flux<float, false, F, false, STAGE, L><<<n_blk, block, 0, st>>>(bm, win, wbase, wout, nullptr, 0, cs, kc, \
-                                                                      pos, dt_local, res);                    \
-    return;                                                                                                   \
+                       const float4* FV, long long total, const Cases<float>& cs, const Consts<float>& kc, int pos,
+                       const float* dt_local, float* res, bool rus, bool muscl, bool local, int n_blk, int block,
+                       cudaStream_t st) {
+#define ESR_FF(F, M, L)                                                                                          \
+  if (rus == (F == 1) && muscl == M && local == L) {                                                             \
+    k_flux<float, false, F, M, STAGE, L><<<n_blk, block, 0, st>>>(bm, win, wbase, wout, FV, total, cs, kc, pos, \
+                                                                  dt_local, res);                               \
+    return;                                                                                                      \
   }
-  ESR_FF(0, false) ESR_FF(0, true) ESR_FF(1, false) ESR_FF(1, true)
+  ESR_FF(0, true, false) ESR_FF(0, true, true) ESR_FF(0, false, false) ESR_FF(0, false, true)
+  ESR_FF(1, true, false) ESR_FF(1, true, true) ESR_FF(1, false, false) ESR_FF(1, false, true)
 #undef ESR_FF
 }
 
 void faithful_flux(int stage, const BlockMap<float>& bm, const float4* win, const float4* wbase, float4* wout,
-                   const Cases<float>& cs, const Consts<float>& kc, int pos, const float* dt_local, float* res,
-                   bool rusanov, bool localdt, int n_blk, int block, cudaStream_t st) {
-  if (stage == ST_FIRST)
-    flux_stage<ST_FIRST>(bm, win, wbase, wout, cs, kc, pos, dt_local, res, rusanov, localdt, n_blk, block, st);
-  else if (stage == ST_SRK2_SECOND)
-    flux_stage<ST_SRK2_SECOND>(bm, win, wbase, wout, cs, kc, pos, dt_local, res, rusanov, localdt, n_blk, block, st);
-  else
-    flux_stage<ST_RK2_SECOND>(bm, win, wbase, wout, cs, kc, pos, dt_local, res, rusanov, localdt, n_blk, block, st);
+                   const float4* FV, long long total, const Cases<float>& cs, const Consts<float>& kc, int pos,
+                   const float* dt_local, float* res, bool rusanov, bool muscl, bool localdt, int n_blk, int block,
+                   cudaStream_t st) {
+  auto* run = stage == ST_FIRST ? flux_stage<ST_FIRST> : stage == ST_SRK2_SECOND ? flux_stage<ST_SRK2_SECOND>
+                                                                                  : flux_stage<ST_RK2_SECOND>;
+  run(bm, win, wbase, wout, FV, total, cs, kc, pos, dt_local, res, rusanov, muscl, localdt, n_blk, block, st);
 }
 
 void faithful_dtmin(dim3 grid, int threads, const Seg<float>* segs, CaseMap cm, const float4* W, const int* due,

@@ -157,7 +157,7 @@ struct SolverT : SolverBase {
   bool k1_alt = false, k2_alt = false, kp_alt = false;
   // MUSCL stages by the fused kernel (esr_stage.cuh); the separate K1 / K2
   // remain for fast float32 HLLC at launch shapes that ask for them and for
-  // float64 in the reference's sequence
+  // reference fidelity (float64, and float32 batches)
   bool fused = false;
   DevBuf<int4> d_sblk;   // several meshes: (segment, tile, first slot) per block
   StageLaunch<T> stage{};
@@ -252,7 +252,16 @@ struct SolverT : SolverBase {
   // Float64 in the reference's operation sequence (fidelity reference) runs the
   // separate kernels: they are that sequence and no fused stage computes it
   bool sequence64() const { return sizeof(T) == 8 && P.fidelity == ESR_FIDELITY_REFERENCE; }
-  bool stage_form() const { return muscl() && !sequence64(); }   // the fused stage kernel applies
+  // The fused stage kernel runs (patch_eligible solves can also run the separate
+  // kernels). Reference fidelity in float32 takes it while all blocks of a stage
+  // are resident at once and a thread reconstructs one cell, so that a launch's
+  // latency counts (1 slot x 25,968 cells 37.6 -> 28.7 us per step, 2 x 25,968
+  // 39.2 -> 32.1, 28 x 1,810 37.2 -> 34.2), and the separate kernels beyond
+  // that: its dear reconstruction (four 2x2 solves in float64 a cell) is not
+  // worth repeating for every tile's ring (3 x 25,968 43.0 against 49.4, 32 x
+  // 1,810 36.2 against 39.7, 100 x 25,968 593 against 741).
+  bool stage_form() const { return muscl() && !sequence64() && one_pass; }
+  bool one_pass = true;   // set by build_stage_blocks
   // K2 by patches applies to float32 fast-fidelity HLLC + MUSCL solves
   bool patch_eligible() const {
     return sizeof(T) == 4 && !faithful() && P.flux == ESR_FLUX_HLLC && P.reconstruction == ESR_RECON_MUSCL;
@@ -368,7 +377,7 @@ struct SolverT : SolverBase {
       s.lsq = md.lsq.p;
       s.patch_start = md.patch.p;
       s.n_patches = (int)hm.patch_start.size() - 1;
-      if (stage_form()) ESR_TRY(upload_tiles(md, s, g));
+      if (muscl() && !sequence64()) ESR_TRY(upload_tiles(md, s, g));
       ESR_TRY(set_divider(s));
       h_live_full.push_back(make_int4(s.B, (int)s.b_magic, s.b_shift, 0));
       hsegs.push_back(s);
@@ -382,7 +391,7 @@ struct SolverT : SolverBase {
     hseg0 = hsegs[0];
     ESR_TRY(build_blocks(block));
     ESR_TRY(build_patch_blocks());
-    if (stage_form()) ESR_TRY(build_stage_blocks());
+    if (muscl() && !sequence64()) ESR_TRY(build_stage_blocks(sms));
     ESR_TRY(d_case_seg.alloc(n_slots));
     ESR_TRY(d_case_slot.alloc(n_slots));
     ESR_TRY(d_ncells.alloc(n_slots));
@@ -566,14 +575,16 @@ struct SolverT : SolverBase {
     max_fv = std::max(max_fv, ts.max_slots);
     max_own = std::max(max_own, ts.max_own);
     max_shift = std::max(max_shift, s.slot_shift);
+    for (const TileHead& h : ts.head) max_ring = std::max(max_ring, h.n1 << s.slot_shift);
     n_tiles.push_back(ts.n_tiles);
     return ESR_OK;
   }
   int max_p = 0, max_fv = 0, max_own = 0, max_shift = 0;
+  int max_ring = 0;   // most (own or ring-1 cell, slot) pairs of a block
   std::vector<int> n_tiles;
   // grid of the fused kernel: every tile x groups of slots, the groups of one
   // tile next to each other (their state rows are)
-  int build_stage_blocks() {
+  int build_stage_blocks(int sms) {
     stage.map.segs = d_segs.p;
     stage.map.seg0 = hseg0;
     std::vector<int4> h;
@@ -607,11 +618,16 @@ struct SolverT : SolverBase {
     if (stage.smem > kStageSmemMax) return fail(ESR_ERR_STATE, "stage tiles need more shared memory than a block has");
     const bool rus = P.flux == ESR_FLUX_RUSANOV, local = P.dt_mode == ESR_DT_LOCAL;
     if (faithful()) {
-      if constexpr (sizeof(T) == 4) ESR_CUDA(faithful_allow_stage(rus, local));
+      if constexpr (sizeof(T) == 4) {
+        ESR_CUDA(faithful_allow_stage(rus, local));
+        int resident = 0;
+        ESR_CUDA(faithful_stage_residents(stage, rus, local, &resident));
+        one_pass = max_ring <= stage.threads && stage.blocks <= (long long)resident * sms;
+      }
     } else {
       ESR_CUDA((allow_stage<T, true>(rus, local)));
     }
-    fused = true;
+    fused = one_pass;
     return ESR_OK;
   }
 
@@ -889,9 +905,10 @@ struct SolverT : SolverBase {
     const bool local = P.dt_mode == ESR_DT_LOCAL;
     const bool rus = P.flux == ESR_FLUX_RUSANOV;
     if constexpr (sizeof(T) == 4) {
-      if (faithful()) {   // constant reconstruction
+      if (faithful()) {
         tap_begin(1);
-        faithful_flux(STAGE, bmap(), win, wbase, wout, cs, kc, pos, dt_local.p, res.p, rus, local, n_blk, block, stream);
+        faithful_flux(STAGE, bmap(), win, wbase, wout, FV.p, total, cs, kc, pos, dt_local.p, res.p, rus, muscl(), local,
+                      n_blk, block, stream);
         tap_end();
         ++launches;
         return;
@@ -904,7 +921,7 @@ struct SolverT : SolverBase {
         ++launches;
         return;
       }
-      if (muscl()) {   // fast HLLC; every other float32 MUSCL solve runs fused
+      if (muscl()) {   // fast HLLC (fast Rusanov runs fused)
         if (local) launch_flux<0, true, STAGE, true>(win, wbase, wout, cs, pos);
         else launch_flux<0, true, STAGE, false>(win, wbase, wout, cs, pos);
         return;
@@ -920,16 +937,16 @@ struct SolverT : SolverBase {
   }
   void recon(const V* w, const Cases<T>& cs, int pos, bool write_dt) {
     if (!muscl() && !write_dt) return;   // constant reconstruction needs K1 only for the local dt
-    if (!muscl()) {
-      if constexpr (sizeof(T) == 4) {
-        if (faithful()) {
-          tap_begin(0);
-          faithful_local_dt(bmap(), w, cs, kc, pos, dt_local.p, n_blk, block, stream);
-          tap_end();
-          ++launches;
-          return;
-        }
+    if constexpr (sizeof(T) == 4) {
+      if (faithful()) {
+        tap_begin(0);
+        faithful_recon(bmap(), w, FV.p, total, cs, kc, pos, dt_local.p, muscl(), write_dt, n_blk, block, stream);
+        tap_end();
+        ++launches;
+        return;
       }
+    }
+    if (!muscl()) {
       k_recon<T, kF, false, true><<<n_blk, block, 0, stream>>>(bmap(), w, nullptr, 0, cs, kc, pos, dt_local.p);
       ++launches;
       return;

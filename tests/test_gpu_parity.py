@@ -611,3 +611,29 @@ def test_solvers_share_a_mesh_and_outlive_it(diamond02, precision, fidelity):
         dm.close()
     _, b = states(dm, 2, drop)
     assert np.array_equal(a, own) and np.array_equal(b, own)
+
+
+@pytest.mark.parametrize("slots,fused", [(1, True), (9, True), (100, False)])
+@pytest.mark.parametrize("flux,scheme,dt_mode", [("hllc", "SRK2", "local"), ("rusanov", "RK2", "global"),
+                                                 ("hllc", "EE", "global")])
+def test_reference_fidelity_batches_take_the_separate_kernels(naca02, slots, fused, flux, scheme, dt_mode):
+    """Float32 reference fidelity: the fused stage while one wave of its blocks
+    covers the solve, the separate kernels beyond; both give the bits of a
+    single solve of the same case."""
+    from eulersr_b200.solver import DeviceMesh, FlowCase, Solver
+    dm = DeviceMesh(naca02)
+    r = np.random.default_rng(3)
+    cases = [FlowCase(mach=float(r.uniform(0.7, 3.0)), aoa_deg=float(r.uniform(-5, 5)), tf=1.0, dtype=np.float32)
+             for _ in range(slots)]
+    opts = dict(precision="f32", fidelity="reference", flux=flux, time_scheme=scheme, dt_mode=dt_mode)
+    s = Solver(dm, slots, **opts)
+    s.set_cases(list(range(slots)), cases)
+    assert (s.profile_step(1)["recon_launches"] == 0) == fused
+    s.step(6)
+    for g in sorted({0, slots // 2, slots - 1}):
+        one = Solver(dm, 1, **opts)
+        one.set_case(0, cases[g])
+        one.step(7)
+        assert np.array_equal(one.get_state(0), s.get_state(g)), g
+        one.close()
+    s.close()
