@@ -158,7 +158,7 @@ __device__ __forceinline__ void block_origin(const BlockMap<T>& bm, Seg<T>& s, i
 // divides. Constant reconstruction keeps the sequence in every mode, with
 // __fdividef in fast float32.
 template <typename T, bool FAST> constexpr bool kFastPath = FAST && sizeof(T) == 4;
-// MUSCL kernels whose numerics are the xr:: functions (the Rusanov flux itself has none)
+// MUSCL kernels whose numerics are the xr:: functions (but for the float64 Rusanov flux)
 template <typename T, bool FAST> constexpr bool kXr = FAST;
 template <typename T, bool FAST = (sizeof(T) == 4)>
 __device__ __forceinline__ T dv(T a, T b) {
@@ -550,6 +550,36 @@ __device__ __forceinline__ void hllc(const V PL[4], const V PR[4], Scalar<V> nx_
   F[1] = sub(mul(Fn, nx), mul(Ft, ny));
   F[2] = fma(Fn, ny, mul(Ft, nx));
   F[3] = mul(add(E, p), un);
+}
+// euler_solver.py:203-240 Rusanov flux of two face states (primitive) through
+// the unit normal: the mean of the physical fluxes less C/2 times the jump of
+// the conserved states, C the larger of |un| + a. The sound speed's root is the
+// IEEE one: it scales the whole dissipation.
+__device__ __forceinline__ float root_rn(float x) { return __fsqrt_rn(x); }
+__device__ __forceinline__ float2 root_rn(float2 a) { return make_float2(__fsqrt_rn(a.x), __fsqrt_rn(a.y)); }
+template <typename V>
+__device__ __forceinline__ void rusanov(const V PL[4], const V PR[4], Scalar<V> nx_, Scalar<V> ny_,
+                                        const Consts<Scalar<V>>& k, V F[4]) {
+  const V nx = splat<V>(nx_), ny = splat<V>(ny_), half = splat<V>(k.half);
+  V C, sum[4], jump[4];
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    const V* P = side ? PR : PL;
+    const V r = P[0], u = P[1], v = P[2], p = P[3], un = fma(u, nx, mul(v, ny));
+    const V E = fma(mul(half, r), fma(u, u, mul(v, v)), mul(p, splat<V>(k.inv_gm1)));
+    const V W[4] = {r, mul(r, u), mul(r, v), E}, m = mul(r, un);
+    const V Fk[4] = {m, fma(m, u, mul(p, nx)), fma(m, v, mul(p, ny)), mul(add(E, p), un)};
+    const V c = add(root_rn(mag(mul(mul(splat<V>(k.gamma), p), rcp(r)))), mag(un));
+    C = side ? upper(c, C) : c;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      sum[i] = side ? add(sum[i], Fk[i]) : Fk[i];
+      jump[i] = side ? sub(W[i], jump[i]) : W[i];
+    }
+  }
+  const V mc = neg(C);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) F[i] = mul(half, fma(mc, jump[i], sum[i]));
 }
 // the canonical flux of a face through the cell's edge of outward normal n:
 // evaluated from the face's owner (the lower cell), negated on the other side

@@ -22,11 +22,7 @@ cudaError_t faithful_allow_stage(bool rusanov, bool local) {
   return allow_stage<float, false>(rusanov, local);
 }
 cudaError_t faithful_stage_residents(const StageLaunch<float>& L, bool rusanov, bool local, int* blocks) {
-  cudaError_t e = cudaSuccess;
-  stage_form(rusanov, ST_FIRST, local, [&](auto f, auto s, auto l) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_stage<float, false, f(), s(), l()>, L.threads, L.smem);
-  });
-  return e;
+  return stage_residents<float, false>(L, rusanov, local, blocks);
 }
 
 template <int STAGE>

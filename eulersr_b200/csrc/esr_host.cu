@@ -582,51 +582,80 @@ struct SolverT : SolverBase {
   int max_p = 0, max_fv = 0, max_own = 0, max_shift = 0;
   int max_ring = 0;   // most (own or ring-1 cell, slot) pairs of a block
   std::vector<int> n_tiles;
-  // grid of the fused kernel: every tile x groups of slots, the groups of one
-  // tile next to each other (their state rows are)
-  int build_stage_blocks(int sms) {
-    stage.map.segs = d_segs.p;
-    stage.map.seg0 = hseg0;
-    std::vector<int4> h;
+  // Grid and shared memory of the fused kernel: every tile x groups of slots.
+  // packed: pairs of slots (k_stage_pair), whose blocks all cover the widest
+  // mesh's number of slots; otherwise each mesh has groups of its own width.
+  int group_width(int m, bool packed) const { return 1 << (packed ? max_shift : slot_shift_of(meshes[m]->B)); }
+  int layout_stage(bool packed) {
     long long blocks = 0;
-    const bool packed = patch_eligible() && max_shift >= 1;
     for (int m = 0; m < (int)meshes.size(); ++m) {
-      const int w = 1 << (packed ? max_shift : slot_shift_of(meshes[m]->B)), groups = (meshes[m]->B + w - 1) / w;
-      blocks += (long long)n_tiles[m] * groups;
-      stage.map.groups = groups;
-      if (meshes.size() > 1)
-        for (int t = 0; t < n_tiles[m]; ++t)
-          for (int q = 0; q < groups; ++q) h.push_back(make_int4(m, t, q * w, 0));
+      const int w = group_width(m, packed);
+      blocks += (long long)n_tiles[m] * ((meshes[m]->B + w - 1) / w);
     }
     if (blocks > INT_MAX) return fail(ESR_ERR_ARG, "solver: too many tiles x slot groups");
-    if (meshes.size() > 1) {
-      ESR_TRY(d_sblk.alloc(h.size()));
-      ESR_CUDA(cudaMemcpy(d_sblk.p, h.data(), h.size() * sizeof(int4), cudaMemcpyHostToDevice));
-      stage.map.groups = 0;
-    }
-    stage.map.blk = d_sblk.p;
     stage.blocks = (int)blocks;
-    // pairs of slots once any mesh has two: the packed kernel (fast float32
-    // HLLC), whose blocks all cover the widest mesh's number of slots
-    stage.pairs = patch_eligible() && max_shift >= 1 ? max_shift - 1 : -1;
-    stage.threads = stage.pairs >= 0 ? kPairThreads : (max_own << max_shift) <= 64 ? 128 : kStageThreads<T>;
-    const int rows = stage.pairs >= 0 ? stage.pairs : max_shift;
+    stage.pairs = packed ? max_shift - 1 : -1;
+    stage.threads = packed ? kPairThreads : (max_own << max_shift) <= 64 ? 128 : kStageThreads<T>;
+    const int rows = packed ? stage.pairs : max_shift;
     stage.p_rows = max_p << rows;
     stage.fv_rows = max_fv << rows;
     const int fx_rows = faithful() ? (3 * max_own) << rows : 0;
-    stage.smem = (stage.p_rows + stage.fv_rows + fx_rows) * (int)sizeof(V) * (stage.pairs >= 0 ? 2 : 1);
+    stage.smem = (stage.p_rows + stage.fv_rows + fx_rows) * (int)sizeof(V) * (packed ? 2 : 1);
     if (stage.smem > kStageSmemMax) return fail(ESR_ERR_STATE, "stage tiles need more shared memory than a block has");
+    return ESR_OK;
+  }
+  // all blocks of the laid-out k_stage are resident at once and no thread
+  // reconstructs more than `passes` cells: a launch's latency is what counts
+  int latency_bound(int passes, int sms, bool* yes) {
+    const bool rus = P.flux == ESR_FLUX_RUSANOV, local = P.dt_mode == ESR_DT_LOCAL;
+    int resident = 0;
+    if (faithful()) {
+      if constexpr (sizeof(T) == 4) ESR_CUDA(faithful_stage_residents(stage, rus, local, &resident));
+    } else {
+      ESR_CUDA((stage_residents<T, true>(stage, rus, local, &resident)));
+    }
+    *yes = max_ring <= passes * stage.threads && stage.blocks <= (long long)resident * sms;
+    return ESR_OK;
+  }
+  // Which form runs, and its block table (the groups of one tile are next to
+  // each other: their state rows are)
+  int build_stage_blocks(int sms) {
     const bool rus = P.flux == ESR_FLUX_RUSANOV, local = P.dt_mode == ESR_DT_LOCAL;
     if (faithful()) {
-      if constexpr (sizeof(T) == 4) {
-        ESR_CUDA(faithful_allow_stage(rus, local));
-        int resident = 0;
-        ESR_CUDA(faithful_stage_residents(stage, rus, local, &resident));
-        one_pass = max_ring <= stage.threads && stage.blocks <= (long long)resident * sms;
-      }
+      if constexpr (sizeof(T) == 4) ESR_CUDA(faithful_allow_stage(rus, local));
     } else {
       ESR_CUDA((allow_stage<T, true>(rus, local)));
     }
+    ESR_TRY(layout_stage(false));
+    if (faithful()) ESR_TRY(latency_bound(1, sms, &one_pass));
+    // Pairs of slots once any mesh has two (fast float32). Rusanov, whose flux
+    // is the cheaper one, keeps k_stage where latency bounds the solve (us per
+    // step of 9 x 1,810 cells 9.6 against 12.5, 3 x 25,968 15.4 against 16.5, but 5 x
+    // 25,968 23.8 against 22.6 and 256 x 25,968 618 against 440).
+    bool packed = fast_float() && max_shift >= 1;
+    if (packed && rus) {
+      bool small = false;
+      ESR_TRY(latency_bound(2, sms, &small));
+      packed = !small;
+    }
+    if (packed) ESR_TRY(layout_stage(true));
+    std::vector<int4> h;
+    stage.map.segs = d_segs.p;
+    stage.map.seg0 = hseg0;
+    stage.map.groups = 0;
+    if (meshes.size() == 1) {
+      const int w = group_width(0, packed);
+      stage.map.groups = (meshes[0]->B + w - 1) / w;
+    } else {
+      for (int m = 0; m < (int)meshes.size(); ++m) {
+        const int w = group_width(m, packed);
+        for (int t = 0; t < n_tiles[m]; ++t)
+          for (int b0 = 0; b0 < meshes[m]->B; b0 += w) h.push_back(make_int4(m, t, b0, 0));
+      }
+      ESR_TRY(d_sblk.alloc(h.size()));
+      ESR_CUDA(cudaMemcpy(d_sblk.p, h.data(), h.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    }
+    stage.map.blk = d_sblk.p;
     fused = one_pass;
     return ESR_OK;
   }

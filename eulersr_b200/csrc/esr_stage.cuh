@@ -124,6 +124,8 @@ template <typename T, bool FAST, int FLUX>
 __device__ __forceinline__ void stage_flux(T qL[4], T qR[4], T nx, T ny, const Consts<T>& kc, T F[4]) {
   if constexpr (kXr<T, FAST> && FLUX == 0) {
     xr::hllc<T>(qL, qR, nx, ny, kc, F);
+  } else if constexpr (kFastPath<T, FAST>) {
+    xr::rusanov<T>(qL, qR, nx, ny, kc, F);
   } else {
     const V4<T> WL = cons<T, FAST>(qL, kc.gm1, kc.inv_gm1, kc.half), WR = cons<T, FAST>(qR, kc.gm1, kc.inv_gm1, kc.half);
     if constexpr (!kXr<T, FAST>) {   // the reference's conserved round trip
@@ -357,7 +359,7 @@ __device__ __forceinline__ void base_pair(const float4* p, int dB, bool wide, fl
   }
 }
 
-// The same stage for batches of the fast float32 HLLC solve, two case slots
+// The same stage for batches of the fast float32 solve, two case slots
 // per thread: every multiply and add of the pair is one packed instruction,
 // and the geometry, the neighbour records and the addresses are fetched once
 // for both. 1 << SH pairs of slots per block. The roundings are k_stage's.
@@ -388,7 +390,7 @@ __device__ __forceinline__ void pair_of(const float4& a, const float4& b, float2
   q[2] = make_float2(a.z, b.z); q[3] = make_float2(a.w, b.w);
 }
 
-template <int STAGE, bool LOCALDT, int SH>
+template <int FLUX, int STAGE, bool LOCALDT, int SH>
 __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
     const StageMap<float> sm, const float4* __restrict__ Win, const float4* Wbase, float4* Wout, Cases<float> cs,
     Consts<float> kc, int pos, float* __restrict__ dt_local, float* __restrict__ res_out, int p_rows, int fv_rows) {
@@ -507,7 +509,8 @@ __global__ void __launch_bounds__(kPairThreads, ESR_PAIR_MINB) k_stage_pair(
     float2 qL[4], qR[4], F[4];
     load_pair(F0, F1, iL, qL);
     load_pair(inner ? F0 : P0, inner ? F1 : P1, iR, qR);
-    xr::hllc<float2>(qL, qR, f.nx, f.ny, kc, F);
+    if constexpr (FLUX == 0) xr::hllc<float2>(qL, qR, f.nx, f.ny, kc, F);
+    else xr::rusanov<float2>(qL, qR, f.nx, f.ny, kc, F);
     store_pair(F0, F1, iL, F);
     if (inner) {
 #pragma unroll
@@ -603,9 +606,10 @@ void stage_form(bool rusanov, int stage, bool local, F&& fn) {
   if (rusanov) with_stage(std::integral_constant<int, 1>{});
   else with_stage(std::integral_constant<int, 0>{});
 }
-template <int STAGE, bool LOCALDT>
+template <int FLUX, int STAGE, bool LOCALDT>
 auto pair_kernel(int sh) {
-  return sh == 0 ? k_stage_pair<STAGE, LOCALDT, 0> : sh == 1 ? k_stage_pair<STAGE, LOCALDT, 1> : k_stage_pair<STAGE, LOCALDT, 2>;
+  return sh == 0 ? k_stage_pair<FLUX, STAGE, LOCALDT, 0>
+       : sh == 1 ? k_stage_pair<FLUX, STAGE, LOCALDT, 1> : k_stage_pair<FLUX, STAGE, LOCALDT, 2>;
 }
 template <typename T, bool FAST>
 cudaError_t launch_stage(const StageLaunch<T>& L, bool rusanov, int stage, bool local, const V4<T>* win,
@@ -624,9 +628,18 @@ cudaError_t launch_stage(const StageLaunch<T>& L, bool rusanov, int stage, bool 
   cudaError_t e = cudaSuccess;
   stage_form(rusanov, stage, local, [&](auto f, auto s, auto l) {
     auto* k = &k_stage<T, FAST, f(), s(), l()>;
-    if constexpr (kFastPath<T, FAST> && f() == 0)
-      if (L.pairs >= 0) k = pair_kernel<s(), l()>(L.pairs);
+    if constexpr (kFastPath<T, FAST>)
+      if (L.pairs >= 0) k = pair_kernel<f(), s(), l()>(L.pairs);
     e = cudaLaunchKernelEx(&cfg, k, L.map, win, wbase, wout, cs, kc, pos, dt_local, res, L.p_rows, L.fv_rows);
+  });
+  return e;
+}
+// blocks of a k_stage of this layout that an SM holds at once
+template <typename T, bool FAST>
+cudaError_t stage_residents(const StageLaunch<T>& L, bool rusanov, bool local, int* blocks) {
+  cudaError_t e = cudaSuccess;
+  stage_form(rusanov, ST_FIRST, local, [&](auto f, auto s, auto l) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_stage<T, FAST, f(), s(), l()>, L.threads, L.smem);
   });
   return e;
 }
@@ -642,9 +655,9 @@ cudaError_t allow_stage(bool rusanov, bool local) {
       const cudaError_t r = cudaFuncSetAttribute(k_stage<T, FAST, f(), s(), l()>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmemMax);
       if (e == cudaSuccess) e = r;
-      if constexpr (kFastPath<T, FAST> && f() == 0)
+      if constexpr (kFastPath<T, FAST>)
         for (int sh = 0; sh <= 2 && e == cudaSuccess; ++sh)
-          e = cudaFuncSetAttribute(pair_kernel<s(), l()>(sh), cudaFuncAttributeMaxDynamicSharedMemorySize,
+          e = cudaFuncSetAttribute(pair_kernel<f(), s(), l()>(sh), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kStageSmemMax);
     });
   return e;

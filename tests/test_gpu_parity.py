@@ -637,3 +637,41 @@ def test_reference_fidelity_batches_take_the_separate_kernels(naca02, slots, fus
         assert np.array_equal(one.get_state(0), s.get_state(g)), g
         one.close()
     s.close()
+
+
+@pytest.mark.parametrize("slots", [2, 3, 8, 9, 90, 131])
+@pytest.mark.parametrize("scheme,dt_mode", [("SRK2", "global"), ("RK2", "local"), ("EE", "global")])
+def test_rusanov_batches_equal_single_solves(diamond02, naca02, slots, scheme, dt_mode):
+    """Fast float32 Rusanov: k_stage while latency bounds the solve, pairs of
+    slots (k_stage_pair) beyond, give the bits of a single solve of the case,
+    on one mesh and on two of unequal slot counts, with a slot left idle."""
+    from eulersr_b200.solver import DeviceMesh, FlowCase, Solver
+    dms = [DeviceMesh(naca02), DeviceMesh(diamond02)]
+    opts = dict(precision="f32", flux="rusanov", time_scheme=scheme, dt_mode=dt_mode)
+    r = np.random.default_rng(slots)
+    for counts in ([slots], [slots, max(1, slots // 3)]):
+        n = sum(counts)
+        cases = [FlowCase(mach=float(r.uniform(0.7, 3.0)), aoa_deg=float(r.uniform(-5, 5)), tf=1.0, dtype=np.float32)
+                 for _ in range(n)]
+        s = Solver(dms[:len(counts)], counts, **opts)
+        run = [g for g in range(n) if n < 3 or g != 1]
+        s.set_cases(run, [cases[g] for g in run])
+        s.step(7)
+        for g in sorted({0, slots // 2, slots - 1, n - 1} & set(run)):
+            one = Solver(dms[0 if g < slots else 1], 1, **opts)
+            one.set_case(0, cases[g])
+            one.step(7)
+            want, got = one.get_state(0), s.get_state(g)
+            assert np.isfinite(want).all() and np.array_equal(want, got), (counts, g)
+            one.close()
+        s.close()
+
+
+def test_rusanov_fast_f32_is_as_exact_as_the_reference_float32(diamond02):
+    """20 steps of the fast float32 Rusanov solve end no further from the
+    float64 oracle than 1.5 times the oracle's own float32 (the bar of the
+    HLLC solve above)."""
+    Wo32, _, _, _ = _oracle_steps(diamond02, np.float32, 2.5, 5.0, 20, flux="rusanov")
+    Wo64, _, _, _ = _oracle_steps(diamond02, np.float64, 2.5, 5.0, 20, flux="rusanov")
+    Wg, _, _ = _gpu_steps(diamond02, "f32", 2.5, 5.0, 20, flux="rusanov", fidelity="fast")
+    assert rel_err(Wg, Wo64) <= 1.5 * rel_err(Wo32, Wo64)
