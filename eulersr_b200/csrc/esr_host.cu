@@ -494,6 +494,24 @@ struct SolverT : SolverBase {
     const long long enough = (long long)ESR_STAGE_BLOCKS * sms;
     if (blocks() < enough) tile_cells = std::min(tile_cells, 32);
     if (blocks() < enough) slot_bytes = 64;
+    // k_stage_pair gives every mesh groups of the widest mesh's number of slots.
+    // Half the width where that leaves a fifth fewer slots computed for nothing
+    // (us per step, 8 -> 4 slots a group: 9 x 25,968 cells 40.1 -> 33.1, 17 53.3 ->
+    // 48.9, 1 x 25,968 beside 64 x 1,810 35.2 -> 28.7; below that the full lines
+    // win, 33 x 25,968 77.0 against 79.1, 24 x 25,968 50.6 against 55.4).
+    if (fast_float() && slot_bytes == 128) {
+      const double full = (double)group_slots(nm);
+      slot_bytes = 64;
+      if (full < 1.2 * (double)group_slots(nm)) slot_bytes = 128;
+    }
+  }
+  // cells x slots that blocks as wide as the widest mesh's groups compute
+  long long group_slots(int nm) const {
+    int sh = 0;
+    long long n = 0;
+    for (int m = 0; m < nm; ++m) sh = std::max(sh, slot_shift_of(meshes[m]->B));
+    for (int m = 0; m < nm; ++m) n += (long long)meshes[m]->hm->n_cells * ((meshes[m]->B + (1 << sh) - 1) >> sh << sh);
+    return n;
   }
   int slot_shift_of(int B) const {
     int sh = 0;
@@ -632,7 +650,19 @@ struct SolverT : SolverBase {
     // is the cheaper one, keeps k_stage where latency bounds the solve (us per
     // step of 9 x 1,810 cells 9.6 against 12.5, 3 x 25,968 15.4 against 16.5, but 5 x
     // 25,968 23.8 against 22.6 and 256 x 25,968 618 against 440).
+    // Neither where meshes of one slot make up most of the solve: each mesh has
+    // groups of its own width in k_stage, and a pair costs 0.7 of two single slots
+    // (one slot on each of 25,968 and 19,384 cells beside 64 x 1,810: equal, 32.1
+    // and 31.5 us per step, at 1.84 times the slots).
     bool packed = fast_float() && max_shift >= 1;
+    if (packed) {
+      long long own = 0;
+      for (const auto& md : meshes) {
+        const int sh = slot_shift_of(md->B);
+        own += (long long)md->hm->n_cells * ((md->B + (1 << sh) - 1) >> sh << sh);
+      }
+      packed = group_slots((int)meshes.size()) < 2 * own;
+    }
     if (packed && rus) {
       bool small = false;
       ESR_TRY(latency_bound(2, sms, &small));

@@ -104,3 +104,33 @@ def test_full_batch_slots_equal_single_solves(naca_hr):
         assert np.array_equal(one.get_state(0).astype(np.float32), states[b]), b
         one.close()
     s.close()
+
+
+@pytest.mark.parametrize("counts", [(8,), (9,), (16, 3), (17, 1), (1, 40), (3, 64), (2, 2)])
+@pytest.mark.parametrize("options", [dict(), dict(time_scheme="RK2", dt_mode="local"), dict(stop_rule="density_l2"),
+                                     dict(flux="rusanov", time_scheme="EE")],
+                         ids=["srk2", "rk2-local", "density-l2", "rusanov-ee"])
+def test_slot_groups_of_full_size_solves_equal_single_solves(naca_hr, diamond02, counts, options):
+    """What a full-size float32 batch runs (64-cell tiles; groups of 8 slots, of
+    4 where 8 would leave a fifth of them empty, each mesh its own width where
+    single-slot meshes prevail) on one mesh and on two of unequal slot counts,
+    with an idle slot in the first group: every sampled slot ends bitwise equal
+    to the same case advanced alone."""
+    from eulersr_b200.solver import DeviceMesh, FlowCase, Solver
+    meshes = [DeviceMesh(naca_hr), DeviceMesh(diamond02)][:len(counts)]
+    n = sum(counts)
+    r = np.random.default_rng(n)
+    cases = [FlowCase(mach=float(r.uniform(0.7, 3.0)), aoa_deg=float(r.uniform(-5, 5)), cfl=0.6, tf=1e9, dtype=np.float32,
+                      threshold=1e-30) for _ in range(n)]
+    s = Solver(meshes, list(counts), precision="f32", **options)
+    run = [g for g in range(n) if counts[0] < 3 or g != 1]
+    s.set_cases(run, [cases[g] for g in run])
+    s.step(9)
+    for g in sorted({0, counts[0] // 2, counts[0] - 1, n - 1} & set(run)):
+        one = Solver(meshes[0 if g < counts[0] else 1], 1, precision="f32", **options)
+        one.set_case(0, cases[g])
+        one.step(9)
+        want, got = one.get_state(0), s.get_state(g)
+        assert np.isfinite(want).all() and np.array_equal(want, got), g
+        one.close()
+    s.close()
