@@ -274,7 +274,7 @@ def workload_config(args, mesh):
                         f"(Mach~U[0.7,3] seed 1, alpha in -5..5 step 0.5), SRK2 chunk of {args.chunk} steps",
             "cells": int(mesh.n_cells), "cases_per_gpu": args.cases, "srk2_steps_per_bench_step": args.chunk,
             "scheme": "HLLC + MUSCL/Venkatakrishnan + SRK2, global dt, CFL 0.6 (0.45 transonic)",
-            "l2": "working set > L2 (state 3x + face states 3x of 16 B per cell and case)",
+            "l2": "working set > L2 (state 3x of 16 B per cell and case)",
             "parallelism": f"cases sharded, {args.cases} per GPU"}
 
 

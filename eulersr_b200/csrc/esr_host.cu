@@ -57,10 +57,15 @@ struct DevBuf {
   ~DevBuf() { if (p) cudaFree(p); }
   int alloc(size_t count) {
     if (p) { cudaFree(p); p = nullptr; }
-    n = count;
+    n = 0;
     if (count == 0) return ESR_OK;
     cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-    if (e != cudaSuccess) { p = nullptr; return fail(ESR_ERR_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e)); }
+    if (e != cudaSuccess) {
+      cudaGetLastError();   // reported here, not by the next launch's check
+      p = nullptr;
+      return fail(ESR_ERR_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
+    n = count;
     return ESR_OK;
   }
   // at least `count` elements, keeping the buffer when it is large enough: a
@@ -267,7 +272,9 @@ struct SolverT : SolverBase {
     return sizeof(T) == 4 && !faithful() && P.flux == ESR_FLUX_HLLC && P.reconstruction == ESR_RECON_MUSCL;
   }
 
-  int init(const esr_mesh* const* ms, const int32_t* slots, int nm, const esr_params* p) {
+  // record: measure the launch shapes that a solver of these parameters could
+  // be set to (get_tuning's own instance), also where it would run fused
+  int init(const esr_mesh* const* ms, const int32_t* slots, int nm, const esr_params* p, bool record = false) {
     P = *p;
     device = p->device;
     ESR_CUDA(cudaSetDevice(device));
@@ -436,7 +443,12 @@ struct SolverT : SolverBase {
     ESR_CUDA(cudaStreamSynchronize(stream));
     if (p->block_size != 0 && patch_eligible()) fused = false;   // a launch shape was asked for
     if (muscl() && !fused) ESR_TRY(FV.reserve(3 * total));
-    if (p->block_size == 0) ESR_TRY(autotune());
+    // the fused stage kernel leaves nothing to choose
+    if (p->block_size == 0 && (!fused || record)) ESR_TRY(autotune());
+    created = chosen;
+    created.block = block;
+    created.fused = fused;
+    created.patches = use_patch;
     return ESR_OK;
   }
 
@@ -709,9 +721,9 @@ struct SolverT : SolverBase {
     return ESR_OK;
   }
 
-  // Autotuner: time one full step of every slot (the solver's own meshes,
-  // scheme and slot counts; a uniform finite state, all slots live) for each
-  // launch shape and keep the fastest. Shapes: the cell kernels at 64, 128
+  // Autotuner of the separate kernels: time one full step of every slot (the
+  // solver's own meshes, scheme and slot counts; a uniform finite state, all slots
+  // live) for each launch shape and keep the fastest. Shapes: the cell kernels at 64, 128
   // and 256 threads per block; at the best of those, K2's second register
   // budget, K2 by patches at both budgets, then K1's second budget with the
   // best K2. Results do not depend on the choice: every item is computed the
@@ -720,7 +732,8 @@ struct SolverT : SolverBase {
   // cells and slots), so a second solver of the same shape skips the timing.
   struct TuneChoice {
     int block = 256;
-    bool patches = false, k1 = false, k2 = false, kp = false, fused = false;
+    bool patches = false, k1 = false, k2 = false, kp = false;
+    bool fused = false;   // patch_eligible solvers: the fused stage kernel, not K1 and K2
   };
   struct TuneEntry {
     TuneChoice choice;
@@ -746,10 +759,11 @@ struct SolverT : SolverBase {
     return c.k2 ? ESR_K2_MINB_ALT : ESR_K2_MINB;
   }
   int apply_choice(const TuneChoice& c) {
+    const bool stage_runs = stage_form() && (c.fused || !patch_eligible());
+    if (muscl() && !stage_runs) ESR_TRY(FV.reserve(3 * total));   // before anything changes
     ESR_TRY(build_blocks(c.block));
     use_patch = c.patches && patch_eligible();
-    fused = stage_form() && (c.fused || !patch_eligible());
-    if (muscl() && !fused) ESR_TRY(FV.reserve(3 * total));
+    fused = stage_runs;
     k1_alt = c.k1;
     k2_alt = c.k2;
     kp_alt = c.kp;
@@ -777,8 +791,9 @@ struct SolverT : SolverBase {
   }
   esr_tuning tuning{};
   TuneChoice chosen;
+  TuneChoice created;       // what the solver was created with (set_shape can return to it)
+  bool shape_set = false;
   int autotune() {
-    if (stage_form() && !patch_eligible()) return ESR_OK;   // the fused stage kernel alone: nothing to choose
     const std::string key = tune_key();
     {
       std::lock_guard<std::mutex> lock(tune_mutex());
@@ -842,15 +857,6 @@ struct SolverT : SolverBase {
       ESR_TRY(consider(c));
     }
     chosen = best_c;
-    // The fused stage kernel runs unless a launch shape is asked for: it was
-    // faster than the best separate pair at every size measured (us per step,
-    // 1 slot of 1,450 cells 9 against 25, 32 x 1,810 cells 14 against 26,
-    // 32 x 25,968 62 against 76, 256 x 25,049 386 against 456). The record
-    // above serves callers that set a shape.
-    if (patch_eligible()) {
-      chosen.fused = true;
-      ESR_TRY(FV.alloc(0));   // the face states of the separate kernels
-    }
     launches = before;
     ESR_TRY(apply_choice(chosen));
     tuning.block_size = chosen.block;
@@ -872,6 +878,7 @@ struct SolverT : SolverBase {
   // a launch shape given by the caller (one recorded by an earlier
   // autotuning, say); the chunk graphs are captured again at the next step
   int set_shape(const esr_tuning_variant* v) {
+    if (v->block_size == 0 && !v->k2_patches && !v->k1_minb && !v->k2_minb) return use_shape(created, false);
     if (v->block_size != 64 && v->block_size != 128 && v->block_size != 256)
       return fail(ESR_ERR_ARG, "set_shape: block_size must be 64, 128 or 256");
     if (v->k2_patches != 0 && v->k2_patches != 1) return fail(ESR_ERR_ARG, "set_shape: k2_patches must be 0 or 1");
@@ -898,26 +905,58 @@ struct SolverT : SolverBase {
                                      ") of a float32 fast-fidelity HLLC + MUSCL solver");
       (c.patches ? c.kp : c.k2) = v->k2_minb == alt;
     }
+    return use_shape(c, true);
+  }
+  int use_shape(const TuneChoice& c, bool given) {
     ESR_TRY(apply_choice(c));
     chosen = c;
+    shape_set = given;
     if (g_run) cudaGraphExecDestroy(g_run);
     if (g_plain) cudaGraphExecDestroy(g_plain);
     g_run = g_plain = nullptr;
     g_run_len = g_plain_len = 0;
-    tuning.block_size = c.block;
-    tuning.k2_patches = use_patch ? 1 : 0;
-    tuning.k1_minb = k1_minb_of(c);
-    tuning.k2_minb = k2_minb_of(c);
     return ESR_OK;
   }
+  // The record of the shapes that set_shape takes. A solver that runs the
+  // separate kernels by default has it from its creation, where it chose among
+  // them. One that runs fused is not made to wait (or to allocate 48 B of face
+  // states per item) for kernels that it does not run: they are timed at the
+  // first request, by an instance of their own on the same meshes, and the
+  // record stays empty where the device has no room for that one.
+  void measure_shapes() {
+    if (P.block_size != 0 || !stage_form() || tuning.n_variants > 0) return;
+    {
+      std::lock_guard<std::mutex> lock(tune_mutex());
+      auto it = tune_cache().find(tune_key());
+      if (it != tune_cache().end()) {
+        tuning = it->second.record;
+        tuning.cached = 1;
+        return;
+      }
+    }
+    std::vector<std::unique_ptr<esr_mesh>> ms;
+    std::vector<const esr_mesh*> handles;
+    std::vector<int32_t> slots;
+    for (const auto& md : meshes) {
+      ms.push_back(std::unique_ptr<esr_mesh>(new esr_mesh{std::const_pointer_cast<HostMesh>(md->own)}));
+      handles.push_back(ms.back().get());
+      slots.push_back(md->B);
+    }
+    SolverT<T> probe;
+    if (probe.init(handles.data(), slots.data(), (int)slots.size(), &P, true) == ESR_OK) tuning = probe.tuning;
+  }
   int get_tuning(esr_tuning* out) {
+    measure_shapes();
     *out = tuning;
-    if (out->block_size == 0) out->block_size = block;   // given, not measured
-    out->k2_patches = use_patch ? 1 : 0;
-    TuneChoice now = chosen;
-    now.patches = use_patch;
-    out->k1_minb = k1_minb_of(now);
-    out->k2_minb = k2_minb_of(now);
+    out->fused = fused ? 1 : 0;
+    if (shape_set || tuning.n_variants == 0 || !stage_form()) {   // the shape in use, else the record's fastest
+      out->block_size = block;
+      out->k2_patches = use_patch ? 1 : 0;
+      TuneChoice now = chosen;
+      now.patches = use_patch;
+      out->k1_minb = k1_minb_of(now);
+      out->k2_minb = k2_minb_of(now);
+    }
     return ESR_OK;
   }
 
@@ -2338,7 +2377,9 @@ int esr_solver_num_slots(const esr_solver* solver, int32_t* n) {
 
 int esr_solver_tuning(const esr_solver* solver, esr_tuning* out) {
   if (!solver || !out) return fail(ESR_ERR_ARG, "null argument");
+  ESR_GUARD_BEGIN
   return dispatch_any(const_cast<esr_solver*>(solver), [&](auto& s) { return s.get_tuning(out); });
+  ESR_GUARD_END
 }
 
 int esr_solver_set_shape(esr_solver* solver, const esr_tuning_variant* shape) {

@@ -430,14 +430,18 @@ class Solver:
         return int(v.value)
 
     def tuning(self) -> dict:
-        """Block size in use and, when autotuned, the step time per candidate."""
+        """Whether the fused stage kernel runs, and the record of launch shapes
+        (``step_ms`` per candidate, every shape in ``variants``; empty when
+        ``block_size`` was given). A fused solver measures them at its first
+        call, on the device."""
         t = F.Tuning()
         F.check(F.lib().esr_solver_tuning(self.handle, C.byref(t)))
         return t.as_dict()
 
     def set_shape(self, block_size: int, k2_patches: bool = False, k1_minb: int = 0, k2_minb: int = 0):
         """Run with this launch shape (one of ``tuning()['variants']``, say);
-        a register budget of 0 is the kernel's default."""
+        a register budget of 0 is the kernel's default. ``set_shape(0)`` returns
+        to what the solver was created with."""
         v = F.TuningVariant(block_size=int(block_size), k2_patches=int(bool(k2_patches)), k1_minb=int(k1_minb),
                             k2_minb=int(k2_minb), step_ms=0.0)
         F.check(F.lib().esr_solver_set_shape(self.handle, C.byref(v)))

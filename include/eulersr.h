@@ -315,22 +315,26 @@ typedef struct esr_kernel_times {
 } esr_kernel_times;
 int esr_profile_step(esr_solver* solver, int32_t nsteps, esr_kernel_times* out);
 
-/* The record of launch shapes: MUSCL solves run each Runge-Kutta stage as one
- * fused kernel. A float32 fast-fidelity HLLC solver can also run it as the
- * separate kernels K1 (reconstruction) and K2 (fluxes), at a shape given by
- * esr_params.block_size or esr_solver_set_shape; with block_size = 0 it times
- * one full step of all its slots for each of those shapes at creation and
- * records them, with the fastest in the fields below (no reference
- * counterpart: XLA picks launch shapes). Constant reconstruction has no fused
- * form: its solver keeps the fastest block size. Shapes: the
- * cell kernels at 64, 128 and 256 threads per block; at the best of those,
- * where the float32 fast kernels run, K2's second register budget, K2 by
- * patches at both of its budgets (float32 fast fidelity, HLLC + MUSCL), and
- * K1's second budget with the best K2. A register budget is the number of
- * resident blocks per SM a kernel is compiled for. The choice is kept for
- * the process per solver shape (device, precision, scheme, each mesh's cells
- * and slots): a second solver of the same shape takes it without timing
- * (cached = 1). Results do not depend on the choice. */
+/* The record of launch shapes (no reference counterpart: XLA picks launch
+ * shapes). MUSCL solves run each Runge-Kutta stage as one fused kernel (`fused`
+ * = 1), except float64 with fidelity reference and larger float32 solves with
+ * fidelity reference, which run the separate kernels K1 (reconstruction) and K2
+ * (fluxes), as constant reconstruction runs K2. A float32 fast-fidelity HLLC
+ * solver can also run the separate kernels, at a shape given by
+ * esr_params.block_size or esr_solver_set_shape. With block_size = 0 a solver of
+ * separate kernels times one full step of all its slots for each shape at
+ * creation and keeps the fastest; a fused one times them at the first
+ * esr_solver_tuning (an instance of its own on the device, 96 B of state per cell
+ * and slot; without room for it the record stays empty) and runs none of them.
+ * The fields in front are the shape in use, or for a fused solver the record's
+ * fastest. Shapes: the cell kernels at 64, 128 and 256 threads per block; at the
+ * best of those, where the float32 fast HLLC + MUSCL kernels run, K2's second
+ * register budget, K2 by patches at both of its budgets, and K1's second budget
+ * with the best K2. A register budget is the number of resident blocks per SM a
+ * kernel is compiled for. The record is kept for the process per solver shape
+ * (device, precision, scheme, each mesh's cells and slots): a second solver of
+ * the same shape takes it without timing (cached = 1). Results do not depend on
+ * the choice. */
 #define ESR_TUNING_MAX_VARIANTS 12
 typedef struct esr_tuning_variant {
     int32_t block_size;       /* threads per block of K1 (and of the per-cell K2) */
@@ -350,13 +354,14 @@ typedef struct esr_tuning {
     int32_t k1_minb;          /* register budgets in use (0: not constrained) */
     int32_t k2_minb;
     int32_t n_variants;       /* every shape timed, in order */
-    int32_t reserved;
+    int32_t fused;            /* 1: the fused stage kernel runs */
     esr_tuning_variant variants[ESR_TUNING_MAX_VARIANTS];
 } esr_tuning;
 int esr_solver_tuning(const esr_solver* solver, esr_tuning* out);
 /* Run the solver with the given launch shape (a variant recorded by an
  * earlier autotuning, or chosen by hand); step_ms is ignored, a budget of 0
- * means the kernel's default. ESR_ERR_ARG for a shape this solver cannot run
+ * means the kernel's default. Where K1 and K2 can run they replace the fused
+ * kernel; a shape of zeros returns to what the solver was created with. ESR_ERR_ARG for a shape this solver cannot run
  * (K2 by patches or a second budget outside float32 fast fidelity, HLLC +
  * MUSCL), ESR_ERR_STATE while a submitted batch owns the slots. Results do
  * not depend on the shape. */

@@ -675,3 +675,52 @@ def test_rusanov_fast_f32_is_as_exact_as_the_reference_float32(diamond02):
     Wo64, _, _, _ = _oracle_steps(diamond02, np.float64, 2.5, 5.0, 20, flux="rusanov")
     Wg, _, _ = _gpu_steps(diamond02, "f32", 2.5, 5.0, 20, flux="rusanov", fidelity="fast")
     assert rel_err(Wg, Wo64) <= 1.5 * rel_err(Wo32, Wo64)
+
+
+def test_fused_solver_is_not_tuned_at_creation(naca02):
+    """A solver that runs the fused stage kernel is created without the
+    separate kernels' face states (48 B per cell and slot): it fits where they
+    do not, and its record of shapes is then empty instead of an error. With
+    room, the record is measured at the first request and says what runs;
+    set_shape(0) returns to the fused kernel, and f64 and Rusanov solvers have a
+    record as well."""
+    import gc
+    import torch
+    from eulersr_b200.solver import DeviceMesh, FlowCase, Solver
+    dm = DeviceMesh(naca02)
+    case = FlowCase(mach=1.4, aoa_deg=2.0, tf=1.0, dtype=np.float32)
+    one = Solver(dm, 1, precision="f32")
+    one.set_case(0, case)
+    one.step(5)
+    want = one.get_state(0)
+    slots = 29000                                  # 20.0 M items: 0.96 GB of state, 0.96 GB of face states
+    items = naca02.n_cells * slots
+    torch.cuda.synchronize()
+    gc.collect()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    fill = torch.empty(free - int(1.45 * 48 * items), dtype=torch.uint8, device="cuda")
+    try:
+        s = Solver(dm, slots, precision="f32")
+        t = s.tuning()
+        assert t["fused"] and t["variants"] == [] and t["step_ms"] == {}
+        s.set_case(slots - 1, case)
+        s.step(5)
+        assert np.array_equal(s.get_state(slots - 1), want)
+        s.close()
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    t = one.tuning()
+    assert t["fused"] and len(t["variants"]) == 7 and not t["cached"]
+    v = t["variants"][0]
+    one.set_shape(v["block_size"], v["k2_patches"], v["k1_minb"], v["k2_minb"])
+    assert not one.tuning()["fused"] and one.profile_step(1)["recon_launches"] > 0
+    one.set_shape(0)
+    assert one.tuning()["fused"] and one.profile_step(1)["recon_launches"] == 0
+    for opts in (dict(precision="f64"), dict(precision="f32", flux="rusanov"),
+                 dict(precision="f32", fidelity="reference")):
+        t = Solver(dm, 3, **opts).tuning()
+        assert t["fused"] and sorted(t["step_ms"]) == [64, 128, 256] and all(x > 0 for x in t["step_ms"].values())
+    t = Solver(dm, 3, precision="f64", fidelity="reference").tuning()
+    assert not t["fused"] and sorted(t["step_ms"]) == [64, 128, 256]
