@@ -134,3 +134,24 @@ def test_slot_groups_of_full_size_solves_equal_single_solves(naca_hr, diamond02,
         assert np.isfinite(want).all() and np.array_equal(want, got), g
         one.close()
     s.close()
+
+
+@pytest.mark.parametrize("counts", [(4,), (6,), (3, 20)])
+@pytest.mark.parametrize("dt_mode", ["global", "local"])
+def test_float64_slot_groups_of_full_size_solves_equal_single_solves(naca_hr, diamond02, counts, dt_mode):
+    """The same for the float64 stage kernel's 64-cell tiles and groups of 4."""
+    from eulersr_b200.solver import DeviceMesh, FlowCase, Solver
+    meshes = [DeviceMesh(naca_hr), DeviceMesh(diamond02)][:len(counts)]
+    n = sum(counts)
+    r = np.random.default_rng(n)
+    cases = [FlowCase(mach=float(r.uniform(0.7, 3.0)), aoa_deg=float(r.uniform(-5, 5)), cfl=0.6, tf=1e9) for _ in range(n)]
+    s = Solver(meshes, list(counts), precision="f64", dt_mode=dt_mode)
+    s.set_cases(list(range(n)), cases)
+    s.step(6)
+    for g in sorted({0, counts[0] - 1, n - 1}):
+        one = Solver(meshes[0 if g < counts[0] else 1], 1, precision="f64", dt_mode=dt_mode)
+        one.set_case(0, cases[g])
+        one.step(6)
+        assert np.array_equal(one.get_state(0), s.get_state(g)), g
+        one.close()
+    s.close()

@@ -724,3 +724,41 @@ def test_fused_solver_is_not_tuned_at_creation(naca02):
         assert t["fused"] and sorted(t["step_ms"]) == [64, 128, 256] and all(x > 0 for x in t["step_ms"].values())
     t = Solver(dm, 3, precision="f64", fidelity="reference").tuning()
     assert not t["fused"] and sorted(t["step_ms"]) == [64, 128, 256]
+
+
+@pytest.mark.parametrize("counts", [(3,), (4,), (5,), (8,), (9,), (9, 2), (1, 8), (2, 5)])
+@pytest.mark.parametrize("options", [dict(precision="f64"), dict(precision="f64", flux="rusanov", time_scheme="RK2"),
+                                     dict(precision="f64", dt_mode="local", time_scheme="EE"),
+                                     dict(precision="f32", fidelity="reference", dt_mode="local"),
+                                     dict(precision="f32", time_scheme="RK2"), dict(precision="f32", time_scheme="EE")],
+                         ids=lambda o: "-".join(map(str, o.values())))
+def test_stage_groups_equal_single_solves(naca02, diamond02, counts, options):
+    """Several slots per block (full groups, a part-filled last one, an idle
+    slot in the first) and meshes of unequal slot counts, whose groups differ in
+    width: every slot ends bitwise equal to a single solve of its case, and the
+    density residual of the stop rule is the same number."""
+    from eulersr_b200.solver import DeviceMesh, FlowCase, Solver
+    meshes = [DeviceMesh(naca02), DeviceMesh(diamond02)][:len(counts)]
+    n = sum(counts)
+    r = np.random.default_rng(n)
+    dtype = np.float64 if options["precision"] == "f64" else np.float32
+    opts = dict(options, stop_rule="density_l2", threshold=1e-30, check_every=4)
+    cases = [FlowCase(mach=float(r.uniform(0.7, 3.0)), aoa_deg=float(r.uniform(-5, 5)), cfl=0.6, max_steps=9, dtype=dtype)
+             for _ in range(n)]
+
+    def solve(solver, slots, cases):
+        for g, c in zip(slots, cases):
+            solver.set_case(g, c)
+        res = solver.run()
+        return [(solver.get_state(g), res[g]) for g in slots]
+
+    run = [g for g in range(n) if counts[0] < 3 or g != 1]
+    s = Solver(meshes, list(counts), **opts)
+    got = solve(s, run, [cases[g] for g in run])
+    s.close()
+    for g, (state, result) in zip(run, got):
+        one = Solver(meshes[0 if g < counts[0] else 1], 1, **opts)
+        want, result1 = solve(one, [0], [cases[g]])[0]
+        assert np.isfinite(want).all() and np.array_equal(want, state), g
+        assert result["steps"] == result1["steps"] and result["last_rel"] == result1["last_rel"] > 0, g
+        one.close()
