@@ -27,9 +27,16 @@ N_OUT = 4
 ROW_TILE = 128  # the GEMM tiles rows by 128
 
 
+def _address(t):
+    """Device address of a CUDA tensor. A tensor in host memory is refused here:
+    the kernels would dereference its address."""
+    if not t.is_cuda:
+        raise ValueError(f"expected a CUDA tensor, got one on {t.device}")
+    return t.data_ptr()
+
+
 def _p(t):
-    """Device address of a CUDA tensor for a kernel argument. A tensor in host
-    memory is refused here: the kernels would dereference its address."""
+    """The address as a kernel argument, or None."""
     if t is None:
         return None
     if not t.is_cuda:
@@ -38,8 +45,8 @@ def _p(t):
 
 
 def _array(tensors):
-    """Host array of four device addresses, or None; host tensors are refused as in _p."""
-    return (C.c_void_p * 4)(*[_p(t) for t in tensors]) if tensors is not None else None
+    """Host array of four device addresses, or None."""
+    return (C.c_void_p * 4)(*[_address(t) for t in tensors]) if tensors is not None else None
 
 
 def _aligned(*tensors):
@@ -126,7 +133,7 @@ class MLP:
         tag = "k" if keep else "f"
         y = self._buf(f"{tag}y", (rows, N_OUT), torch.float32)
         # the layer calls take biases at any address (flat vectors that are views of a larger one)
-        if self.fused and _aligned(self.p):
+        if self.fused and self.p.data_ptr() % 16 == 0:
             h = z = None
             if keep:
                 h, z = ([self._buf(f"k{n}{l}", (rows, H), torch.bfloat16) for l in range(4)] for n in "hz")
@@ -151,19 +158,19 @@ class MLP:
         """The network's device addresses (the flat vectors may be replaced between calls)."""
         return self._addresses(self.p, self.pb)
 
+    def _flat(self, t):
+        """Address of a flat vector. One in host memory or too short for the layout is refused: kernels use it."""
+        if t.numel() < self.n_params:
+            raise ValueError(f"a flat vector of {t.numel()} values cannot hold the network's {self.n_params}")
+        if not t.is_cuda:
+            raise ValueError(f"expected a CUDA tensor, got one on {t.device}")
+        return t.data_ptr()
+
     def _addresses(self, flat, weights=None):
-        """Device addresses of every weight and bias in `flat`; those of W0..W3 in the BF16 copy, if given.
-        A flat vector in host memory or too short for the layout is refused: kernels use these addresses."""
-        for t in (flat,) if weights is None else (flat, weights):
-            if t.numel() < self.n_params:
-                raise ValueError(f"a flat vector of {t.numel()} values cannot hold the network's {self.n_params}")
-        p = _p(flat).value
-        w = (4, p) if weights is None else (2, _p(weights).value)
-        n = F.MlpNet()
-        n.W[:] = [w[1] + w[0] * self.offsets[f"W{l}"][0] for l in range(4)]
-        n.b[:] = [p + 4 * self.offsets[f"b{l}"][0] for l in range(4)]
-        n.W4, n.b4 = p + 4 * self.offsets["W4"][0], p + 4 * self.offsets["b4"][0]
-        return n
+        """Device addresses of every weight and bias in `flat`; those of W0..W3 in the BF16 copy, if given."""
+        p = self._flat(flat)
+        w = [p + 4 * o for o in _W_AT] if weights is None else [q + 2 * o for q in (self._flat(weights),) for o in _W_AT]
+        return F.MlpNet((C.c_void_p * 4)(*w), (C.c_void_p * 4)(*[p + 4 * o for o in _B_AT]), p + 4 * _W4_AT, p + 4 * _B4_AT)
 
     # ----------------------------------------------------------- backward
     def backward(self, acts, dY, splits=None):
@@ -240,3 +247,16 @@ class MLP:
 
     def grads_numpy(self):
         return {name: self.gview(name).detach().cpu().numpy().astype(np.float64) for name, _ in self.SHAPES}
+
+
+def _layout():
+    at, off = {}, 0
+    for name, shape in MLP.SHAPES:
+        at[name] = off
+        off += math.prod(shape)
+    return at
+
+
+_AT = _layout()
+_W_AT, _B_AT = [_AT[f"W{l}"] for l in range(4)], [_AT[f"b{l}"] for l in range(4)]
+_W4_AT, _B4_AT = _AT["W4"], _AT["b4"]
