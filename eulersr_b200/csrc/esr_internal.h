@@ -33,7 +33,7 @@ struct HostMesh {
   std::vector<float> wall_n_ref32, wall_ds_ref32;
   std::vector<double> wall_n_ref64, wall_ds_ref64;
   std::vector<int> nbr;           // 4 x n_cells (x,y,z neighbours, w packed)
-  std::vector<float> centre;      // barycentres (x, y), renumbered
+  std::vector<float> centre;      // barycentres (x, y) from the first point, renumbered
   std::vector<int> wall_cell;     // renumbered owner cell of each force face
   std::vector<double> wall_n;     // (nx, ny) per force face
   std::vector<double> wall_ds;    // face length per force face

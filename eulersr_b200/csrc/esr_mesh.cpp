@@ -522,8 +522,9 @@ int prepare_mesh(const esr_mesh_desc& d, HostMesh& hm, std::string& err) {
       G(G_C0Y + 2 * k, i) = w[k] * (-a12 * dxk[k][0] + a11 * dxk[k][1]) / det;
     }
     G(G_AREA, i) = area[c];
-    hm.centre[2 * i] = (float)bary[2 * c];
-    hm.centre[2 * i + 1] = (float)bary[2 * c + 1];
+    // from the mesh's first point: a mesh far from the origin keeps its shape in float32
+    hm.centre[2 * i] = (float)(bary[2 * c] - d.points[0]);
+    hm.centre[2 * i + 1] = (float)(bary[2 * c + 1] - d.points[1]);
     double bl = 0.0;
     if (d.sponge) {
       const double y = bary[2 * c + 1];
