@@ -259,6 +259,29 @@ def ragged_workload(n_cases=1024, seed=2, rank=0, world=1):
     return meshes, per
 
 
+LINE_MAX = 8000   # characters of the JSON line: a reader that keeps a few KB of output must get all of it
+# What a longer line gives up, to a JSON line on standard error
+DETAILS = (("converged_cases_per_s", "per_case"), ("converged_cases_per_s", "by_case_class"),
+           ("converged_cases_per_s", "details"), ("converged_cases_per_s", "warm_passes"),
+           ("converged_cases_per_s", "warm_mlp_streamed"), ("converged_cases_per_s", "warm_mlp_lr_longest_first_queue"),
+           ("converged_cases_per_s", "unsteady_capped_protocol"), ("cell_updates", "config"), ("config", "training"),
+           ("config", "tuning"))
+
+
+def emit(line):
+    """Print the bench's one JSON line on standard output. When it is too long
+    its breakdowns go to standard error instead, as one JSON object."""
+    if len(json.dumps(line)) > LINE_MAX:
+        line, moved = dict(line), {}
+        for group, key in DETAILS:
+            if isinstance(line.get(group), dict) and key in line[group]:
+                moved.setdefault(group, {})[key] = line[group][key]
+                line[group] = {k: v for k, v in line[group].items() if k != key}
+        print(json.dumps({"details": moved}), file=sys.stderr, flush=True)
+        line["details"] = "standard error"
+    print(json.dumps(line), flush=True)
+
+
 def workload_config(args, mesh):
     if getattr(args, "workload", "naca") == "ragged":
         meshes, per = mesh
@@ -349,7 +372,7 @@ def run_single(args, world, rank, local):
                         "api": "esr_set_case (freestream) + esr_run, results read back; wall clock"},
                 "roofline": roofline, "cpu_baseline": cpu, "clocks": clk, "gpu_launches": int(launches),
                 "kernel_times_ms": kt}
-        print(json.dumps(line), flush=True)
+        emit(line)
     barrier(world)
     s.close()
     return 0
@@ -510,7 +533,7 @@ def run_throughput(args, world, rank, local, report=True):
                 "alg_bytes_per_cell_update": alg_step_bytes,
                 "roofline": roofline, "e2e": e2e, "cpu_baseline": cpu, "clocks": clk,
                 "gpu_launches": int(launches), "kernel_times_ms": kt}
-        print(json.dumps(line), flush=True)
+        emit(line)
     barrier(world)
     s.close()
     return out
@@ -675,7 +698,7 @@ def run_reference_warm(args, world, rank):
             "cpu_baseline": {"value": value, "unit": WARM_UNIT, "cores": thr, "kind": "port", "sample": sample},
             "e2e": {"value": value, "unit": WARM_UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
             "per_case": recs, "note": f"host has {os.cpu_count()} cores"}
-    print(json.dumps(line), flush=True)
+    emit(line)
     return 0
 
 
@@ -894,7 +917,7 @@ def run_warm(args, world, rank, local):
                                                       "config")},
                 "cpu_baseline": cpu, "clocks": clk, "gpu_launches": int(launches),
                 "gpu_launches_throughput_leg": thr["gpu_launches"]}
-        print(json.dumps(line), flush=True)
+        emit(line)
     return 0
 
 
@@ -926,7 +949,7 @@ def main():
     ap.add_argument("--make-truth", action="store_true", help="write the held-out cases' reference CDs and exit")
     ap.add_argument("--make-plain-truth", action="store_true",
                     help="write the reference CDs of the throughput workload's NACA0012 cases and exit")
-    ap.add_argument("--block", default="0", help="throughput workloads: 0 (autotuned), 64, 128, 256 or patches")
+    ap.add_argument("--block", default="0", help="throughput workloads: 0 (the solver's own choice), 64, 128, 256 or patches")
     args = ap.parse_args()
     args.block = args.block if args.block == "patches" else int(args.block)
     args.warmup = max(3, args.warmup)

@@ -443,3 +443,25 @@ def test_throughput_over_two_gloo_ranks():
     assert n0 + n1 == 128 and v0 == v1
     assert v0 == 1000 * 128 * 50 * 2 / (2 * 25.0 * 1e-3)
     assert text1.strip() == "" and json.loads(text0.strip().splitlines()[-1])["n_gpus"] == 2
+
+
+def test_headline_line_stays_short(monkeypatch, capsys):
+    """With the real number of cases the per-case and by-class breakdowns make
+    a line of more than 20 KB, of which a reader that keeps the last few KB gets no
+    JSON. The line stays below 8,000 characters with every key that it is read
+    for; the breakdowns are one JSON object on standard error."""
+    import json
+    _install_warm_fakes(monkeypatch.setattr)
+    args = _warm_args()
+    args.n_eval = 128
+    assert bench.run_warm(args, 1, 0, 0) == 0
+    out, err = capsys.readouterr()
+    assert len(out.strip().splitlines()) == 1 and len(out) <= 8000
+    line = json.loads(out)
+    for key in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+                "scaling", "vs_baseline", "dtype", "data", "config", "e2e", "roofline", "cpu_baseline", "clocks",
+                "gpu_launches"):
+        assert key in line, key
+    assert line["value"] > 0 and line["converged_cases_per_s"]["plain_single_case"] > 0
+    details = json.loads(err.strip().splitlines()[-1])["details"]["converged_cases_per_s"]
+    assert len(details["per_case"]["mlp"]["steps"]) == 128 and details["by_case_class"]["by_mach_band"]
