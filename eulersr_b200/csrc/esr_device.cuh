@@ -1,9 +1,10 @@
 // esr_device.cuh -- device numerics and kernels of the explicit FVM solve.
 //
 // Every formula restates the EulerSR JAX solver (citations are paths inside
-// the EulerSR checkout) with its evaluation order, so float32/float64 results
-// track the reference's rounding; the data layout and the kernel split are
-// this project's own:
+// the EulerSR checkout): with its evaluation order in reference fidelity and in
+// constant reconstruction, equal in real arithmetic in fast MUSCL solves (the
+// precision policy below). The data layout and the kernel split are this
+// project's own:
 //
 //   state      W[item], item = seg.off + cell * B + slot  (one float4/double4
 //              per cell and case, cases of one mesh innermost so a warp of a

@@ -10,16 +10,18 @@
 //      leaves the block),
 //   C  evaluates the face fluxes of the tile's cells,
 //   D  sums them per cell in edge order, applies the sponge and the stage update.
-// What bounds it: instruction issue in large batches (58 % of issue slots,
-// 660 instructions per item of which 325 are phase B's, 19 MB of DRAM traffic
-// per million items), the latency of one launch and its four dependent phases
-// in single solves. The separate K1 / K2 pass 96 B of face states per item and
-// stage through memory and pay two launches; here a stage moves the state
-// alone, for about a third more reconstructions. Measured (us per SRK2 step,
-// separate kernels -> fused): 1 slot x 1,450 cells 20.0 -> 7.4, 1 x 25,968
-// 21.0 -> 9.1, 32 x 1,810 19.9 -> 12.4, 32 x 25,968 88 -> 60, 256 x 25,049
-// 569 -> 382; float64 1 x 19,384 37 -> 14, 24 x 25,968 282 -> 153; reference
-// fidelity 1 x 19,384 29 -> 24.
+// What bounds it: instruction issue in large batches (57-60 % of issue slots,
+// 660-677 thread instructions per cell and slot, of which 324 are phase B's; 19
+// B of DRAM traffic per cell and slot in a first stage, 35 in a second), the
+// latency of one launch and its four dependent phases in single solves. The
+// separate K1 / K2 pass 96 B of face states per item and stage through memory
+// and pay two launches; here a stage moves the state alone, for about a third
+// more reconstructions. Measured 400 steps from freestream, us per SRK2 step,
+// the separate kernels of this build at their best shape -> fused: 1 slot x
+// 1,450 cells 15.1 -> 7.1, 1 x 25,968 16.8 -> 8.7, 32 x 1,810 15.6 -> 11.9, 32 x
+// 25,968 64.4 -> 58.8, 256 x 25,049 460 -> 388. Where this build has no separate
+// form, against the earlier one: float64 1 x 19,384 37.1 -> 13.7, 24 x 25,968
+// 224 -> 129; reference fidelity 1 x 19,384 34.2 -> 26.7.
 //
 // CANON (fast fidelity): each face of the tile once, from its owner (the
 // lower cell), the flux stored over the two face states it came from, negated
@@ -370,8 +372,9 @@ __device__ __forceinline__ void base_pair(const float4* p, int dB, bool wide, fl
 #define ESR_PAIR_THREADS 128
 #endif
 // 128 threads and 5 blocks per SM (94 registers, 45 KB of shared memory at 64
-// cells x 8 slots): 404 us per step of 256 x 25,049 against 448 at 4 blocks,
-// 413 at 80 cells x 160 threads x 4, 419 at 96 x 192 x 3, 429-455 at 48 cells
+// cells x 8 slots), swept on an earlier build (with IEEE square roots; 388 us now):
+// 404 us per step of 256 x 25,049 against 448 at 4 blocks, 413 at 80 cells x
+// 160 threads x 4, 419 at 96 x 192 x 3, 429-455 at 48 cells
 constexpr int kPairThreads = ESR_PAIR_THREADS;
 constexpr int kLoads = 4;            // state rows a thread has in flight
 constexpr uint32_t kAnyBoundary = 7u | 7u << 6 | 7u << 12;   // kind bits of the packed slot word
