@@ -504,33 +504,42 @@ __global__ void __launch_bounds__(256) k_reduce_splits(const __grid_constant__ R
 }
 
 // column sums of a BF16 [rows x C] matrix in fixed row blocks, row by row
-// (bias gradients). A thread owns two columns with 32 rows in flight:
-// 32,768 x 256 (16.8 MB) takes 5 us (as a quarter of one launch), 22 us load by load.
+// (bias gradients), 32 rows in flight. A thread owns two columns in 4-byte
+// loads (VEC), one where C is odd or X not aligned for them: 32,768 x 256 (16.8
+// MB) takes 5 us (as a quarter of one launch), 22 us load by load; 32,768 x 7
+// 6 us, 16 us with two columns a thread.
 template <bool VEC>
 __global__ void __launch_bounds__(128) k_colsum_part(const bf16* __restrict__ X, int rows, int C, int rows_per_block,
                                                      float* __restrict__ part) {
   constexpr int U = 32;
-  const int c = 2 * (blockIdx.y * blockDim.x + threadIdx.x);
+  const int c = (VEC ? 2 : 1) * (blockIdx.y * blockDim.x + threadIdx.x);
   if (c >= C) return;
   const int r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
   float s0 = 0.f, s1 = 0.f;
-  if (c + 1 < C) {
-    int r = r0;
+  int r = r0;
+  if constexpr (VEC) {
     for (; r + U <= r1; r += U) {
       __nv_bfloat162 v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = load2<VEC>(X + (size_t)(r + u) * C + c);
+      for (int u = 0; u < U; ++u) v[u] = load2<true>(X + (size_t)(r + u) * C + c);
 #pragma unroll
       for (int u = 0; u < U; ++u) { s0 += __bfloat162float(v[u].x); s1 += __bfloat162float(v[u].y); }
     }
     for (; r < r1; ++r) {
-      const __nv_bfloat162 v = load2<VEC>(X + (size_t)r * C + c);
+      const __nv_bfloat162 v = load2<true>(X + (size_t)r * C + c);
       s0 += __bfloat162float(v.x);
       s1 += __bfloat162float(v.y);
     }
     part[(size_t)blockIdx.x * C + c + 1] = s1;
   } else {
-    for (int r = r0; r < r1; ++r) s0 += __bfloat162float(X[(size_t)r * C + c]);
+    for (; r + U <= r1; r += U) {
+      bf16 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = X[(size_t)(r + u) * C + c];
+#pragma unroll
+      for (int u = 0; u < U; ++u) s0 += __bfloat162float(v[u]);
+    }
+    for (; r < r1; ++r) s0 += __bfloat162float(X[(size_t)r * C + c]);
   }
   part[(size_t)blockIdx.x * C + c] = s0;
 }
@@ -1752,8 +1761,9 @@ int esr_mlp_backward(const esr_mlp_net* net, const void* X, int32_t rows, const 
 
 int esr_colsum_bf16(const void* X, int32_t rows, int32_t C, int32_t rpb, float* part, void* stream) {
   if (!X || !part || rows <= 0 || C <= 0 || rpb <= 0) return mfail(ESR_ERR_ARG, "colsum: bad argument");
-  dim3 grid((rows + rpb - 1) / rpb, (C + 255) / 256);
-  auto* k = C % 2 == 0 && ((uintptr_t)X & 3) == 0 ? k_colsum_part<true> : k_colsum_part<false>;
+  const bool vec = C % 2 == 0 && ((uintptr_t)X & 3) == 0;
+  dim3 grid((rows + rpb - 1) / rpb, vec ? (C + 255) / 256 : (C + 127) / 128);
+  auto* k = vec ? k_colsum_part<true> : k_colsum_part<false>;
   k<<<grid, 128, 0, (cudaStream_t)stream>>>((const bf16*)X, rows, C, rpb, part);
   cudaError_t err = cudaGetLastError();
   return err == cudaSuccess ? ESR_OK : mfail(ESR_ERR_CUDA, cudaGetErrorString(err));
