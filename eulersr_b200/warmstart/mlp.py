@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import struct
 
 import numpy as np
 import torch
@@ -169,8 +170,9 @@ class MLP:
     def _addresses(self, flat, weights=None):
         """Device addresses of every weight and bias in `flat`; those of W0..W3 in the BF16 copy, if given."""
         p = self._flat(flat)
-        w = [p + 4 * o for o in _W_AT] if weights is None else [q + 2 * o for q in (self._flat(weights),) for o in _W_AT]
-        return F.MlpNet((C.c_void_p * 4)(*w), (C.c_void_p * 4)(*[p + 4 * o for o in _B_AT]), p + 4 * _W4_AT, p + 4 * _B4_AT)
+        q, (w0, w1, w2, w3) = (p, _W_F32) if weights is None else (self._flat(weights), _W_BF16)
+        b0, b1, b2, b3, w4, b4 = _REST
+        return F.MlpNet.from_buffer_copy(_pack(q + w0, q + w1, q + w2, q + w3, p + b0, p + b1, p + b2, p + b3, p + w4, p + b4))
 
     # ----------------------------------------------------------- backward
     def backward(self, acts, dY, splits=None):
@@ -249,14 +251,16 @@ class MLP:
         return {name: self.gview(name).detach().cpu().numpy().astype(np.float64) for name, _ in self.SHAPES}
 
 
-def _layout():
+def _byte_offsets(names, size):
+    """Where each named parameter starts in a flat vector of `size`-byte values."""
     at, off = {}, 0
     for name, shape in MLP.SHAPES:
-        at[name] = off
+        at[name] = off * size
         off += math.prod(shape)
-    return at
+    return tuple(at[n] for n in names)
 
 
-_AT = _layout()
-_W_AT, _B_AT = [_AT[f"W{l}"] for l in range(4)], [_AT[f"b{l}"] for l in range(4)]
-_W4_AT, _B4_AT = _AT["W4"], _AT["b4"]
+# the addresses of an esr_mlp_net in its order: W0..W3 in either precision, then the FP32 rest
+_W_F32, _W_BF16 = (_byte_offsets(("W0", "W1", "W2", "W3"), size) for size in (4, 2))
+_REST = _byte_offsets(("b0", "b1", "b2", "b3", "W4", "b4"), 4)
+_pack = struct.Struct("10P").pack
