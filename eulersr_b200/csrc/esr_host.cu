@@ -942,8 +942,13 @@ struct SolverT : SolverBase {
       handles.push_back(ms.back().get());
       slots.push_back(md->B);
     }
-    SolverT<T> probe;
-    if (probe.init(handles.data(), slots.data(), (int)slots.size(), &P, true) == ESR_OK) tuning = probe.tuning;
+    int current = device;
+    cudaGetDevice(&current);   // init selects the solver's
+    {
+      SolverT<T> probe;
+      if (probe.init(handles.data(), slots.data(), (int)slots.size(), &P, true) == ESR_OK) tuning = probe.tuning;
+    }
+    cudaSetDevice(current);
   }
   int get_tuning(esr_tuning* out) {
     measure_shapes();
